@@ -205,8 +205,9 @@ void launch_aw_l2r_weights(cudaStream_t s, const float *wr, const float *wt, con
                            int W, int D, int r);
 void launch_aw_r2l_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,
                            int W, int D, int r);
-void launch_disp_refine(cudaStream_t s, const uint8_t *in, uint8_t *out, const int *horz, const int *vert, int H,
-                        int W, int D);
+// in place; runs: scratch [H][W] words (the copy the votes are read from); two launches
+void launch_disp_refine(cudaStream_t s, uint8_t *disp, uint16_t *runs, const int *horz, const int *vert, int H, int W,
+                        int D);
 // k_wta.cu
 void launch_wta_local(cudaStream_t s, const float *cost, uint16_t *raw, int *row_last, int H, int W, int D,
                       int argmax);

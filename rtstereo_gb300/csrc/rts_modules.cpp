@@ -410,23 +410,19 @@ rts_status rts_disp_refinement(rts_ctx *ctx, rts_mem m, uint8_t *disp, const int
                                int D) {
     PROLOGUE(ctx);
     RTS_TRY(check_dims(c, D, H, W));
-    void *dd, *tmp;
+    void *dd, *runs;
     const void *dh, *dv;
     RTS_TRY(stage_inout(c, m, SL_IN0, disp, pix(H, W), &dd));
     RTS_TRY(stage_in(c, m, SL_IN1, horz, pix(H, W) * 8, &dh));
     RTS_TRY(stage_in(c, m, SL_IN2, vert, pix(H, W) * 8, &dv));
-    RTS_TRY(scratch(c, SL_TMP0, pix(H, W), &tmp));
+    RTS_TRY(scratch(c, SL_TMP0, pix(H, W) * 2, &runs));
     {
         StageScope sc(c, "disp_refine");
-        launch_disp_refine(c->stream, (const uint8_t *)dd, (uint8_t *)tmp, (const int *)dh, (const int *)dv, H, W, D);
-        count_launch(c);
+        launch_disp_refine(c->stream, (uint8_t *)dd, (uint16_t *)runs, (const int *)dh, (const int *)dv, H, W, D);
+        count_launch(c, 2);
     }
     RTS_TRY(check_launch(c, "disp_refine"));
-    if (m == RTS_DEVICE) {
-        RTS_CU(c, cudaMemcpyAsync(disp, tmp, pix(H, W), cudaMemcpyDeviceToDevice, c->stream));
-        return RTS_OK;
-    }
-    RTS_TRY(finish_out(c, m, disp, tmp, pix(H, W)));
+    RTS_TRY(finish_out(c, m, disp, dd, pix(H, W)));
     return finish(c, m);
 }
 
