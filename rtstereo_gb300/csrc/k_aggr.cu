@@ -385,37 +385,6 @@ __global__ void k_prefix_h(float *__restrict__ cost, int H, int W, int D) {
     }
 }
 
-// Cross-based aggregation (seq/CrossBasedAggregation.cpp:127-169).
-__global__ void k_cross_aggr(const float *__restrict__ pre, float *__restrict__ out, const int *__restrict__ hr,
-                             const int *__restrict__ ht, const int *__restrict__ vr, const int *__restrict__ vt, int H,
-                             int W, int D) {
-    const int y = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * D) return;
-    const int x = i / D, d = i - x * D;
-    const int xt = tar_col(x, d, W, 1);
-    const long p = (long)y * W + x, q = (long)y * W + xt;
-    const int t = imin(vr[2 * p], vt[2 * q]);
-    const int b = imin(vr[2 * p + 1], vt[2 * q + 1]);
-    float sum = 0.f;
-    int cnt = 0;
-    for (int yy = y - t; yy <= y + b; yy++) {
-        if (yy < 0 || yy >= H) continue;
-        const long pr = (long)yy * W + x, pt = (long)yy * W + xt;
-        const int l = imin(hr[2 * pr], ht[2 * pt]);
-        const int r = imin(hr[2 * pr + 1], ht[2 * pt + 1]);
-        int xl = x - l - 1, xrr = x + r;
-        if (xl < 0) xl = 0;  // :153-156 the clamped pixel is excluded from the sum, still counted
-        else if (xrr >= W) xrr = W - 1;
-        if (xl >= 0 && xrr < W && xl < W && xrr >= 0) {  // :157, always true for arms made by findCross
-            const float *row = pre + (size_t)yy * W * D + d;
-            sum = __fadd_rn(sum, __fsub_rn(row[(size_t)xrr * D], row[(size_t)xl * D]));
-            cnt += r + l + 1;
-        }
-    }
-    out[((size_t)p) * D + d] = __fdiv_rn(sum, (float)cnt);
-}
-
 // Adaptive support weights (seq/AdaptiveWeightAggregation.cpp:33-71):
 // w[p][k] = pw[k] * G[|Lab(p)-Lab(q)|^2], 0 outside the image.  G is the
 // host-computed expf(-sqrtf(n)/gamma_s), so the product is the reference's.
@@ -505,7 +474,7 @@ __global__ void k_disp_runs(const uint8_t *__restrict__ in, uint16_t *__restrict
 // words, so that a warp's counters lie in distinct banks whatever the disparities
 // (a slice per thread put all 32 lanes in one bank).  Bound: the chain of
 // dependent shared-memory updates, one per run.  640x480, D = 64, arms near 17:
-// 2114 us with per-thread slices and one update a pixel, 176 us now.
+// 2114 us with per-thread slices and one update a pixel, 136 us now.
 constexpr int kRefT = 64;
 __global__ void __launch_bounds__(kRefT) k_disp_refine(const uint16_t *__restrict__ runs, uint8_t *__restrict__ out,
                                                        const int *__restrict__ horz, const int *__restrict__ vert,
@@ -663,10 +632,6 @@ void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W
 void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D) {
     const long n = (long)H * D;
     k_prefix_h<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(cost, H, W, D);
-}
-void launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
-                       const int *vt, int H, int W, int D) {
-    k_cross_aggr<<<row_grid((long)W * D, H, 256), 256, 0, s>>>(pre, out, hr, ht, vr, vt, H, W, D);
 }
 void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw, const float *g, float *w, int H, int W,
                             int r) {

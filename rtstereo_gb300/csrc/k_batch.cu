@@ -728,7 +728,7 @@ int stage_items(int stage, const ViewDesc &v, int vert_rows) {
     return 0;
 }
 
-static int num_sms() {
+int sm_count() {
     static int n = 0;
     if (!n) {
         int dev = 0;
@@ -818,7 +818,7 @@ rts_status launch_cross_views(rts_ctx *c, const rts_params &p, const ViewTable &
     // record colour word: 2 rank, 1 gray byte, 0 packed RGB
     const int grayrec = rank ? 2 : (mode == 1 && gray) ? 1 : 0;
     cudaStream_t s = c->stream;
-    const int sms = num_sms();
+    const int sms = sm_count();
     auto grid = [&](int items, int per_block, int per_sm) {
         const long need = ((long)items + per_block - 1) / per_block;
         const long cap = tune.persistent ? (long)sms * per_sm : need;

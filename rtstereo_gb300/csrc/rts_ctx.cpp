@@ -26,9 +26,8 @@ rts_status cuda_check(rts_ctx *c, cudaError_t e, const char *what) {
     return set_error(c, RTS_ERR_CUDA, m);
 }
 
-rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out) {
+static rts_status dev_alloc_once(rts_ctx *c, size_t bytes, void **out) {
     *out = nullptr;
-    if (bytes == 0) bytes = 256;
     if (c->budget && c->used + bytes > c->budget)
         return set_error(c, RTS_ERR_OOM, "HBM budget of the context exceeded (" + std::to_string(c->used + bytes) +
                                              " > " + std::to_string(c->budget) + " bytes)");
@@ -39,6 +38,47 @@ rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out) {
     }
     c->used += bytes;
     return RTS_OK;
+}
+
+rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out) {
+    if (bytes == 0) bytes = 256;
+    rts_status s = dev_alloc_once(c, bytes, out);
+    if (s != RTS_ERR_OOM || c->work.empty()) return s;
+    // give the optional scratch back once the device is done with it
+    RTS_CU(c, cudaDeviceSynchronize());
+    for (auto &w : c->work) dev_free(c, w.buf.ptr, w.buf.bytes);
+    c->work.clear();
+    return dev_alloc_once(c, bytes, out);
+}
+
+void *stream_work(rts_ctx *c, size_t bytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    size_t i = 0;
+    while (i < c->work.size() && c->work[i].stream != c->stream) i++;
+    if (i < c->work.size() && c->work[i].buf.bytes >= bytes) return c->work[i].buf.ptr;
+    if (i == c->work.size() && i == kMaxWork) return nullptr;
+    const std::string msg = c->last_error;
+    if (i < c->work.size()) {
+        if (cudaStreamSynchronize(c->stream) != cudaSuccess) return nullptr;
+        dev_free(c, c->work[i].buf.ptr, c->work[i].buf.bytes);
+        c->work.erase(c->work.begin() + i);
+    }
+    StreamWork w;
+    w.stream = c->stream;
+    w.buf.bytes = (bytes + bytes / 8 + 4095) & ~size_t(4095);  // room for slightly larger shapes
+    if (dev_alloc_once(c, w.buf.bytes, &w.buf.ptr) != RTS_OK) {
+        w.buf.bytes = bytes;
+        if (dev_alloc_once(c, w.buf.bytes, &w.buf.ptr) != RTS_OK) {
+            c->last_error = msg;  // not this call's failure
+            return nullptr;
+        }
+    }
+    c->work.push_back(w);
+    return w.buf.ptr;
 }
 
 void dev_free(rts_ctx *c, void *p, size_t bytes) {
@@ -305,6 +345,7 @@ void rts_ctx_destroy(rts_ctx *c) {
         if (b.ptr) cudaFree(b.ptr);
     for (auto &b : c->extra)
         if (b.ptr) cudaFree(b.ptr);
+    for (auto &w : c->work) cudaFree(w.buf.ptr);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }

@@ -43,6 +43,12 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+// Optional scratch of one stream (stream_work).
+struct StreamWork {
+    cudaStream_t stream = nullptr;
+    DevBuf buf;
+};
+
 struct StageTimer {
     std::string name;
     uint64_t launches = 0;
@@ -67,6 +73,7 @@ struct rts_ctx {
     std::recursive_mutex mu;
     rts::DevBuf slots[rts::SL_COUNT];
     std::vector<rts::DevBuf> extra;  // batch / server buffers
+    std::vector<rts::StreamWork> work;  // at most rts::kMaxWork (stream_work)
     // cached host-computed lookup tables (the key is what the table was made for)
     rts::LutKey lut_key[2];
     bool rcp_ready = false;
@@ -99,8 +106,18 @@ rts_status cuda_check(rts_ctx *c, cudaError_t e, const char *what);
 // arena ----------------------------------------------------------------------
 // Returns a device buffer of at least `bytes` for `slot` (grown if needed).
 rts_status scratch(rts_ctx *c, int slot, size_t bytes, void **out);
+// Device memory within the context's budget; optional scratch (stream_work) is given
+// back first where it stands in the way.
 rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out);
 void dev_free(rts_ctx *c, void *p, size_t bytes);
+
+// Optional scratch of the context's current stream, for calls that can also do without
+// (their general kernels need none): at least `bytes`, kept per stream so that calls on
+// different streams of one context do not share it; null where there is no room, on a
+// stream that is being captured (a graph would keep the address) or past kMaxWork
+// streams.
+constexpr size_t kMaxWork = 4;
+void *stream_work(rts_ctx *c, size_t bytes);
 
 // host <-> device staging for RTS_HOST calls -------------------------------
 // Input: returns a device pointer holding `bytes` from `src` (copied if HOST).
@@ -148,6 +165,9 @@ rts_status lab_weight_lut(rts_ctx *c, float gamma_s, const float **g);
 // proximity weights pw[k] (seq/AdaptiveWeightAggregation.cpp:11-18), device copy
 rts_status prox_weights(rts_ctx *c, float gamma_p, int rad, const float **pw);
 void host_prox_weight(float *pw, float gamma_p, int rad);
+
+// SMs of the current device (k_batch.cu)
+int sm_count();
 
 // ---------------------------------------------------------------------------
 // kernel launchers (defined in the .cu files); all enqueue on `s`.
@@ -197,8 +217,12 @@ void launch_find_cross(cudaStream_t s, const uint8_t *rgb, int *horz, int *vert,
 inline bool median_ksize_ok(int k) { return k >= 3 && k <= 15 && (k & 1); }
 void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W, int ch, int k);
 void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D);
-void launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
-                       const int *vt, int H, int W, int D);
+// k_cross_mod.cu: work: cross_aggr_bytes() of scratch, or null (the general kernel
+// alone); returns the kernels launched
+size_t cross_aggr_bytes(int H, int W, int D);
+int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
+                      const int *vt, int H, int W, int D, void *work);
+// k_aggr.cu
 void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw, const float *g, float *w, int H,
                             int W, int r);
 void launch_aw_l2r_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,

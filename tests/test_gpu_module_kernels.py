@@ -28,3 +28,38 @@ def test_disp_refinement(ctx, oracle_mod, H, W, D, arm):
                  rng.integers(0, 256, (H, W))):  # votes at or above D count for nothing
         disp = np.ascontiguousarray(disp.astype(np.uint8))
         assert bits_equal(ctx.disp_refinement(disp, horz, vert, D), O.disp_refinement(disp, horz, vert, D))
+
+
+def patches_pair(seed, H, W):
+    a, b = patches(seed, H, W), patches(seed + 100, H, W)
+    b[:, : W // 2] = np.roll(a, 3, 1)[:, : W // 2]  # half of it matches: arms of both lengths
+    return a, b
+
+
+# one chunk, ragged chunks, strips (64 rows and more of few columns), one row and column; arms above
+# kModArm = 20 and foreign arms (outside the image, negative) take the general kernel
+@pytest.mark.parametrize("H,W,D", [(1, 1, 1), (6, 33, 32), (131, 40, 33), (200, 9, 5), (50, 300, 70), (9, 257, 256)])
+@pytest.mark.parametrize("arm", [0, 17, 20, 21])
+def test_cross_aggregation(ctx, oracle_mod, H, W, D, arm):
+    O = oracle_mod
+    a, b = patches_pair(H + W, H, W)
+    ha, va = ctx.findCross(a, arm, 20)
+    hb, vb = ctx.findCross(b, arm, 20)
+    assert bits_equal(ha, O.find_cross(a, arm, 20)[0]) and bits_equal(va, O.find_cross(a, arm, 20)[1])
+    cost = np.random.default_rng(D).normal(0.5, 1.0, (H, W, D)).astype(np.float32)  # sums of either sign
+    pre = ctx.aggregate_cost_horizontal(cost)
+    want = O.prefix_h(cost)
+    assert bits_equal(pre, want)
+    assert bits_equal(ctx.cross_stereo_aggregation(pre, ha, hb, va, vb), O.cross_aggr(want, ha, hb, va, vb))
+
+
+def test_cross_aggregation_foreign_arms(ctx, oracle_mod):
+    """Arms that leave the image go to the general kernel, whatever image they are in."""
+    H, W, D = 20, 50, 12
+    a, b = patches_pair(3, H, W)
+    (ha, va), (hb, vb) = ctx.findCross(a, 17, 20), ctx.findCross(b, 17, 20)
+    pre = ctx.aggregate_cost_horizontal(np.random.default_rng(1).random((H, W, D), dtype=np.float32))
+    for arr, at, v in ((ha, (0, 0, 0), 5), (hb, (3, 7, 1), 60), (va, (H - 1, 4, 1), 2), (vb, (2, 2, 0), 19)):
+        arms = [x.copy() for x in (ha, hb, va, vb)]
+        arms[[id(ha), id(hb), id(va), id(vb)].index(id(arr))][at] = v
+        assert bits_equal(ctx.cross_stereo_aggregation(pre, *arms), oracle_mod.cross_aggr(pre, *arms))
