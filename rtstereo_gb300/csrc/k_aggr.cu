@@ -371,20 +371,6 @@ __global__ void k_find_cross(const uint8_t *__restrict__ rgb, int *__restrict__ 
     horz[2 * p + 1] = cross_arm(rgb, p, 1, W - 1 - x, L, tau);
 }
 
-// In-place running sum along x per (y, d) (seq/CrossBasedAggregation.cpp:117-125):
-// one thread per chain, consecutive threads on consecutive d (coalesced).
-__global__ void k_prefix_h(float *__restrict__ cost, int H, int W, int D) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)H * D) return;
-    const int y = (int)(i / D), d = (int)(i - (long)y * D);
-    float *p = cost + (size_t)y * W * D + d;
-    float acc = p[0];
-    for (int x = 1; x < W; x++) {
-        acc = __fadd_rn(p[(size_t)x * D], acc);
-        p[(size_t)x * D] = acc;
-    }
-}
-
 // Adaptive support weights (seq/AdaptiveWeightAggregation.cpp:33-71):
 // w[p][k] = pw[k] * G[|Lab(p)-Lab(q)|^2], 0 outside the image.  G is the
 // host-computed expf(-sqrtf(n)/gamma_s), so the product is the reference's.
@@ -628,10 +614,6 @@ void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W
     const size_t smem = (size_t)(kMedTX + 2 * r) * (kMedTY + 2 * r) * 4;
     if (ch == 3) k_median<3><<<g, b, smem, s>>>(in, out, H, W, r);
     else k_median<1><<<g, b, smem, s>>>(in, out, H, W, r);
-}
-void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D) {
-    const long n = (long)H * D;
-    k_prefix_h<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(cost, H, W, D);
 }
 void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw, const float *g, float *w, int H, int W,
                             int r) {

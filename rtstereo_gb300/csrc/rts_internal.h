@@ -216,8 +216,9 @@ void launch_find_cross(cudaStream_t s, const uint8_t *rgb, int *horz, int *vert,
 // per-channel median of the k x k window, borders replicated (ch 1 or 3)
 inline bool median_ksize_ok(int k) { return k >= 3 && k <= 15 && (k & 1); }
 void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W, int ch, int k);
+// k_cross_mod.cu
 void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D);
-// k_cross_mod.cu: work: cross_aggr_bytes() of scratch, or null (the general kernel
+// work: cross_aggr_bytes() of scratch, or null (the general kernel
 // alone); returns the kernels launched
 size_t cross_aggr_bytes(int H, int W, int D);
 int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,

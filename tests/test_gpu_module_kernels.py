@@ -63,3 +63,25 @@ def test_cross_aggregation_foreign_arms(ctx, oracle_mod):
         arms = [x.copy() for x in (ha, hb, va, vb)]
         arms[[id(ha), id(hb), id(va), id(vb)].index(id(arr))][at] = v
         assert bits_equal(ctx.cross_stereo_aggregation(pre, *arms), oracle_mod.cross_aggr(pre, *arms))
+
+
+# rows shorter than a warp's 32 pixels, warps that end a row, a ragged last warp; rows without a winner
+@pytest.mark.parametrize("H,W,D", [(1, 1, 1), (7, 3, 3), (5, 33, 32), (9, 40, 33), (3, 299, 256), (40, 64, 2)])
+def test_wta(ctx, oracle_mod, H, W, D):
+    O = oracle_mod
+    rng = np.random.default_rng(H * W + D)
+    cost = rng.integers(0, 6, (H, W, D)).astype(np.float32)  # ties
+    cost[rng.random((H, W)) < 0.3, 0] = -1.0                 # no winner of their own: carried
+    cost[H // 2] = 0.0                                       # a whole row carried
+    special = rng.random((H, W, D)) < 0.03
+    cost[special] = rng.choice(np.array([np.nan, np.inf, -np.inf, -0.0, 3.4028235e38], np.float32), special.sum())
+    assert bits_equal(ctx.WTA(cost), O.wta(cost))
+    assert bits_equal(ctx.WTA_NCC(cost), O.wta(cost, True))
+
+
+# batches of 32 columns: shorter, exact, one more; chains across a block's end
+@pytest.mark.parametrize("H,W,D", [(1, 1, 1), (3, 31, 5), (2, 32, 33), (5, 33, 64), (1, 65, 256), (70, 100, 3)])
+def test_prefix(ctx, oracle_mod, H, W, D):
+    cost = np.random.default_rng(W).normal(0.0, 1.0, (H, W, D)).astype(np.float32)
+    cost[0, 0, 0] = -0.0
+    assert bits_equal(ctx.aggregate_cost_horizontal(cost), oracle_mod.prefix_h(cost))
