@@ -6,8 +6,8 @@
 // (raster order, across rows).  On the GPU this is two passes:
 //   1. k_wta_local: per pixel, the first strict arg-min (arg-max) and whether
 //      any d >= 1 won ("found"); found pixels raise row_last[y] to their x.
-//      Warp per pixel, lane = disparity, so a warp reads its pixel's D costs
-//      as whole lines; the winner is the least {wta_key, d};
+//      Lane = disparity, so a warp reads a pixel's D costs as whole lines; the
+//      winner is the least {wta_key, d};
 //   2. k_wta_fill: one warp per row takes the incoming winner from the nearest
 //      earlier row that has a found pixel, then propagates within the row with
 //      a ballot scan.
@@ -19,24 +19,32 @@
 
 namespace rts {
 
-constexpr int kWtaWarps = 8, kWtaPix = 4;  // warps of a block; pixels of a warp at a time
+// Pass 1: a warp takes kWtaPix consecutive pixels at a time, every pixel's loads of a
+// 32-disparity step in flight together, 32 pixels in all; lane i keeps pixel i's
+// winner, so winners leave as one line and a row's last winner as one atomic per warp
+// (one lane's store, division and atomic per pixel made half of the instructions:
+// 640x480, D = 64 104 us; 37 us now).  Bound: instruction issue (the two reductions and the keys).
+constexpr int kWtaWarps = 8, kWtaPix = 8;
 __global__ void __launch_bounds__(kWtaWarps * 32) k_wta_local(const float *__restrict__ cost, uint16_t *__restrict__ raw,
                                                               int *__restrict__ row_last, int H, int W, int D,
                                                               int argmax) {
     const int lane = threadIdx.x & 31;
     const long np = (long)H * W;
-    // resident blocks stride over the pixels, a warp kWtaPix consecutive pixels at a
-    // time, every pixel's loads of a 32-disparity step in flight together
-    const long stride = (long)gridDim.x * kWtaWarps * kWtaPix;
-    for (long p0 = ((long)blockIdx.x * kWtaWarps + (threadIdx.x >> 5)) * kWtaPix; p0 < np; p0 += stride) {
+    const long p0 = ((long)blockIdx.x * kWtaWarps + (threadIdx.x >> 5)) * 32;
+    if (p0 >= np) return;
+    const int n = (int)(np - p0 < 32 ? np - p0 : 32);
+    const float *row = cost + p0 * D + lane;
+    uint32_t mine = 0;  // the winner of pixel p0 + lane
+#pragma unroll 1
+    for (int i0 = 0; i0 < n; i0 += kWtaPix, row += (size_t)kWtaPix * D) {
         uint32_t bk[kWtaPix], bd[kWtaPix];
 #pragma unroll
         for (int j = 0; j < kWtaPix; j++) bk[j] = bd[j] = 0xffffffffu;
 #pragma unroll 2
-        for (int d = lane; d < D; d += 32) {
+        for (int d = lane, o = 0; d < D; d += 32, o += 32) {
             float v[kWtaPix];
 #pragma unroll
-            for (int j = 0; j < kWtaPix; j++) v[j] = __ldg(cost + (p0 + j < np ? p0 + j : np - 1) * D + d);
+            for (int j = 0; j < kWtaPix; j++) v[j] = __ldg(row + (size_t)(i0 + j < n ? j : n - 1 - i0) * D + o);
 #pragma unroll
             for (int j = 0; j < kWtaPix; j++) {
                 const uint32_t k = wta_key(v[j], d, argmax);
@@ -50,14 +58,18 @@ __global__ void __launch_bounds__(kWtaWarps * 32) k_wta_local(const float *__res
         for (int j = 0; j < kWtaPix; j++) {
             const uint32_t mn = __reduce_min_sync(0xffffffffu, bk[j]);
             const uint32_t win = __reduce_min_sync(0xffffffffu, bk[j] == mn ? bd[j] : 0xffffffffu);
-            const long p = p0 + j;
-            if (lane == 0 && p < np) {
-                const bool found = win != 0;  // some d >= 1 strictly better than d = 0
-                raw[p] = found ? (uint16_t)(0x100 | win) : (uint16_t)0;
-                if (found) atomicMax(row_last + p / W, (int)(p % W));
-            }
+            if (lane == i0 + j) mine = win;
         }
     }
+    const bool found = lane < n && mine != 0;  // some d >= 1 strictly better than d = 0
+    const int y0 = (int)(p0 / W), x0 = (int)(p0 - (long)y0 * W) + lane;
+    const int y = y0 + x0 / W, x = x0 % W;
+    if (lane < n) raw[p0 + lane] = found ? (uint16_t)(0x100 | mine) : (uint16_t)0;
+    // the last found pixel of each row the warp meets
+    const uint32_t fm = __ballot_sync(0xffffffffu, found);
+    const uint32_t later = lane < 31 ? fm >> (lane + 1) : 0u;
+    const int ny = __shfl_sync(0xffffffffu, y, later ? lane + __ffs(later) : lane);
+    if (found && (!later || ny != y)) atomicMax(row_last + y, x);
 }
 
 __global__ void k_wta_fill(const uint16_t *__restrict__ raw, const int *__restrict__ row_last,
@@ -125,16 +137,9 @@ __global__ void k_flip(const uint8_t *__restrict__ in, uint8_t *__restrict__ out
 
 void launch_wta_local(cudaStream_t s, const float *cost, uint16_t *raw, int *row_last, int H, int W, int D,
                       int argmax) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 132;
-    }
-    const long np = (long)H * W, per_block = (long)kWtaWarps * kWtaPix;
-    const long blocks = std::min((np + per_block - 1) / per_block, (long)sms * 8);
-    k_wta_local<<<(unsigned)blocks, kWtaWarps * 32, 0, s>>>(cost, raw, row_last, H, W, D, argmax);
+    const long per_block = 32L * kWtaWarps;
+    k_wta_local<<<(unsigned)(((long)H * W + per_block - 1) / per_block), kWtaWarps * 32, 0, s>>>(cost, raw, row_last, H,
+                                                                                               W, D, argmax);
 }
 void launch_wta_diag(cudaStream_t s, const float *vol, uint16_t *raw, int *row_last, int H, int W, int D) {
     k_wta_diag<<<dim3((W + kDiagT - 1) / kDiagT, H), kDiagT, 0, s>>>(vol, raw, row_last, W, D);
