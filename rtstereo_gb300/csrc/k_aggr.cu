@@ -330,6 +330,128 @@ __global__ void __launch_bounds__(256, 2) k_box_best_dp(const __grid_constant__ 
     box_dp_tile<R, POS, RV>(bt2, best, best_r, H, W, D, argmax, rcp_area, x0, y0, d);
 }
 
+// Box mean to a volume (radius 1..8): block per (16 x 8 pixel tile, 32 DW disparities),
+// the tile and its R-pixel wrapped border staged once, a lane on DW adjacent
+// disparities, a warp on one tile row of 16 pixels; each sum is the reference's single
+// chain, rows outer and columns inner.  DW = 2 (D above 32) adds the pair by packed
+// f32x2 instructions; DW = 1 leaves no half of a warp idle at D <= 32.  Inner tiles
+// arrive by TMA as in k_box_best_dp; others, and volumes TMA does not take, by
+// cp.async (8 bytes a lane where `wide`: even D and an 8-byte aligned volume).
+// Bound: the FP32 pipe ((2R+1)^2 adds per entry); k_box, which reads every window cell
+// from L1, took 3240 us at 1280x720, D = 64, R = 4; this one 181 us.
+template <int R, int DW>
+__global__ void __launch_bounds__(256, DW == 1 ? 3 : 2)
+    k_box_vol(const __grid_constant__ CUtensorMap tmap, int use_tma, const float *__restrict__ vol,
+              float *__restrict__ out, int H, int W, int D, int wide, float rcp_area) {
+    constexpr int TW = kBoxDpTX + 2 * R, TH = kBoxDpTY + 2 * R, AREA = (2 * R + 1) * (2 * R + 1), CD = 32 * DW;
+    constexpr int G = kBoxDpTX;
+    extern __shared__ __align__(128) float bv[];  // [TH][TW][CD]
+    __shared__ __align__(8) uint64_t bar;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int x0 = blockIdx.x * kBoxDpTX, y0 = blockIdx.y * kBoxDpTY, d = blockIdx.z * CD + DW * lane;
+    const bool inner = x0 >= R && x0 + kBoxDpTX + R <= W;
+    const bool tma = use_tma && inner && y0 >= R && y0 + kBoxDpTY + R <= H &&
+                     ((uint32_t)__cvta_generic_to_shared(bv) & 127) == 0;
+    if (tma) {
+        const uint32_t ba = (uint32_t)__cvta_generic_to_shared(&bar);
+        if (threadIdx.x == 0) mbar_init(ba);
+        __syncthreads();
+        if (threadIdx.x == 0)
+            tma_load_3d((uint32_t)__cvta_generic_to_shared(bv), &tmap, (int)blockIdx.z * CD, x0 - R, y0 - R, ba,
+                        (uint32_t)(TW * TH * CD * sizeof(float)));
+        // the block decides together, so that no thread waits at a later barrier
+        if (__syncthreads_or(!mbar_wait(ba, 0))) {
+            if (threadIdx.x == 0) atomicAdd(&g_box_tma_timeouts, 1);
+            mbar_wait(ba, 0);  // the copy may still land in this block's shared memory
+            return;
+        }
+    } else {
+        // single wrap as in seq/ConstBlockAggregation.cpp:19-24; cells past the last pixel's
+        // window are clamped into range (never read); zero fill past D
+        for (int i = warp; i < TH; i += 8) {
+            const int yy = wrap1(imin(y0 - R + i, H - 1 + R), H);
+            const float *rowp = vol + (size_t)yy * W * D;
+            uint32_t dst = (uint32_t)__cvta_generic_to_shared(bv + i * TW * CD + DW * lane);
+#pragma unroll 4
+            for (int j = 0; j < TW; j++, dst += 4 * CD) {
+                const int xx = wrap1(imin(x0 - R + j, W - 1 + R), W);
+                const float *src = rowp + (size_t)xx * D;
+                if (DW == 2 && wide) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src + (d < D ? d : 0)),
+                                 "r"(d < D ? 8 : 0)
+                                 : "memory");
+                } else {
+#pragma unroll
+                    for (int h = 0; h < DW; h++)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst + 4 * h),
+                                     "l"(src + (d + h < D ? d + h : 0)), "r"(d + h < D ? 4 : 0)
+                                     : "memory");
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+    }
+    const int y = y0 + warp;
+    if (y >= H) return;
+    // mean = sum / AREA correctly rounded (seq/ConstBlockAggregation.cpp:31): Markstein's
+    // correction in the range where it is exact (box_dp_tile), else the division itself
+    auto mean = [&](float sm) {
+        const float a = fabsf(sm);
+        if (a >= 0x1p-100f && a <= 0x1p+126f) {
+            const float q0 = __fmul_rn(sm, rcp_area);
+            return __fmaf_rn(__fmaf_rn(-(float)AREA, q0, sm), rcp_area, q0);
+        }
+        return __fdiv_rn(sm, (float)AREA);
+    };
+    float *op = out + ((size_t)y * W + x0) * D + d;
+    if constexpr (DW == 2) {
+        float2 sum[G];
+#pragma unroll
+        for (int m = 0; m < G; m++) sum[m] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int dy = 0; dy <= 2 * R; dy++) {
+            const float2 *rp = reinterpret_cast<const float2 *>(bv) + (warp + dy) * TW * 32 + lane;
+            float2 v[TW];
+#pragma unroll
+            for (int k = 0; k < TW; k++) v[k] = rp[k * 32];
+#pragma unroll
+            for (int m = 0; m < G; m++)
+#pragma unroll
+                for (int dx = 0; dx <= 2 * R; dx++) sum[m] = __fadd2_rn(sum[m], v[m + dx]);
+        }
+#pragma unroll
+        for (int m = 0; m < G; m++, op += D) {
+            if (x0 + m >= W) break;
+            const float2 q = make_float2(mean(sum[m].x), mean(sum[m].y));
+            if ((D & 1) == 0 && d < D) {
+                *reinterpret_cast<float2 *>(op) = q;  // the scratch volume is 256-byte aligned
+            } else {
+                if (d < D) op[0] = q.x;
+                if (d + 1 < D) op[1] = q.y;
+            }
+        }
+    } else {
+        float sum[G];
+#pragma unroll
+        for (int m = 0; m < G; m++) sum[m] = 0.f;
+#pragma unroll
+        for (int dy = 0; dy <= 2 * R; dy++) {
+            const float *rp = bv + (warp + dy) * TW * 32 + lane;
+            float v[TW];
+#pragma unroll
+            for (int k = 0; k < TW; k++) v[k] = rp[k * 32];
+#pragma unroll
+            for (int m = 0; m < G; m++)
+#pragma unroll
+                for (int dx = 0; dx <= 2 * R; dx++) sum[m] = __fadd_rn(sum[m], v[m + dx]);
+        }
+#pragma unroll
+        for (int m = 0; m < G; m++, op += D)
+            if (x0 + m < W && d < D) *op = mean(sum[m]);
+    }
+}
+
 // per-pixel minimum -> WTA winner word and row summary (see k_wta.cu)
 // (mirror: raw and row_last in the mirrored columns of a right view)
 __global__ void k_best_raw(const unsigned long long *__restrict__ best, uint16_t *__restrict__ raw,
@@ -550,6 +672,34 @@ __global__ void __launch_bounds__(kMedTX *kMedTY)
 static dim3 row_grid(long per_row, int H, int threads) { return dim3((unsigned)((per_row + threads - 1) / threads), H); }
 
 void launch_box(cudaStream_t s, const float *in, float *out, int H, int W, int D, int r) {
+    // the tiled kernel up to the radius whose tile fits shared memory
+    const int dw = D > 32 ? 2 : 1;
+    auto go = [&](auto kern, int R) {
+        const int area = (2 * R + 1) * (2 * R + 1);
+        const size_t smem = (size_t)(kBoxDpTX + 2 * R) * (kBoxDpTY + 2 * R) * 32 * dw * sizeof(float);
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        CUtensorMap tm{};
+        const int use_tma = volume_tensor_map(&tm, in, H, W, D, 4, 32 * dw, kBoxDpTX + 2 * R, kBoxDpTY + 2 * R) ? 1 : 0;
+        const int wide = D % 2 == 0 && ((uintptr_t)in & 7) == 0 ? 1 : 0;
+        const dim3 g((W + kBoxDpTX - 1) / kBoxDpTX, (H + kBoxDpTY - 1) / kBoxDpTY, (D + 32 * dw - 1) / (32 * dw));
+        kern<<<g, 256, smem, s>>>(tm, use_tma, in, out, H, W, D, wide, 1.0f / (float)area);
+    };
+#define RTS_BOXV(RR)                                \
+    case RR:                                        \
+        if (dw == 2) go(k_box_vol<RR, 2>, RR);      \
+        else go(k_box_vol<RR, 1>, RR);              \
+        return;
+    switch (r) {
+        RTS_BOXV(1)
+        RTS_BOXV(2)
+        RTS_BOXV(3)
+        RTS_BOXV(4)
+        RTS_BOXV(5)
+        RTS_BOXV(6)
+        RTS_BOXV(7)
+        RTS_BOXV(8)
+    }
+#undef RTS_BOXV
     k_box<<<row_grid((long)W * D, H, 256), 256, 0, s>>>(in, out, H, W, D, r);
 }
 bool box_best_supported(int r) { return r >= 1 && r <= 8; }

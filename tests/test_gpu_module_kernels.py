@@ -85,3 +85,19 @@ def test_prefix(ctx, oracle_mod, H, W, D):
     cost = np.random.default_rng(W).normal(0.0, 1.0, (H, W, D)).astype(np.float32)
     cost[0, 0, 0] = -0.0
     assert bits_equal(ctx.aggregate_cost_horizontal(cost), oracle_mod.prefix_h(cost))
+
+
+# both lane widths, odd and ragged disparities, tiles inside (TMA where D % 4 == 0) and at the wrap,
+# the smallest and largest tiled radius, radius 9 and 0 (untiled)
+@pytest.mark.parametrize("H,W,D,r", [(10, 11, 1, 1), (40, 70, 32, 4), (41, 50, 33, 4), (33, 67, 64, 2), (40, 60, 68, 8),
+                                     (25, 45, 130, 3), (20, 30, 31, 8), (24, 50, 12, 5), (21, 40, 9, 9), (5, 6, 40, 0)])
+def test_box(ctx, oracle_mod, H, W, D, r):
+    rng = np.random.default_rng(D * r)
+    cost = rng.normal(0.2, 1.0, (H, W, D)).astype(np.float32)
+    assert bits_equal(ctx.boxAggregate(cost, r), oracle_mod.box(cost, r))
+    cost[rng.random(cost.shape) < 0.9] = 0.0  # zero and tiny sums, then infinite and NaN ones
+    cost *= np.float32(1e-37)
+    cost[rng.random(cost.shape) < 0.001] = np.inf
+    cost[rng.random(cost.shape) < 0.001] = -np.inf
+    got, want = ctx.boxAggregate(cost, r), oracle_mod.box(cost, r)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and bits_equal(np.nan_to_num(got), np.nan_to_num(want))
