@@ -5,59 +5,111 @@
 // Float arithmetic that must match the reference bit for bit is written with
 // explicit round-to-nearest intrinsics in the reference's order; the library
 // is compiled with -fmad=false so no multiply-add is fused behind our back.
+#include <algorithm>
+
 #include "rts_common.cuh"
 
 namespace rts {
 
 // ---------------------------------------------------------------------------
-// Absolute differences.  Grid: x-blocks over W*D of one row, y over rows; the
-// cost volume is written with d fastest, so consecutive threads store
-// consecutive floats.
-
-template <typename T>
-__global__ void k_ad_1ch(const T *__restrict__ ref, const T *__restrict__ tar, float *__restrict__ cost, int D,
-                         int H, int W, int dir) {
-    const int y = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * D) return;
-    const int x = i / D, d = i - x * D;
-    const int xt = tar_col(x, d, W, dir);
-    const size_t row = (size_t)y * W;
-    float v;
-    if constexpr (sizeof(T) == 1) {
-        // seq/PixelBasedCost.cpp:22 abs of an int difference
-        v = (float)abs((int)ref[row + x] - (int)tar[row + xt]);
-    } else {
-        // seq/PixelBasedCost.cpp:48-50 float difference then sign flip
-        v = __fsub_rn(ref[row + x], tar[row + xt]);
-        if (v < 0) v = -v;
+// Cost volumes from two images: cost[y][x][d] = K::cost(ref word of x, target word of
+// x -+ d).  Block per (row, kRowTX pixels): the words of the pixels and of every target
+// column they meet (wrapped once, D <= W) are made once in shared memory, then the
+// block's kRowTX D consecutive entries are written in order, a line of 32 per warp and
+// step.  magic = ceil(2^20 / D): i / D for i below 16 * 256 (the error is below 1 / 256,
+// at most 1 / D), so each half of the block has indices of its own.
+// Bound: instruction issue, then the volume's write (a division, two dependent image
+// reads and byte loads per entry before: colour AD 640x480, D = 64 79 us; 30 us now).
+constexpr int kRowTX = 32;
+template <typename K>
+__global__ void __launch_bounds__(256) k_cost_rows(K k, float *__restrict__ cost, int D, int W, int dir,
+                                                   uint32_t magic) {
+    using T = typename K::T;
+    __shared__ T ref[kRowTX], tar[kRowTX + 255];
+    const int tid = threadIdx.x, x0 = blockIdx.x * kRowTX;
+    const size_t row = (size_t)blockIdx.y * W;
+    const int t0 = dir > 0 ? x0 - D + 1 : x0;  // target column of tar[0]
+    for (int i = tid; i < kRowTX + D - 1; i += 256) {
+        int xt = t0 + i;
+        if (xt < 0) xt += W;                                  // seq/PixelBasedCost.cpp:19-20
+        else if (dir < 0 && xt >= W) xt -= W;                 // :32-33
+        tar[i] = k.load_tar(row + imin(xt, W - 1));           // columns of no pixel are clamped
     }
-    cost[(row + x) * D + d] = v;
+    if (tid < kRowTX) ref[tid] = k.load_ref(row + imin(x0 + tid, W - 1));
+    __syncthreads();
+    const int n = imin(kRowTX, W - x0) * D, half = kRowTX / 2 * D;
+    float *out = cost + (row + x0) * D;
+#pragma unroll 2
+    for (int i = tid; i < n; i += 256) {
+        const int up = i >= half ? kRowTX / 2 : 0, j = i - (up ? half : 0);
+        const int px = (int)(((uint32_t)j * magic) >> 20), d = j - px * D, x = px + up;
+        out[i] = k.cost(ref[x], tar[dir > 0 ? x + D - 1 - d : x + d]);
+    }
 }
 
-__global__ void k_ad_color(const uint8_t *__restrict__ ref, const uint8_t *__restrict__ tar,
-                           float *__restrict__ cost, int D, int H, int W, int dir, int use_trunc, float trunc,
-                           int norm) {
-    const int y = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * D) return;
-    const int x = i / D, d = i - x * D;
-    const int xt = tar_col(x, d, W, dir);
-    const size_t row = (size_t)y * W;
-    const uint8_t *a = ref + 3 * (row + x);
-    const uint8_t *b = tar + 3 * (row + xt);
-    const int sad = abs((int)a[0] - (int)b[0]) + abs((int)a[1] - (int)b[1]) + abs((int)a[2] - (int)b[2]);
-    // seq/PixelBasedCost.cpp:86-91,106-112: min(sad, trunc), then (float)1/(float)3 * v
-    float v = (float)sad;
-    if (use_trunc) v = (v > trunc) ? trunc : v;
-    if (norm) v = __fmul_rn(1.0f / 3.0f, v);
-    cost[(row + x) * D + d] = v;
-}
+// seq/PixelBasedCost.cpp:22 abs of an int difference
+struct CostGray {
+    using T = uint32_t;
+    const uint8_t *r, *t;
+    __device__ T load_ref(size_t p) const { return r[p]; }
+    __device__ T load_tar(size_t p) const { return t[p]; }
+    __device__ float cost(T a, T b) const { return (float)abs((int)a - (int)b); }
+};
+// seq/PixelBasedCost.cpp:48-50 float difference then sign flip
+struct CostFloat {
+    using T = float;
+    const float *r, *t;
+    __device__ T load_ref(size_t p) const { return r[p]; }
+    __device__ T load_tar(size_t p) const { return t[p]; }
+    __device__ float cost(T a, T b) const {
+        const float v = __fsub_rn(a, b);
+        return v < 0 ? -v : v;
+    }
+};
+// seq/PixelBasedCost.cpp:86-91,106-112: min(sad, trunc), then (float)1/(float)3 * v
+struct CostColor {
+    using T = uint32_t;  // packed RGB
+    const uint8_t *r, *t;
+    int use_trunc, norm;
+    float trunc;
+    static __device__ T pack(const uint8_t *q) {
+        return (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16);
+    }
+    __device__ T load_ref(size_t p) const { return pack(r + 3 * p); }
+    __device__ T load_tar(size_t p) const { return pack(t + 3 * p); }
+    __device__ float cost(T a, T b) const {
+        float v = (float)__vsadu4(a, b);
+        if (use_trunc) v = (v > trunc) ? trunc : v;
+        return norm ? __fmul_rn(1.0f / 3.0f, v) : v;
+    }
+};
+// seq/CensusTransform.cpp:60, from packed codes of NW words
+template <int NW> struct CostHamming {
+    struct T {
+        uint64_t w[NW];
+    };
+    const uint64_t *r, *t;
+    static __device__ T load(const uint64_t *c, size_t p) {
+        T v;
+#pragma unroll
+        for (int j = 0; j < NW; j++) v.w[j] = c[p * NW + j];
+        return v;
+    }
+    __device__ T load_ref(size_t p) const { return load(r, p); }
+    __device__ T load_tar(size_t p) const { return load(t, p); }
+    __device__ float cost(const T &a, const T &b) const {
+        int cnt = 0;
+#pragma unroll
+        for (int j = 0; j < NW; j++) cnt += __popcll(a.w[j] ^ b.w[j]);
+        return (float)cnt;
+    }
+};
 
 // ---------------------------------------------------------------------------
 // Census.  Module form writes the reference's bool layout, one byte per bit;
 // the pipeline uses packed 64-bit words (bit k of the window in word k/64).
 
+// any window: a thread per bit
 __global__ void k_census_bits(const uint8_t *__restrict__ img, uint8_t *__restrict__ bits, int hr, int wr, int H,
                               int W) {
     const int y = blockIdx.y;
@@ -69,6 +121,47 @@ __global__ void k_census_bits(const uint8_t *__restrict__ img, uint8_t *__restri
     const uint8_t c = img[(size_t)y * W + x];
     const uint8_t n = img[(size_t)wrap1(y + dy, H) * W + wrap1(x + dx, W)];
     bits[((size_t)y * W + x) * nb + k] = (c > n) ? 1 : 0;  // seq/CensusTransform.cpp:31 strict
+}
+
+// Windows of up to kBitsMax bits: block per 128 consecutive pixels (of all rows), a
+// thread per pixel.  The pixel's bytes go to shared memory, then the block's 128 nb
+// bytes leave as 16-byte lines (`wide`: a 16-byte aligned output; 128 nb is a multiple
+// of 16, so every block then starts on one).  Bound: the window's reads (one byte
+// load and compare a bit; two divisions a bit before: 640x480, 9x7 72 us an image; 19 us
+// now).
+constexpr int kBitsT = 128, kBitsMax = 256;
+__global__ void __launch_bounds__(kBitsT) k_census_bits_px(const uint8_t *__restrict__ img, uint8_t *__restrict__ bits,
+                                                           int hr, int wr, int H, int W, int wide) {
+    extern __shared__ __align__(16) uint8_t sb[];  // [128][nb]
+    const int nb = (2 * hr + 1) * (2 * wr + 1), tid = threadIdx.x;
+    const long np = (long)H * W, p0 = (long)blockIdx.x * kBitsT, p = p0 + tid;
+    if (p < np) {
+        const int y = (int)(p / W), x = (int)(p - (long)y * W);
+        const uint8_t c = img[p];
+        uint8_t *o = sb + tid * nb;
+        if (x >= wr && x < W - wr && y >= hr && y < H - hr) {
+            // the window inside the image: no wrapping
+            const uint8_t *row = img + p - (size_t)hr * W - wr;
+            for (int dy = -hr; dy <= hr; dy++, row += W)
+#pragma unroll 7
+                for (int dx = 0; dx <= 2 * wr; dx++) *o++ = c > row[dx] ? 1 : 0;
+        } else {
+            for (int dy = -hr; dy <= hr; dy++) {
+                const uint8_t *row = img + (size_t)wrap1(y + dy, H) * W;
+                for (int dx = -wr; dx <= wr; dx++) *o++ = c > row[wrap1(x + dx, W)] ? 1 : 0;
+            }
+        }
+    }
+    __syncthreads();
+    const int n = (int)(np - p0 < kBitsT ? np - p0 : kBitsT) * nb;
+    uint8_t *out = bits + (size_t)p0 * nb;
+    int i = 0;
+    if (wide) {
+        for (int q = tid; q < n / 16; q += kBitsT)
+            reinterpret_cast<uint4 *>(out)[q] = reinterpret_cast<const uint4 *>(sb)[q];
+        i = n / 16 * 16;
+    }
+    for (i += tid; i < n; i += kBitsT) out[i] = sb[i];
 }
 
 template <int NW>
@@ -102,37 +195,36 @@ __global__ void k_census_codes(const uint8_t *__restrict__ img, uint64_t *__rest
     for (int j = 0; j < NW; j++) codes[((size_t)y * W + x) * NW + j] = w[j];
 }
 
+// The bool layout packed again: block per 128 pixels, their 128 nb bytes staged in
+// shared memory by 16-byte loads (`wide`: a 16-byte aligned input), then a thread per
+// pixel (its own bytes straight from memory are 32 different lines a load; packing and
+// distances 640x480, D = 64: 88 us before, 54 us now).
 template <int NW>
-__global__ void k_bits_pack(const uint8_t *__restrict__ bits, uint64_t *__restrict__ codes, int nb, long npix) {
-    const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npix) return;
-    const uint8_t *b = bits + (size_t)p * nb;
-    uint64_t w[NW];
-#pragma unroll
-    for (int j = 0; j < NW; j++) w[j] = 0;
-    for (int k = 0; k < nb; k++) {
-        const uint64_t bit = b[k] ? 1ull : 0ull;
-#pragma unroll
-        for (int j = 0; j < NW; j++)
-            if ((k >> 6) == j) w[j] |= bit << (k & 63);
+__global__ void __launch_bounds__(kBitsT) k_bits_pack(const uint8_t *__restrict__ bits, uint64_t *__restrict__ codes,
+                                                      int nb, long npix, int wide) {
+    extern __shared__ __align__(16) uint8_t sb[];  // [128][nb]
+    const int tid = threadIdx.x;
+    const long p0 = (long)blockIdx.x * kBitsT;
+    const int np = (int)(npix - p0 < kBitsT ? npix - p0 : kBitsT), n = np * nb;
+    const uint8_t *in = bits + (size_t)p0 * nb;
+    int i = 0;
+    if (wide) {
+        for (int q = tid; q < n / 16; q += kBitsT)
+            reinterpret_cast<uint4 *>(sb)[q] = reinterpret_cast<const uint4 *>(in)[q];
+        i = n / 16 * 16;
     }
+    for (i += tid; i < n; i += kBitsT) sb[i] = in[i];
+    __syncthreads();
+    if (tid >= np) return;
+    const uint8_t *b = sb + tid * nb;
 #pragma unroll
-    for (int j = 0; j < NW; j++) codes[(size_t)p * NW + j] = w[j];
-}
-
-template <int NW>
-__global__ void k_hamming(const uint64_t *__restrict__ cr, const uint64_t *__restrict__ ct, float *__restrict__ cost,
-                          int D, int H, int W) {
-    const int y = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * D) return;
-    const int x = i / D, d = i - x * D;
-    const int xt = tar_col(x, d, W, 1);
-    const size_t row = (size_t)y * W;
-    int cnt = 0;
-#pragma unroll
-    for (int j = 0; j < NW; j++) cnt += __popcll(cr[(row + x) * NW + j] ^ ct[(row + xt) * NW + j]);
-    cost[(row + x) * D + d] = (float)cnt;  // seq/CensusTransform.cpp:60
+    for (int j = 0; j < NW; j++) {
+        uint64_t w = 0;
+        const int e = imin(64, nb - 64 * j);
+#pragma unroll 8
+        for (int k = 0; k < e; k++) w |= (uint64_t)(b[64 * j + k] != 0) << k;
+        codes[(size_t)(p0 + tid) * NW + j] = w;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -341,13 +433,27 @@ __global__ void __launch_bounds__(256) k_cost_log_census(const float *__restrict
     }
 }
 
-__global__ void k_combine(float *__restrict__ c1, const float *__restrict__ c2, long n, const float *__restrict__ lut1,
-                          const float *__restrict__ lut2, float lambda1, float lambda2) {
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const float a = combine_term(c1[i], lut1, lambda1);
-        const float b = combine_term(c2[i], lut2, lambda2);
-        c1[i] = __fadd_rn(a, b);
+// In place, four entries a thread where both volumes are 16-byte aligned (n4 groups of
+// four, then the rest one by one).  Bound: memory (two reads and a write), and for costs
+// that are not whole numbers the expf and division of both terms (640x480, D = 64 whole
+// numbers 79 -> 48 us; 1280x720, D = 64 others 237 -> 140 us).
+__global__ void __launch_bounds__(256) k_combine(float *__restrict__ c1, const float *__restrict__ c2, long n, long n4,
+                                                 const float *__restrict__ lut1, const float *__restrict__ lut2,
+                                                 float lambda1, float lambda2) {
+    const long step = (long)gridDim.x * 256, i0 = (long)blockIdx.x * 256 + threadIdx.x;
+    auto one = [&](float a, float b) {
+        return __fadd_rn(combine_term(a, lut1, lambda1), combine_term(b, lut2, lambda2));
+    };
+    for (long i = i0; i < n4; i += step) {
+        float4 a = reinterpret_cast<float4 *>(c1)[i];
+        const float4 b = reinterpret_cast<const float4 *>(c2)[i];
+        a.x = one(a.x, b.x);
+        a.y = one(a.y, b.y);
+        a.z = one(a.z, b.z);
+        a.w = one(a.w, b.w);
+        reinterpret_cast<float4 *>(c1)[i] = a;
     }
+    for (long i = 4 * n4 + i0; i < n; i += step) c1[i] = one(c1[i], c2[i]);
 }
 
 // ---------------------------------------------------------------------------
@@ -355,18 +461,27 @@ __global__ void k_combine(float *__restrict__ c1, const float *__restrict__ c2, 
 
 static dim3 row_grid(long per_row, int H, int threads) { return dim3((unsigned)((per_row + threads - 1) / threads), H); }
 
+template <typename K> static void cost_rows(cudaStream_t s, const K &k, float *cost, int D, int H, int W, int dir) {
+    k_cost_rows<<<dim3((W + kRowTX - 1) / kRowTX, H), 256, 0, s>>>(k, cost, D, W, dir, ((1u << 20) + D - 1) / D);
+}
 void launch_ad_gray(cudaStream_t s, const uint8_t *ref, const uint8_t *tar, float *cost, int D, int H, int W, int dir) {
-    k_ad_1ch<uint8_t><<<row_grid((long)W * D, H, 256), 256, 0, s>>>(ref, tar, cost, D, H, W, dir);
+    cost_rows(s, CostGray{ref, tar}, cost, D, H, W, dir);
 }
 void launch_ad_float(cudaStream_t s, const float *ref, const float *tar, float *cost, int D, int H, int W, int dir) {
-    k_ad_1ch<float><<<row_grid((long)W * D, H, 256), 256, 0, s>>>(ref, tar, cost, D, H, W, dir);
+    cost_rows(s, CostFloat{ref, tar}, cost, D, H, W, dir);
 }
 void launch_ad_color(cudaStream_t s, const uint8_t *ref, const uint8_t *tar, float *cost, int D, int H, int W, int dir,
                      int use_trunc, float trunc, int norm) {
-    k_ad_color<<<row_grid((long)W * D, H, 256), 256, 0, s>>>(ref, tar, cost, D, H, W, dir, use_trunc, trunc, norm);
+    cost_rows(s, CostColor{ref, tar, use_trunc, norm, trunc}, cost, D, H, W, dir);
 }
 void launch_census_bits(cudaStream_t s, const uint8_t *img, uint8_t *bits, int hr, int wr, int H, int W) {
     const long nb = (long)(2 * hr + 1) * (2 * wr + 1);
+    if (nb <= kBitsMax) {
+        const int wide = ((uintptr_t)bits & 15) == 0 ? 1 : 0;
+        k_census_bits_px<<<(unsigned)(((long)H * W + kBitsT - 1) / kBitsT), kBitsT, (size_t)kBitsT * nb, s>>>(
+            img, bits, hr, wr, H, W, wide);
+        return;
+    }
     k_census_bits<<<row_grid(W * nb, H, 256), 256, 0, s>>>(img, bits, hr, wr, H, W);
 }
 int census_words(int hr, int wr) {
@@ -382,16 +497,17 @@ void launch_census_codes(cudaStream_t s, const uint8_t *img, uint64_t *codes, in
     }
 }
 void launch_bits_pack(cudaStream_t s, const uint8_t *bits, uint64_t *codes, int nb, long npix) {
-    const unsigned g = (unsigned)((npix + 127) / 128);
-    if (nb <= 64) k_bits_pack<1><<<g, 128, 0, s>>>(bits, codes, nb, npix);
-    else if (nb <= 128) k_bits_pack<2><<<g, 128, 0, s>>>(bits, codes, nb, npix);
-    else k_bits_pack<4><<<g, 128, 0, s>>>(bits, codes, nb, npix);
+    const unsigned g = (unsigned)((npix + kBitsT - 1) / kBitsT);
+    const size_t smem = (size_t)kBitsT * nb;  // at most 32 KB
+    const int wide = ((uintptr_t)bits & 15) == 0 ? 1 : 0;
+    if (nb <= 64) k_bits_pack<1><<<g, kBitsT, smem, s>>>(bits, codes, nb, npix, wide);
+    else if (nb <= 128) k_bits_pack<2><<<g, kBitsT, smem, s>>>(bits, codes, nb, npix, wide);
+    else k_bits_pack<4><<<g, kBitsT, smem, s>>>(bits, codes, nb, npix, wide);
 }
 void launch_hamming(cudaStream_t s, const uint64_t *cr, const uint64_t *ct, float *cost, int nw, int D, int H, int W) {
-    const dim3 g = row_grid((long)W * D, H, 256);
-    if (nw == 1) k_hamming<1><<<g, 256, 0, s>>>(cr, ct, cost, D, H, W);
-    else if (nw == 2) k_hamming<2><<<g, 256, 0, s>>>(cr, ct, cost, D, H, W);
-    else k_hamming<4><<<g, 256, 0, s>>>(cr, ct, cost, D, H, W);
+    if (nw == 1) cost_rows(s, CostHamming<1>{cr, ct}, cost, D, H, W, 1);
+    else if (nw == 2) cost_rows(s, CostHamming<2>{cr, ct}, cost, D, H, W, 1);
+    else cost_rows(s, CostHamming<4>{cr, ct}, cost, D, H, W, 1);
 }
 void launch_rank(cudaStream_t s, const uint8_t *img, uint8_t *out, int m, int H, int W) {
     k_rank<<<row_grid(W, H, 128), 128, 0, s>>>(img, out, m, H, W);
@@ -419,9 +535,9 @@ void launch_cost_log_census(cudaStream_t s, const float *lr, const float *lt, co
 }
 void launch_combine(cudaStream_t s, float *c1, const float *c2, long n, const float *lut1, const float *lut2,
                     float lambda1, float lambda2) {
-    long blocks = (n + 255) / 256;
-    if (blocks > 152L * 64) blocks = 152L * 64;
-    k_combine<<<(unsigned)blocks, 256, 0, s>>>(c1, c2, n, lut1, lut2, lambda1, lambda2);
+    const long n4 = (((uintptr_t)c1 | (uintptr_t)c2) & 15) == 0 ? n / 4 : 0;
+    const long blocks = std::min((std::max(n4, n - 4 * n4) + 255) / 256, 152L * 64);
+    k_combine<<<(unsigned)blocks, 256, 0, s>>>(c1, c2, n, n4, lut1, lut2, lambda1, lambda2);
 }
 
 }  // namespace rts

@@ -101,3 +101,74 @@ def test_box(ctx, oracle_mod, H, W, D, r):
     cost[rng.random(cost.shape) < 0.001] = -np.inf
     got, want = ctx.boxAggregate(cost, r), oracle_mod.box(cost, r)
     assert np.array_equal(np.isnan(got), np.isnan(want)) and bits_equal(np.nan_to_num(got), np.nan_to_num(want))
+
+
+# whole and partial pixel blocks of a row, every code width, both directions
+@pytest.mark.parametrize("H,W,D", [(1, 1, 1), (3, 31, 9), (2, 64, 64), (5, 33, 33), (2, 300, 256), (70, 20, 20)])
+def test_cost_rows(ctx, oracle_mod, H, W, D):
+    O = oracle_mod
+    rng = np.random.default_rng(W + D)
+    L, R = rng.integers(0, 256, (2, H, W), dtype=np.uint8)
+    Lc, Rc = rng.integers(0, 256, (2, H, W, 3), dtype=np.uint8)
+    Lf, Rf = rng.normal(0, 90, (2, H, W)).astype(np.float32)
+    for d, gray, colour, fl in ((O.L2R, ctx.pixelBasedL2R, ctx.pixelBasedCostL2R_Color, ctx.pixelBasedCostL2R_Float),
+                                (O.R2L, ctx.pixelBasedR2L, ctx.pixelBasedR2L_Color, ctx.pixelBasedCostR2L_Float)):
+        assert bits_equal(gray(L, R, D), O.ad_gray(L, R, D, d))
+        assert bits_equal(colour(Lc, Rc, D, 1, 100.5), O.ad_color(Lc, Rc, D, d, 100.5, 1))
+        assert bits_equal(fl(Lf, Rf, D), O.ad_float(Lf, Rf, D, d))
+    for nb in ((0, 0), (0, 4), (0, 60)):  # 1, 9 and 121 bits; nonzero bytes count as set
+        b = rng.integers(0, 3, (2, H, W, 2 * nb[1] + 1), dtype=np.uint8)
+        want = O.hamming((b[0] != 0).astype(np.uint8), (b[1] != 0).astype(np.uint8), D, *nb)
+        assert bits_equal(ctx.calcHammingDist(b[0], b[1], D, *nb), want)
+
+
+# windows up to and above the 256 bits of the pixel kernel, images narrower than a block of 128
+@pytest.mark.parametrize("H,W,hr,wr", [(1, 1, 0, 0), (9, 15, 4, 3), (40, 33, 7, 8), (30, 130, 8, 7), (20, 40, 3, 18), (30, 40, 9, 9)])
+def test_census_bits(ctx, oracle_mod, H, W, hr, wr):
+    img = np.random.default_rng(W).integers(0, 9, (H, W), dtype=np.uint8)
+    assert bits_equal(ctx.calcCensusTrans(img, hr, wr), oracle_mod.census(img, hr, wr))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 7, 1025])
+def test_combine_remainders(ctx, oracle_mod, n):
+    c1 = np.arange(n, dtype=np.float32).reshape(1, n, 1)
+    assert bits_equal(ctx.combineCost(c1, c1[:, ::-1].copy(), 10.0, 30.0), oracle_mod.combine(c1, c1[:, ::-1].copy(), 10.0, 30.0))
+
+
+def test_device_buffers_without_vector_alignment(ctx, oracle_mod):
+    """Device buffers aligned to their element alone: the wide loads and stores must not be used."""
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    O, dev = oracle_mod, R.DEVICE
+    H, W, D = 21, 50, 36
+    rng = np.random.default_rng(5)
+
+    def put(a):
+        """The array one element past an aligned address."""
+        t = torch.empty(a.size + 1, dtype=torch.from_numpy(a).dtype, device="cuda")[1:].view(a.shape)
+        return t.copy_(torch.from_numpy(a))
+
+    img = rng.integers(0, 256, (H, W), dtype=np.uint8)
+    c1, c2 = rng.integers(0, 60, (2, H, W, D)).astype(np.float32)
+    rgb = patches(8, H, W)
+    bits, cost, comb = put(np.zeros((H, W, 63), np.uint8)), put(c1), put(c1)
+    horz, vert = (put(np.zeros((H, W, 2), np.int32)) for _ in range(2))
+    disp = put(img % 16)
+    ham, fin = put(c2), put(c2)
+    args = [put(x) for x in (img, c2, rgb)]
+    torch.cuda.synchronize()
+    ctx.call("calcCensusTrans", dev, args[0], bits, 4, 3, H, W)
+    ctx.call("calcHammingDist", dev, bits, bits, ham, 4, 3, H, W, D)
+    ctx.call("combineCost", dev, comb, args[1], 10.0, 10.0, H, W, D)
+    ctx.call("boxAggregate", dev, cost, H, W, D, 3)
+    ctx.call("findCross", dev, args[2], horz, vert, H, W)
+    ctx.call("cross_stereo_aggregation", dev, cost, fin, horz, horz, vert, vert, H, W, D)
+    ctx.call("disp_refinement", dev, disp, horz, vert, H, W, D)
+    ctx.synchronize()
+    b, box = O.census(img, 4, 3), O.box(c1, 3)
+    h, v = O.find_cross(rgb)
+    assert bits_equal(bits.cpu().numpy(), b) and bits_equal(ham.cpu().numpy(), O.hamming(b, b, D, 4, 3))
+    assert bits_equal(comb.cpu().numpy(), O.combine(c1, c2, 10.0, 10.0)) and bits_equal(cost.cpu().numpy(), box)
+    assert bits_equal(horz.cpu().numpy(), h) and bits_equal(vert.cpu().numpy(), v)
+    assert bits_equal(fin.cpu().numpy(), O.cross_aggr(box, h, h, v, v))
+    assert bits_equal(disp.cpu().numpy(), O.disp_refinement(img % 16, h, v, D))
