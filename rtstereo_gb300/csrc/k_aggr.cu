@@ -1,5 +1,5 @@
-// k_aggr.cu -- aggregation kernels, module form (seq/ConstBlockAggregation.cpp,
-// seq/CrossBasedAggregation.cpp, seq/AdaptiveWeightAggregation.cpp).
+// k_aggr.cu -- aggregation kernels, module form (seq/ConstBlockAggregation.cpp; cross
+// arms, refinement and median of seq/CrossBasedAggregation.cpp).
 //
 // These follow the reference's per-entry summation order exactly (sequential
 // float adds in window order, no fused multiply-add), so their results are
@@ -493,75 +493,6 @@ __global__ void k_find_cross(const uint8_t *__restrict__ rgb, int *__restrict__ 
     horz[2 * p + 1] = cross_arm(rgb, p, 1, W - 1 - x, L, tau);
 }
 
-// Adaptive support weights (seq/AdaptiveWeightAggregation.cpp:33-71):
-// w[p][k] = pw[k] * G[|Lab(p)-Lab(q)|^2], 0 outside the image.  G is the
-// host-computed expf(-sqrtf(n)/gamma_s), so the product is the reference's.
-__global__ void k_compute_weights(const uint8_t *__restrict__ lab, const float *__restrict__ pw,
-                                  const float *__restrict__ g, float *__restrict__ w, int H, int W, int r) {
-    const int y = blockIdx.y;
-    const int e = 2 * r + 1, area = e * e;
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)W * area) return;
-    const int x = (int)(i / area), k = (int)(i - (long)x * area);
-    const int dy = k / e - r, dx = k - (k / e) * e - r;
-    const int yy = y + dy, xx = x + dx;
-    float v = 0.f;
-    if (yy >= 0 && yy < H && xx >= 0 && xx < W) {
-        const uint8_t *a = lab + 3 * ((size_t)y * W + x);
-        const uint8_t *b = lab + 3 * ((size_t)yy * W + xx);
-        const int d0 = (int)a[0] - b[0], d1 = (int)a[1] - b[1], d2 = (int)a[2] - b[2];
-        v = __fmul_rn(pw[k], g[d0 * d0 + d1 * d1 + d2 * d2]);
-    }
-    w[((size_t)y * W + x) * area + k] = v;
-}
-
-// Adaptive-weight cost from weight arrays (seq/AdaptiveWeightAggregation.cpp:73-111):
-// sequential sums over the window in raster order; weight = wR*wT, score += C*weight.
-__global__ void k_aw_l2r_w(const float *__restrict__ wr, const float *__restrict__ wt, const float *__restrict__ cost,
-                           float *__restrict__ out, int H, int W, int D, int r) {
-    const int y = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * D) return;
-    const int x = i / D, d = i - x * D;
-    const int e = 2 * r + 1, area = e * e;
-    const float *a = wr + ((size_t)y * W + x) * area;
-    const float *b = wt + ((size_t)y * W + tar_col(x, d, W, 1)) * area;
-    float sw = 0.f, sc = 0.f;
-    int k = 0;
-    for (int dy = -r; dy <= r; dy++) {
-        const float *crow = cost + (size_t)wrap1(y + dy, H) * W * D + d;
-        for (int dx = -r; dx <= r; dx++, k++) {
-            const float wgt = __fmul_rn(a[k], b[k]);
-            sw = __fadd_rn(sw, wgt);
-            sc = __fadd_rn(sc, __fmul_rn(crow[(size_t)wrap1(x + dx, W) * D], wgt));
-        }
-    }
-    out[((size_t)y * W + x) * D + d] = __fdiv_rn(sc, sw);
-}
-
-// R2L form, out of place (contract for seq/AdaptiveWeightAggregation.cpp:113-150):
-// the weights are taken at the window pixel and at the window pixel +d.
-__global__ void k_aw_r2l_w(const float *__restrict__ wr, const float *__restrict__ wt, const float *__restrict__ cost,
-                           float *__restrict__ out, int H, int W, int D, int r) {
-    const int y = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= W * D) return;
-    const int x = i / D, d = i - x * D;
-    const int e = 2 * r + 1, area = e * e;
-    float sw = 0.f, sc = 0.f;
-    int k = 0;
-    for (int dy = -r; dy <= r; dy++) {
-        const size_t row = (size_t)wrap1(y + dy, H) * W;
-        for (int dx = -r; dx <= r; dx++, k++) {
-            const int xr = wrap1(x + dx, W), xt = wrap1(x + dx + d, W);
-            const float wgt = __fmul_rn(wr[(row + xr) * area + k], wt[(row + xt) * area + k]);
-            sw = __fadd_rn(sw, wgt);
-            sc = __fadd_rn(sc, __fmul_rn(cost[(row + xr) * D + d], wgt));
-        }
-    }
-    out[((size_t)y * W + x) * D + d] = __fdiv_rn(sc, sw);
-}
-
 // Disparity refinement (contract for seq/CrossBasedAggregation.cpp:171-212 with the
 // votes of the unmodified input): mode of the input disparities over rows
 // y-top .. y+bottom-1 of the cross, segment x-left .. x+right; strict first maximum
@@ -764,19 +695,6 @@ void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W
     const size_t smem = (size_t)(kMedTX + 2 * r) * (kMedTY + 2 * r) * 4;
     if (ch == 3) k_median<3><<<g, b, smem, s>>>(in, out, H, W, r);
     else k_median<1><<<g, b, smem, s>>>(in, out, H, W, r);
-}
-void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw, const float *g, float *w, int H, int W,
-                            int r) {
-    const long area = (long)(2 * r + 1) * (2 * r + 1);
-    k_compute_weights<<<row_grid(W * area, H, 256), 256, 0, s>>>(lab, pw, g, w, H, W, r);
-}
-void launch_aw_l2r_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,
-                           int W, int D, int r) {
-    k_aw_l2r_w<<<row_grid((long)W * D, H, 128), 128, 0, s>>>(wr, wt, cost, out, H, W, D, r);
-}
-void launch_aw_r2l_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,
-                           int W, int D, int r) {
-    k_aw_r2l_w<<<row_grid((long)W * D, H, 128), 128, 0, s>>>(wr, wt, cost, out, H, W, D, r);
 }
 void launch_disp_refine(cudaStream_t s, uint8_t *disp, uint16_t *runs, const int *horz, const int *vert, int H, int W,
                         int D) {

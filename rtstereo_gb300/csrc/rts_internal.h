@@ -223,13 +223,14 @@ void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D);
 size_t cross_aggr_bytes(int H, int W, int D);
 int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
                       const int *vt, int H, int W, int D, void *work);
-// k_aggr.cu
+// k_aw_mod.cu
 void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw, const float *g, float *w, int H,
                             int W, int r);
 void launch_aw_l2r_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,
                            int W, int D, int r);
 void launch_aw_r2l_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,
                            int W, int D, int r);
+// k_aggr.cu
 // in place; runs: scratch [H][W] words (the copy the votes are read from); two launches
 void launch_disp_refine(cudaStream_t s, uint8_t *disp, uint16_t *runs, const int *horz, const int *vert, int H, int W,
                         int D);

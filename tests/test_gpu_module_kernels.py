@@ -172,3 +172,28 @@ def test_device_buffers_without_vector_alignment(ctx, oracle_mod):
     assert bits_equal(horz.cpu().numpy(), h) and bits_equal(vert.cpu().numpy(), v)
     assert bits_equal(fin.cpu().numpy(), O.cross_aggr(box, h, h, v, v))
     assert bits_equal(disp.cpu().numpy(), O.disp_refinement(img % 16, h, v, D))
+
+
+# both tile widths, pixels and disparities past their tiles' ends, windows below and above a warp's 32
+# taps; weights of any value, outside the image too
+@pytest.mark.parametrize("H,W,D,r", [(1, 1, 1, 0), (3, 64, 32, 1), (7, 65, 33, 2), (20, 140, 64, 16), (17, 90, 66, 5),
+                                     (18, 40, 7, 17), (3, 260, 129, 2), (47, 80, 33, 46)])
+def test_adaptive_weight_tiles(ctx, oracle_mod, H, W, D, r):
+    O = oracle_mod
+    rng = np.random.default_rng(W + r)
+    lab = patches(r, H, W)
+    pw = O.prox_weight(36.0, r)
+    assert bits_equal(ctx.computeWeights(pw, lab, 7.0, r), O.compute_weights(pw, lab, 7.0, r))
+    wl, wr = rng.normal(0.5, 0.5, (2, H, W, (2 * r + 1) ** 2)).astype(np.float32)
+    cost = rng.normal(0.0, 1.0, (H, W, D)).astype(np.float32)
+    assert bits_equal(ctx.calcAWCostL2R(wl, wr, cost, r), O.aw_l2r(wl, wr, cost, r))
+    if r + D <= W:
+        assert bits_equal(ctx.calcAWCostR2L(wl, wr, cost, r), O.aw_r2l(wl, wr, cost, r))
+
+
+# radii whose window passes the tiled kernels' shared memory: weights above 46
+@pytest.mark.parametrize("r", [46, 47])
+def test_compute_weights_large_window(ctx, oracle_mod, r):
+    lab = patches(r, r + 2, 20 + r)
+    pw = oracle_mod.prox_weight(36.0, r)
+    assert bits_equal(ctx.computeWeights(pw, lab, 7.0, r), oracle_mod.compute_weights(pw, lab, 7.0, r))
