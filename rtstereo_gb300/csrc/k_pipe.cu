@@ -17,6 +17,7 @@
 #include "rts_fused.cuh"
 #include "rts_pipe.h"
 #include "rts_tma.h"
+#include "rts_views.h"
 
 namespace rts {
 
@@ -861,9 +862,19 @@ rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const
 }
 
 bool cross_fused_supported(const rts_params &p) {
-    // 16-byte row copies in the vertical kernel need D a multiple of 8; the
-    // 64-entry ring of the horizontal kernel bounds the arm length (k_batch.cu)
+    // the 64-entry ring of the horizontal kernel bounds the arm length (k_batch.cu); ranges
+    // that are not a multiple of 8 go the way of cross_ragged_supported
     return p.cross_arm <= 23 && p.disp_range % 8 == 0;
+}
+
+bool cross_ragged_supported(const rts_params &p) {
+    // The view kernels take any range, with the results of the composed module kernels
+    // (450x375, D = 60: 571 us a pair composed, 374 us here) where costs are made from records
+    // and are >= 0 (their quotients take the fast exact division): positive lambdas, no
+    // negative truncation.  Other costs stay composed.
+    return p.aggr == RTS_AGGR_CROSS && p.cross_arm <= 23 && p.disp_range % 8 != 0 && cross_record_costs(p) &&
+           (p.cost2 == RTS_COST_NONE || (p.lambda1 > 0.f && p.lambda2 > 0.f)) &&
+           (p.cost1 != RTS_COST_AD || p.ad_trunc >= 0.f);
 }
 
 rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, const uint8_t *labr,

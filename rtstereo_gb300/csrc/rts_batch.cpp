@@ -189,7 +189,8 @@ rts_status rts_batch_run(rts_ctx *ctx, int n, const rts_pair *pairs, const rts_p
 
 // The batched cross-based pipeline on DEVICE buffers: one view table, autotuned
 // tiles, one captured graph per batch shape.  Callers have validated the pairs.
-rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs) {
+rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs,
+                                bool optional) {
     for (int i = 0; i < n; i++)
         if (!pairs[i].left_gray || !pairs[i].right_gray || !outs[i].disp_left ||
             (params[0].right_view && (!outs[i].disp_right || !outs[i].mask)))
@@ -205,9 +206,6 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
     std::string key = shape_key(n, pairs, params);
     const bool forced = c->force_tune[0] > 0;
     if (forced) key.append((const char *)c->force_tune, sizeof(c->force_tune));
-    const size_t bytes = views_bytes(W.data(), H.data(), D.data(), nv, half);
-    void *arena;
-    RTS_TRY(scratch(c, SL_BATCH0, bytes, &arena));
     // the tables the kernels read must hold this lambda pair before any replay
     RTS_TRY(cross_tables(c, p));
     int gray = 1;  // records hold the gray byte as colour only when no pair has colour images
@@ -228,6 +226,15 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
         }
         median_pairs(c, p.median_ksize, n, pairs, dst.data(), med);
     }
+    // the arena last: a later allocation could give optional scratch back
+    const size_t bytes = views_bytes(W.data(), H.data(), D.data(), nv, half);
+    void *arena;
+    if (optional) {
+        arena = stream_work(c, bytes);
+        if (!arena) return set_error(c, RTS_ERR_OOM, "no optional scratch");
+    } else {
+        RTS_TRY(scratch(c, SL_BATCH0, bytes, &arena));
+    }
     ViewBatch b;
     plan_views_at(arena, W.data(), H.data(), D.data(), nv, half, &b);
     fill_views(b, n, pairs, outs, right, p.median_ksize ? &med : nullptr);
@@ -238,6 +245,19 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
         ft.vert_rows = c->force_tune[0];
         ft.grid_mult = c->force_tune[1];
         ft.persistent = c->force_tune[2];
+        tit = gc->tunes.emplace(key, ft).first;
+    }
+    if (tit == gc->tunes.end() && optional) {
+        // strips that give the vertical kernel some eight blocks for each of two an SM
+        long cols = 0;
+        int h = 1;
+        for (int i = 0; i < nv; i++) {
+            cols += W[i];
+            h = std::max(h, H[i]);
+        }
+        const long strips = std::min((16L * sm_count() + cols - 1) / cols, (h + 95L) / 96);
+        CrossTune ft;
+        ft.vert_rows = (int)((h + strips - 1) / strips);
         tit = gc->tunes.emplace(key, ft).first;
     }
     if (tit == gc->tunes.end()) {

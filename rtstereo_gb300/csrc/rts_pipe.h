@@ -19,6 +19,9 @@ rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const
                             void *vol, int half);
 // the cross-based pipeline runs over view tables (rts_views.h) when this holds
 bool cross_fused_supported(const rts_params &p);
+// ... and for a disparity range that is not a multiple of 8 when this holds (in the plain
+// form, whichever form is asked for: the composed path has no other)
+bool cross_ragged_supported(const rts_params &p);
 // adaptive-weight aggregation + arg-min over a float (half == 0) or __half volume
 rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, const uint8_t *labr,
                     const uint8_t *labt, uint16_t *raw, int *row_last, float *cost_out);

@@ -400,6 +400,27 @@ static rts_status pipeline_cross_views(rts_ctx *c, const rts_params &p, int H, i
                               b.row_last_count);
 }
 
+// The scratch of the composed cross-based path (record costs), both views: a call that
+// goes through the view kernels instead holds it too, so that the same sizes are refused
+// for want of memory and a later captured call finds it allocated.
+static rts_status reserve_composed_cross(rts_ctx *c, const rts_params &p, int H, int W, bool rgb) {
+    const size_t np = (size_t)H * W, ne = np * p.disp_range;
+    const int nw = census_words(p.census_hrad, p.census_wrad);
+    const bool census = p.cost1 == RTS_COST_CENSUS || p.cost2 == RTS_COST_CENSUS;
+    void *q;
+    if (!rgb || p.right_view) RTS_TRY(scratch(c, SL_V_RGB, np * 12, &q));
+    if (p.right_view) RTS_TRY(scratch(c, SL_V_GRAY, np * 2, &q));
+    RTS_TRY(scratch(c, SL_V_COST1, ne * 4, &q));
+    if (p.cost1 == RTS_COST_RANK) RTS_TRY(scratch(c, SL_V_AUX, np * 2, &q));
+    if (census) RTS_TRY(scratch(c, SL_V_CODES, np * nw * 16, &q));
+    if (p.cost2 != RTS_COST_NONE) RTS_TRY(scratch(c, SL_V_COST2, ne * 4, &q));
+    RTS_TRY(scratch(c, SL_V_ARMS, np * 32, &q));
+    RTS_TRY(scratch(c, SL_V_SEG, ne * 4, &q));
+    if (p.median_ksize) RTS_TRY(scratch(c, SL_V_MED, np * 6, &q));
+    RTS_TRY(scratch(c, SL_V_RAW, np * 2, &q));
+    return scratch(c, SL_V_ROWLAST, (size_t)H * 4, &q);
+}
+
 // Prepares device inputs for both views and runs them; all pointers device.
 rts_status pipeline_device(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *lg, const uint8_t *rg,
                            const uint8_t *lc, const uint8_t *rc, const uint8_t *ll, const uint8_t *rl, uint8_t *dl,
@@ -410,6 +431,16 @@ rts_status pipeline_device(rts_ctx *c, const rts_params &p, int H, int W, const 
     if (!cost_out && p.aggr == RTS_AGGR_CROSS && cross_fused_supported(p) && cross_record_costs(p))
         return pipeline_cross_views(c, p, H, W, lg, rg, lc && rc ? lc : nullptr, lc && rc ? rc : nullptr, dl, dr,
                                     mask);
+    if (!cost_out && cross_ragged_supported(p)) {
+        rts_params q = p;
+        q.precision = RTS_PREC_F32;
+        const bool rgb = lc && rc;
+        rts_pair pr{W, H, lg, rg, rgb ? lc : nullptr, rgb ? rc : nullptr, nullptr, nullptr};
+        rts_out o{dl, dr, mask, nullptr};
+        RTS_TRY(reserve_composed_cross(c, p, H, W, rgb));
+        const rts_status st = batch_views_run(c, 1, &pr, &q, &o, true);
+        if (st != RTS_ERR_OOM) return st;  // no room, or a captured stream: the module kernels below
+    }
     const bool need_lab = p.aggr == RTS_AGGR_AW;
     // the fused kernels read packed colour records even for gray-only costs
     const bool need_rgb = true;

@@ -106,6 +106,9 @@ rts_status upload_views(rts_ctx *c, const ViewBatch &b, const CrossTune &tune, v
 
 // The batched cross-based pipeline over n validated pairs (DEVICE buffers, fast
 // costs): autotuned tiles and one captured CUDA graph per batch shape.
-rts_status batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs);
+// optional: in the optional scratch of the stream, tiles by a rule instead of the autotuner;
+// RTS_ERR_OOM, with nothing done, where there is no such scratch.
+rts_status batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs,
+                           bool optional = false);
 
 }  // namespace rts

@@ -1,0 +1,85 @@
+"""Disparity ranges that are not a multiple of 8 in the cross-based pipeline: the view
+kernels' results against the C oracle, bit for bit, over costs, forms, colours and
+sizes; and where the call must fall back to the module kernels."""
+import numpy as np
+import pytest
+
+from conftest import bits_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def pair(seed, W, H, D, colour):
+    import rtstereo_gb300 as R
+    L, Rr, _ = R.synth_pair(seed, W, H, D, 3, 0, 2.0, min(4, D - 1))
+    if not colour:
+        return (L, Rr), (R.gray_to_rgb(L), R.gray_to_rgb(Rr))
+    rng = np.random.default_rng(seed)
+    # blocks of one colour: long arms
+    base = np.repeat(np.repeat(rng.integers(0, 200, (H // 11 + 1, W // 11 + 1, 3)), 11, 0), 11, 1)[:H, :W]
+    Lc = (base + L[..., None] // 16).astype(np.uint8)
+    Rc = np.ascontiguousarray(np.roll(Lc, -min(2, W - 1), 1))
+    return (L, Rr), (Lc, Rc)
+
+
+def check(ctx, O, W, H, D, colour, **kw):
+    import rtstereo_gb300 as R
+    (L, Rr), (Lc, Rc) = pair(W + H + D, W, H, D, colour)
+    p = R.params(disp_range=D, **kw)
+    got = ctx.pipeline(p, L, Rr, Lc, Rc) if colour else ctx.pipeline(p, L, Rr)
+    o = O.pipeline(O.params(cost1=p.cost1, cost2=p.cost2, aggr=3, lambda1=p.lambda1, lambda2=p.lambda2, D=D,
+                            rank_rad=p.rank_rad, cross_L=p.cross_arm, cross_tau=p.cross_tau, ad_trunc=p.ad_trunc,
+                            right_view=p.right_view), L, Rr, Lc, Rc)
+    assert bits_equal(got[0], o[0])
+    if p.right_view:
+        assert bits_equal(got[1], o[1]) and bits_equal(got[2], o[2])
+
+
+@pytest.mark.parametrize("W,H,D", [(9, 12, 1), (20, 11, 7), (61, 40, 20), (90, 33, 60), (140, 20, 129), (300, 9, 255)])
+@pytest.mark.parametrize("colour", [False, True])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_sizes(ctx, oracle_mod, W, H, D, colour, precision):
+    # the FP16 form of such a range has always been the plain one
+    check(ctx, oracle_mod, W, H, D, colour, precision=precision)
+
+
+@pytest.mark.parametrize("kw", [dict(cost1=3, cost2=0), dict(cost1=1, cost2=0), dict(cost1=2, cost2=3, rank_rad=3),
+                                dict(ad_trunc=7.5), dict(cost1=3, cost2=1), dict(right_view=0), dict(cross_arm=23),
+                                dict(cross_arm=24), dict(lambda1=-5.0, lambda2=30.0), dict(ad_trunc=-3.0),
+                                dict(cost1=1, cost2=0, ad_trunc=1000.0)], ids=str)
+def test_options(ctx, oracle_mod, kw):
+    check(ctx, oracle_mod, 70, 45, 20, True, **kw)
+
+
+def test_captured_call(oracle_mod):
+    """On a captured stream the call records the module kernels; replays give the same results."""
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    import ctypes as C
+    W, H, D = 70, 45, 20
+    (L, Rr), _ = pair(5, W, H, D, False)
+    s = torch.cuda.Stream()
+    with R.Context(0) as ctx:
+        ctx.set_stream(s.cuda_stream)
+        l, r = torch.from_numpy(L).cuda(), torch.from_numpy(Rr).cuda()
+        outs = [torch.empty(H, W, dtype=torch.uint8, device="cuda") for _ in range(3)]
+        p = R.params(disp_range=D)
+        prm = (R.Pair(W, H, l.data_ptr(), r.data_ptr(), None, None, None, None), p,
+               R.Out(*[t.data_ptr() for t in outs], None))
+        torch.cuda.synchronize()
+        call = lambda: ctx.call("pipeline_run", R.DEVICE, *[C.byref(x) for x in prm])
+        call()
+        s.synchronize()
+        want = [t.cpu().numpy().copy() for t in outs]
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            call()
+        for t in outs:
+            t.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(outs, want):
+            assert bits_equal(a.cpu().numpy(), b)
+        ctx.set_stream(None)
+    o = oracle_mod.pipeline(oracle_mod.params(D=D), L, Rr, *pair(5, W, H, D, False)[1])
+    assert bits_equal(want[0], o[0]) and bits_equal(want[1], o[1])
