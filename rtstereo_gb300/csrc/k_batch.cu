@@ -10,10 +10,12 @@
 //   hseg   warp per (view, row, 32 disparities): cost, running sum along x
 //          (seq/CrossBasedAggregation.cpp:117-125) and the row segment of every
 //          entry (:151-160)
-//   vert   block per (view, column, strip of rows): row segments streamed down
-//          the column through a shared ring, vertical sums over the cross
-//          (:140-167), the division and the first strict arg-min over d
-//          (seq/WTA.cpp:15-22)
+//   vert   both views of a pair with record costs: warp per (pair, column, strip of
+//          rows, 32 disparities), segments streamed down the column through rings of
+//          each lane's own (k_vert_dual), then k_best_views for the right view's winners;
+//          other views: block per (view, column, strip of rows), a shared ring
+//          (k_vert_views).  Vertical sums over the cross (:140-167), the division and
+//          the first strict arg-min over d (seq/WTA.cpp:15-22)
 //   fill   warp per (view, row): the winner carry of seq/WTA.cpp:12
 //   cc     block per (pair, row): seq/CrossCheck.cpp:10-23
 //
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(kPrepT) k_prep_views(ViewTable t, int hr, int 
             const uint32_t lr = (uint32_t)len[0] | ((uint32_t)len[1] << 16);
             const uint32_t tb = (uint32_t)len[2] | ((uint32_t)len[3] << 16);
             const size_t p = (size_t)y * W + x;
+            if (img && V.best_r) V.best_r[p] = ~0ull;  // the right view's minima start here
             uint32_t cword = med ? pixel_word<GRAYREC>(rgb ? rgb : gray, rgb != nullptr, p) : centre;
             if (rank >= 0) {
                 // seq/RankFilter.cpp:16-29: 1 + neighbours strictly below the centre, as u8
@@ -189,6 +192,13 @@ __global__ void __launch_bounds__(kPrepT) k_prep_views(ViewTable t, int hr, int 
 // (independent), the running sum, the segments of the columns 24 back, then
 // the arm words.  Columns past the row end are computed from clamped records
 // and never written.
+//
+// The right view of a pair whose two views share the vertical kernel (V.skew) writes
+// its segments by LEFT image column, so that the two views' segments of the same pixel
+// pair lie at the same index.  Its columns still run in the mirrored order, but lane
+// by lane one step apart: at step s lane i is at mirrored column s - (31 - i), so all
+// 32 lanes meet the same left pixel (the broadcast record, right to left) and 32
+// consecutive right ones.  Ring slots are steps; a lane's column 0 is slot 31 - i.
 constexpr int kHsegW = 2;   // warps per block
 constexpr int kHLag = 24;   // columns between a column's prefix and its segment
 constexpr int kHSub = 8;    // columns per group
@@ -219,7 +229,11 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
         const bool active = d < D;
         const int dd = active ? d : D - 1;
         const size_t row = (size_t)y * W;
-        const uint4 *rr = V.rref + row, *rt = V.rtar + row;
+        const bool skew = MODE != 0 && V.skew;
+        const int zl = skew ? 31 - lane : 0;  // the ring's index of the lane's column 0
+        // broadcast and lane records: the reference and target images, or (skewed) both of the
+        // left image's and the right image's
+        const uint4 *rr = (skew ? V.rtar : V.rref) + row, *rt = (skew ? V.rref : V.rtar) + row;
         ST *seg = reinterpret_cast<ST *>(V.seg) + row * D + d;
         const float *vol = MODE == 0 ? V.vol + row * D + dd : nullptr;
         // image column of view column xv (any integer: columns past the row end wrap)
@@ -234,7 +248,24 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
             return r;
         };
         uint4 na, nb0, nb1;
+        // skewed: left column of ring step s (below 2 W where the segment is real)
+        auto xo = [&](int s) {
+            const int v = W + 30 + dbase - s;
+            return v >= W ? v - W : v;
+        };
+        const int sD = skew ? -D : D;
+        const uint4 *RBl = RB + (skew ? lane : 31 - lane);  // the lane's record of a group's column 0
         auto fetch = [&](int x0) {
+            if (skew) {
+                // left column of step s: W + 30 + dbase - s (mod W); right column: W + 30 - s - lane
+                int xl = (W + 30 + dbase - x0 - lane) % W;
+                if (xl < 0) xl += W;
+                const int xr = W + 30 - x0 - lane;
+                na = rr[xl];
+                nb0 = rt[imax(imin(xr, W - 1), 0)];
+                nb1 = rt[imax(imin(xr - 32, W - 1), 0)];
+                return;
+            }
             const int t0 = x0 - dbase - 31;  // target column of RB[0]: x - d for x = x0, lane 31
             na = rr[col(imin(x0 + lane, W - 1))];
             nb0 = rt[col(t0 + lane)];
@@ -242,7 +273,8 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
         };
         fetch(0);
         float acc = 0.f;
-        const int xend = W + kHLag;
+        const int xend = W + kHLag + (skew ? 31 : 0);
+        const int inner0 = kHLag + (skew ? 31 : 0);  // first group whose segments are all real
         for (int x0 = 0; x0 < xend; x0 += 32) {
             __syncwarp();
             RA[lane] = fix(na);
@@ -259,7 +291,7 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
 #pragma unroll
                 for (int u = 0; u < kHSub; u++) {
                     const uint4 a = RA[kHSub * h + u];
-                    const uint4 b = RB[kHSub * h + u + 31 - lane];  // target column x - d
+                    const uint4 b = RBl[kHSub * h + u];  // target column x - d
                     if constexpr (MODE == 0) {
                         cv[u] = vol[(size_t)imin(hx + u, W - 1) * D];
                     } else if constexpr (MODE == 1) {
@@ -283,6 +315,8 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
                         cv[u] = pair_cost(a, b, cfg);
                     }
                     lv[u] = __vminu2(a.w, b.w) * 128u + 128u;
+                    // a skewed lane's row begins at step zl
+                    if (decltype(edge)::value && MODE != 0 && hx + u < zl) cv[u] = 0.f;
                 }
                 // running sum, seq/CrossBasedAggregation.cpp:123 (0 + c is c for every cost but -0)
                 float *PRh = PR + ((x0 & 32) + kHSub * h) * 32;
@@ -292,20 +326,24 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
                     else acc = __fadd_rn(acc, cv[u]);
                     PRh[u * 32] = acc;
                 }
+                // where the segment of the group's first column goes, and the step to the next
+                ST *segp = seg + (size_t)(skew ? xo(hx - kHLag) : hx - kHLag) * D;
                 // segments of columns xs = x - 24 (seq/CrossBasedAggregation.cpp:151-160; a left
                 // end before column 0 is clamped to column 0, :153-154)
 #pragma unroll
                 for (int u = 0; u < kHSub; u++) {
                     const int xs = hx - kHLag + u;
-                    if (!decltype(edge)::value || (xs >= 0 && xs < W)) {
+                    if (!decltype(edge)::value || (xs >= zl && xs < W + zl)) {
                         const uint32_t e = LR[((kHSub * h + u - kHLag) & 31) * 32];
                         const int xsl = xs << 7;
-                        const int il = imax(xsl - (int)(e & 0xffffu), 0);
+                        const int il = imax(xsl - (int)(e & 0xffffu), zl << 7);
                         const int ir = xsl + (int)(e >> 16);
                         // slot (column & 63) of the ring: the byte offset is (column << 7) & 0x1f80
                         const float pl = PR[(il & 0x1f80) >> 2];
                         const float pr = PR[(ir & 0x1f80) >> 2];
-                        if (active) seg[(size_t)xs * D] = to_store<ST>(__fsub_rn(pr, pl));
+                        ST *sp = segp + (ptrdiff_t)u * sD;
+                        if (decltype(edge)::value && skew) sp = seg + (size_t)xo(xs) * D;  // may wrap in the group
+                        if (active) *sp = to_store<ST>(__fsub_rn(pr, pl));
                     }
                 }
                 uint32_t *LRh = LR + kHSub * h * 32;
@@ -316,7 +354,9 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
             auto run = [&](auto hc) {
                 constexpr int h = decltype(hc)::value;
                 const int g0 = x0 + kHSub * h;
-                if (g0 >= kHLag && g0 + kHSub - 1 - kHLag < W) group(hc, std::false_type{});
+                // (skewed: nor does the left column wrap inside it, from 0 to W - 1)
+                const int wrap = 30 + dbase - (g0 - kHLag);  // left column - W of its first segment
+                if (g0 >= inner0 && g0 + kHSub - 1 - kHLag < W && !(skew && wrap >= 0 && wrap < kHSub - 1)) group(hc, std::false_type{});
                 else group(hc, std::true_type{});
             };
             run(std::integral_constant<int, 0>{});
@@ -329,7 +369,8 @@ __global__ void __launch_bounds__(kHsegW * 32, 8) k_hseg_views(ViewTable t, Cost
 }
 
 // ---------------------------------------------------------------------------
-// vert: block per (view, column x, strip of rows).  Rows enter a shared ring 8
+// vert, one view (left views alone, precomputed volumes): block per (view, column x,
+// strip of rows).  Rows enter a shared ring 8
 // at a time ("ticks", warp w ingesting row w of the tick); for every entry the
 // ring holds the row segment and the row's pixel count l + r + 1, and the
 // entry's vertical arms t | b << 8.  Each step a warp computes one output row
@@ -658,6 +699,350 @@ __global__ void __launch_bounds__(kVertT, NCH <= 4 ? 2 : 1)
 }
 
 // ---------------------------------------------------------------------------
+// vert, both views of a pair at once.  The entry (left pixel x, d) of the left view and
+// the entry (right pixel x - d mod W, d) of the right view are the same pixel pair: their
+// arms (minima of the two pixels'), so also the rows and the pixel count of their
+// crosses, are the same; only the segments differ (their running sums start at opposite
+// ends of the row).  So one warp streams both down a column x of the left image, for 32
+// disparities (lane = disparity; the right view's segments lie at the same index, see
+// k_hseg_views), and shares everything but the segment loads, the adds and the quotients.
+// Every lane keeps rings of its own in shared memory (no other lane reads them; schedule
+// and depth: rts_vert_ring.h):
+//   segments   [group of 4 rows][lane][4], one per view: a 16-byte (f16: 8-byte) load is
+//              four rows
+//   words      [row][lane]: running sum of l + r down the column (low half, mod 2^16) |
+//              t << 16 | b << 24, the entry's vertical arms
+// Rows enter four at a time, the next four rows' loads in flight meanwhile; a step makes
+// four output rows.  A row read from the ring is added to both views' sums of the outputs
+// whose arm [y - t, y + b] holds it: one bit test for two adds, eight independent chains,
+// rows top to bottom for every output (seq/CrossBasedAggregation.cpp:140-164).  Pixel
+// counts are differences of running sums; integer costs (ST = uint16_t) take their sums
+// the same way from running sums mod 2^32 and walk no rows.  The average is the correctly
+// rounded quotient (:166).
+// Winners: the left view's keys of a step go through a shared tile (two buffers, one
+// barrier a step) to a warp per output row; the right view's keys belong to 32 different
+// pixels and enter {key, d} minima in memory (first strict minimum: the least {key, d}),
+// which k_best_views turns into winners.
+// A block of NWB warps holds the chunks of one column, or of NWB / chunks neighbouring
+// columns.
+// Bound: the latency of a step's serial phases (arm words, counts, walk, quotients, key
+// reduction) with the 12 warps an SM that the f32 rings leave; the issue slots are 54 %
+// used.  Against one launch item per view (k_vert_views: a warp per output row over a
+// ring shared by the block, 105 instructions per 32 entries, 67 here): 1920x1080,
+// D = 128, random dots 2060 -> 1710 us, 640x480, D = 64, long arms 443 -> 232 us, six mixed
+// pairs in the FP16 form 3625 -> 2322 us.
+template <typename ST> struct DRing;
+template <> struct DRing<float> {
+    using In = float;
+    using G4 = float4;  // four rows of a lane
+    static __device__ __forceinline__ G4 pack(const In (&s)[4]) { return make_float4(s[0], s[1], s[2], s[3]); }
+    static __device__ __forceinline__ void rows(G4 g, float (&v)[4]) {
+        v[0] = g.x; v[1] = g.y; v[2] = g.z; v[3] = g.w;
+    }
+};
+template <> struct DRing<__half> {
+    using In = unsigned short;  // f16 bits; widened exactly when a group is read
+    using G4 = uint2;
+    static __device__ __forceinline__ G4 pack(const In (&s)[4]) {
+        return make_uint2((uint32_t)s[0] | ((uint32_t)s[1] << 16), (uint32_t)s[2] | ((uint32_t)s[3] << 16));
+    }
+    static __device__ __forceinline__ void rows(G4 g, float (&v)[4]) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&g.x));
+        const float2 b = __half22float2(*reinterpret_cast<const __half2 *>(&g.y));
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    }
+};
+template <> struct DRing<uint16_t> {
+    using In = unsigned short;  // exact integer segments, held as running sums
+    using G4 = uint4;
+};
+
+// shared bytes of a block: two segment rings and the words of every warp, the key tile
+template <typename ST> static size_t dual_smem(int nwb, int L) {
+    const size_t dep = (size_t)vert_lane_depth(L);
+    return (size_t)nwb * dep * 32 * (2 * sizeof(typename DRing<ST>::G4) / 4 + 4) +
+           (size_t)2 * kVertStep * nwb * 32 * sizeof(uint32_t);
+}
+
+// a += u, b += v where the mask has the bit: one test, two predicated adds
+__device__ __forceinline__ void add2_if_bit(float &a, float &b, uint32_t m, uint32_t bit, float u, float v) {
+    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\t"
+        "@p add.rn.f32 %0, %0, %4;\n\t@p add.rn.f32 %1, %1, %5;\n\t}"
+        : "+f"(a), "+f"(b)
+        : "r"(m), "r"(bit), "f"(u), "f"(v));
+}
+
+// The columns xg .. of this block, rows y0 .. y1-1; warp = column (high) and chunk (low).
+template <typename ST, int NWB>
+__device__ __forceinline__ void dual_item(const ViewDesc &V, const ViewDesc &VR, int xg, int lognch, int y0, int y1,
+                                          int L, int DEP, const float *__restrict__ rcp, unsigned char *vsm) {
+    using RG = DRing<ST>;
+    using In = typename RG::In;
+    using G4 = typename RG::G4;
+    constexpr bool INT = std::is_same<ST, uint16_t>::value;
+    constexpr int S = kVertStep;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int W = V.W, H = V.H, D = V.D;
+    const int x = xg + (warp >> lognch), c = warp & ((1 << lognch) - 1);
+    const int d = 32 * c + lane;
+    const bool live = x < W && 32 * c < D, dok = live && d < D;
+    const int RS = DEP / 4 * 32;  // G4s of one warp's ring
+    G4 *segl = reinterpret_cast<G4 *>(vsm) + (size_t)2 * warp * RS + lane, *segr = segl + RS;  // group g at [32 g]
+    uint32_t *wrd = reinterpret_cast<uint32_t *>(vsm + (size_t)2 * NWB * RS * sizeof(G4)) + (size_t)warp * DEP * 32 +
+                    lane;  // row slot s at [32 s]
+    uint32_t *keys = reinterpret_cast<uint32_t *>(vsm + (size_t)2 * NWB * RS * sizeof(G4)) + (size_t)NWB * DEP * 32;
+    // INT: the rings hold running sums, [row][lane] words
+    uint32_t *Ql = reinterpret_cast<uint32_t *>(vsm) + (size_t)2 * warp * DEP * 32 + lane, *Qr = Ql + DEP * 32;
+    const int ra = imax(0, y0 - L), rb = imin(H, y1 + L);
+    const int xc = live ? x : 0;
+    int xt = xc - (dok ? d : 0);  // the right pixel; a lane past D follows the entry d = 0
+    if (xt < 0) xt += W;          // seq/PixelBasedCost.cpp:19-20 (D <= W)
+    const uint32_t uW = (uint32_t)W;
+    const size_t first = ((size_t)ra * W + xc) * D + (dok ? d : 0);
+    const In *__restrict__ lp = reinterpret_cast<const In *>(V.seg) + first;
+    const In *__restrict__ rp = reinterpret_cast<const In *>(VR.seg) + first;
+    const uint2 *__restrict__ refp = V.aref + (size_t)ra * W + xc, *__restrict__ tarp = V.atar + (size_t)ra * W + xt;
+    const int nrows = rb - ra;  // rows that enter
+    // four rows' loads, in flight while the previous four are used
+    In pl[S], pr[S];
+    uint2 ptar[S], pref[S];
+    const uint32_t uWD = (uint32_t)W * (uint32_t)D;  // 3 W D below 2^32 (shared pairs)
+    auto load_rows = [&](int i) {
+        if (S * (i + 1) <= nrows) {
+#pragma unroll
+            for (uint32_t k = 0; k < S; k++) {
+                pref[k] = __ldg(refp + k * uW);
+                ptar[k] = __ldg(tarp + k * uW);
+                pl[k] = __ldg(lp + k * uWD);
+                pr[k] = __ldg(rp + k * uWD);
+            }
+        } else {
+            // the last rows, and rows with empty arms past them
+#pragma unroll
+            for (uint32_t k = 0; k < S; k++) {
+                const bool in = S * i + (int)k < nrows;
+                pref[k] = in ? __ldg(refp + k * uW) : make_uint2(0u, 0u);
+                ptar[k] = in ? __ldg(tarp + k * uW) : make_uint2(0u, 0u);
+                pl[k] = in ? __ldg(lp + k * uWD) : In(0);
+                pr[k] = in ? __ldg(rp + k * uWD) : In(0);
+            }
+        }
+        refp += (size_t)S * uW;
+        tarp += (size_t)S * uW;
+        lp += (size_t)S * uWD;
+        rp += (size_t)S * uWD;
+    };
+    int ts = 0;        // ring slot of the next rows to enter
+    uint32_t cnt = 0;  // running sum of l + r of the column in the low half
+    uint32_t ql = 0, qr = 0;
+    auto ingest = [&](int i) {
+        uint32_t w[S];
+#pragma unroll
+        for (int k = 0; k < S; k++) {
+            // arm words {l | r << 16, t | b << 16}: minima of the two pixels'
+            const uint32_t lr = __vminu2(pref[k].x, ptar[k].x), tb = __vminu2(pref[k].y, ptar[k].y);
+            cnt = __dp2a_lo(lr, 0x0101u, cnt);        // + l + r
+            w[k] = __byte_perm(cnt, tb, 0x6410);      // low half | t << 16 | b << 24
+        }
+#pragma unroll
+        for (int k = 0; k < S; k++) wrd[32 * (ts + k)] = w[k];
+        if constexpr (INT) {
+#pragma unroll
+            for (int k = 0; k < S; k++) {
+                ql += pl[k];
+                qr += pr[k];
+                Ql[32 * (ts + k)] = ql;
+                Qr[32 * (ts + k)] = qr;
+            }
+        } else {
+            segl[8 * ts] = RG::pack(pl);  // group ts / 4
+            segr[8 * ts] = RG::pack(pr);
+        }
+        ts += S;
+        if (ts == DEP) ts = 0;
+        load_rows(i + 1);
+    };
+    wrd[32 * (DEP - 1)] = 0u;  // the running sums before row ra
+    if constexpr (INT) Ql[32 * (DEP - 1)] = Qr[32 * (DEP - 1)] = 0u;
+    load_rows(0);
+    const int T0 = vert_lane_first(y0, ra, L);
+    int i = 0;
+    for (; i < T0 - 1; i++) ingest(i);
+    const uint32_t end = (uint32_t)DEP * 128u;        // ring bytes of a lane's words
+    uint32_t at0 = (uint32_t)(y0 - ra) * 128u;        // byte offset of the step's first output row (< end)
+    const unsigned char *wb = reinterpret_cast<const unsigned char *>(wrd);
+    auto word = [&](const void *b, uint32_t o) {
+        return *reinterpret_cast<const uint32_t *>(reinterpret_cast<const unsigned char *>(b) + o);
+    };
+    unsigned long long *bp = V.best_r + (size_t)y0 * W + xt;
+    uint16_t *rawx = V.raw + (size_t)y0 * W + xg;
+    int *rowl = V.row_last;
+    uint32_t *kt = keys;
+    for (int y = y0; y < y1; y += S, i++) {
+        ingest(i);
+        const int nj = imin(S, y1 - y);  // output rows of the step (the others' results are dropped)
+        uint32_t key[S];
+        if (live) {
+            float al[S], ar[S], cf[S], rcb[S];  // sums; pixel count and its reciprocal
+            int st[S], ln[S];  // first row of the arm, from the step's first output row; its rows
+#pragma unroll
+            for (int j = 0; j < S; j++) {
+                uint32_t at = at0 + 128u * j;
+                at = min(at, at - end);  // the ring's wrap, by an unsigned minimum
+                const uint32_t w = word(wb, at), t = __byte_perm(w, 0, 0x4442), b = w >> 24;
+                st[j] = j - (int)t;
+                ln[j] = (int)(t + b) + 1;
+                // l + r over the arm's rows: running sums at rows y + b and y - t - 1
+                const uint32_t up = at + 128u * b, dn = at - 128u * t - 128u;
+                const uint32_t oh = min(up, up - end), ol = min(dn, dn + end);
+                const uint32_t cn = ((word(wb, oh) - word(wb, ol)) & 0xffffu) + (uint32_t)ln[j];
+                cf[j] = __uint2float_rn(cn);
+                rcb[j] = __ldg(rcp + cn);  // 1 .. (2 L + 1)^2, of any row in the ring
+                if constexpr (INT) {
+                    al[j] = __uint2float_rn(word(Ql, oh) - word(Ql, ol));
+                    ar[j] = __uint2float_rn(word(Qr, oh) - word(Qr, ol));
+                } else {
+                    al[j] = ar[j] = 0.f;
+                }
+            }
+            if constexpr (!INT) {
+                // rows lo .. hi - 1 hold every lane's arms
+                int lo = imin(imin(st[0], st[1]), imin(st[2], st[3]));
+                int hi = imax(imax(st[0] + ln[0], st[1] + ln[1]), imax(st[2] + ln[2], st[3] + ln[3]));
+                lo = __reduce_min_sync(0xffffffffu, lo);
+                hi = __reduce_max_sync(0xffffffffu, hi);
+                int g = (int)(at0 >> 7) + lo;  // ring slot of row lo
+                g = g < 0 ? g + DEP : g;
+                g = g >= DEP ? g - DEP : g;
+                const int base = lo - (g & 3);  // the aligned group's first row
+                uint32_t m[S];
+#pragma unroll
+                for (int j = 0; j < S; j++)
+                    asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(m[j]) : "r"(st[j] - base), "r"(ln[j]));
+                const int ng = (hi - base + 3) >> 2;
+                const G4 *gp = segl + 8 * (g & ~3), *const gend = segl + 8 * DEP;
+                auto walk = [&](int n) {
+                    for (int q = 0; q < n; q++) {
+                        float u[4], v[4];
+                        RG::rows(gp[0], u);
+                        RG::rows(gp[RS], v);
+#pragma unroll
+                        for (int j = 0; j < S; j++) {
+                            add2_if_bit(al[j], ar[j], m[j], 1u, u[0], v[0]);
+                            add2_if_bit(al[j], ar[j], m[j], 2u, u[1], v[1]);
+                            add2_if_bit(al[j], ar[j], m[j], 4u, u[2], v[2]);
+                            add2_if_bit(al[j], ar[j], m[j], 8u, u[3], v[3]);
+                            m[j] >>= 4;
+                        }
+                        gp += 32;
+                        if (gp == gend) gp = segl;
+                    }
+                };
+                walk(imin(ng, 8));
+                if (ng > 8) {
+                    // rows 32 .. of long arms (at most 2 L + 7 < 64 rows in all)
+#pragma unroll
+                    for (int j = 0; j < S; j++) {
+                        const int f = st[j] - base - 32, f0 = imax(f, 0);
+                        asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(m[j]) : "r"(f0), "r"(imax(f + ln[j] - f0, 0)));
+                    }
+                    walk(ng - 8);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < S; j++) {
+                // sums of non-negative costs: the correctly rounded quotient by Markstein's
+                // correction from a correctly rounded reciprocal (Markstein 1990; exact residual
+                // by FMA), and the bits of a non-negative float order like the float
+                auto quot = [&](float a) {
+                    const float q0 = __fmul_rn(a, rcb[j]);
+                    return __float_as_uint(__fmaf_rn(__fmaf_rn(-cf[j], q0, a), rcb[j], q0));
+                };
+                key[j] = quot(al[j]);
+                if (dok && j < nj) atomicMin(bp + (uint32_t)j * uW, ((unsigned long long)quot(ar[j]) << 32) | (unsigned)d);
+            }
+            bp += (size_t)S * uW;
+        }
+        at0 += 128u * S;
+        at0 = min(at0, at0 - end);
+#pragma unroll
+        for (int j = 0; j < S; j++) kt[j * NWB * 32 + 32 * warp + lane] = dok ? key[j] : 0xffffffffu;
+        // every row of the step is in the tile; the step after next writes this buffer again,
+        // which all warps have read by the next step's barrier
+        __syncthreads();
+        // results (output row j, column col): one warp each, a lane on one key of each chunk
+        auto results = [&](auto lc) {
+            constexpr int LC = decltype(lc)::value, NCH = 1 << LC;
+            for (int q = warp; q < (S * NWB) >> LC; q += NWB) {
+                const int j = q & (S - 1), col = q >> 2;
+                const uint32_t *kr = kt + j * NWB * 32 + 32 * NCH * col + lane;
+                uint32_t bk = kr[0], bd = lane;
+#pragma unroll
+                for (int n = 1; n < NCH; n++) {
+                    const uint32_t k = kr[32 * n];
+                    if (k < bk) {  // strict: the lowest d keeps ties
+                        bk = k;
+                        bd = 32 * n + lane;
+                    }
+                }
+                const uint32_t mn = __reduce_min_sync(0xffffffffu, bk);
+                bd = __reduce_min_sync(0xffffffffu, bk == mn ? bd : 0xffffu);
+                if (lane == 0 && j < nj && xg + col < W) {
+                    const bool found = bd != 0;  // some d >= 1 strictly below cost[0]
+                    rawx[(uint32_t)j * uW + col] = found ? (uint16_t)(0x100 | bd) : (uint16_t)0;
+                    if (found) atomicMax(rowl + y + j, xg + col);
+                }
+            }
+        };
+        if (lognch == 2) results(std::integral_constant<int, 2>{});
+        else if (lognch == 1) results(std::integral_constant<int, 1>{});
+        else if (lognch == 0) results(std::integral_constant<int, 0>{});
+        else if constexpr (NWB == 8) results(std::integral_constant<int, 3>{});
+        rawx += (size_t)S * uW;
+        kt = kt == keys ? keys + S * NWB * 32 : keys;
+    }
+}
+
+template <typename ST, int NWB>
+__global__ void __launch_bounds__(NWB * 32, NWB == 4 ? 3 : 1)
+    k_vert_dual(ViewTable t, int L, int R, int DEP, const float *__restrict__ rcp) {
+    extern __shared__ __align__(16) unsigned char vsm[];
+    const int nv = t.nviews;
+    const int *off = t.off + ST_VERT * (nv + 1);
+    for (int item = blockIdx.x; item < t.total[ST_VERT]; item += gridDim.x) {
+        const int v = find_view(off, nv, item);
+        const ViewDesc &V = t.views[v];
+        const int strips = (V.H + R - 1) / R, local = item - __ldg(off + v);
+        const int lognch = vert_log_chunks(V.D);
+        const int xi = local / strips, y0 = (local - xi * strips) * R;
+        __syncthreads();  // the previous item's reads of the key tile are done
+        dual_item<ST, NWB>(V, t.views[V.partner], xi * (NWB >> lognch), lognch, y0, imin(V.H, y0 + R), L, DEP, rcp,
+                           vsm);
+    }
+}
+
+// best: block per (skewed right view, row); the minima of k_vert_dual into the winner
+// words and row summaries of the view's (mirrored) columns
+__global__ void __launch_bounds__(256) k_best_views(ViewTable t) {
+    const int nv = t.nviews;
+    const int *off = t.off + ST_BEST * (nv + 1);
+    for (int item = blockIdx.x; item < t.total[ST_BEST]; item += gridDim.x) {
+        const int v = find_view(off, nv, item);
+        const ViewDesc &V = t.views[v];
+        const int W = V.W, y = item - __ldg(off + v);
+        const unsigned long long *best = V.best_r + (size_t)y * W;
+        for (int x0 = 0; x0 < W; x0 += 256) {
+            const int x = x0 + (int)threadIdx.x;  // mirrored column
+            const uint32_t win = x < W ? (uint32_t)best[W - 1 - x] : 0u;
+            if (x < W) V.raw[(size_t)y * W + x] = win ? (uint16_t)(0x100 | win) : (uint16_t)0;
+            // some d >= 1 strictly better than d = 0: one maximum a warp
+            const uint32_t last = __reduce_max_sync(0xffffffffu, win ? (uint32_t)x + 1 : 0u);
+            if (last && (threadIdx.x & 31) == 0) atomicMax(V.row_last + y, (int)last - 1);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // fill: warp per (view, row); see k_wta.cu for the carry rule
 __global__ void __launch_bounds__(256) k_fill_views(ViewTable t) {
     const int nv = t.nviews;
@@ -717,11 +1102,20 @@ __global__ void __launch_bounds__(256) k_cc_views(ViewTable t) {
 }
 
 // ---------------------------------------------------------------------------
-int stage_items(int stage, const ViewDesc &v, int vert_rows) {
+// Warps of a k_vert_dual block: the 32-disparity chunks of the launch's widest view (up to
+// 4 chunks share blocks of 4 warps with neighbouring columns).
+static int dual_warps(int max_d) { return max_d <= 128 ? 4 : 8; }
+
+int stage_items(int stage, const ViewDesc &v, int vert_rows, int max_d) {
     switch (stage) {
     case ST_PREP: return v.prep ? 2 * ((v.W + kPrepTW - 1) / kPrepTW) * ((v.H + kPrepTH - 1) / kPrepTH) : 0;
     case ST_HSEG: return v.H * ((v.D + 31) / 32);
-    case ST_VERT: return v.W * ((v.H + vert_rows - 1) / vert_rows);
+    case ST_VERT: {
+        if (v.skew) return 0;  // done with the pair's left view
+        const int cols = v.best_r ? dual_warps(max_d) >> vert_log_chunks(v.D) : 1;  // columns of an item
+        return ((v.W + cols - 1) / cols) * ((v.H + vert_rows - 1) / vert_rows);
+    }
+    case ST_BEST: return v.skew ? v.H : 0;
     case ST_FILL: return v.H;
     case ST_CC: return v.H;
     }
@@ -868,46 +1262,68 @@ rts_status launch_cross_views(rts_ctx *c, const rts_params &p, const ViewTable &
     }
     {
         StageScope sc(c, "cross_vert_wta");
-        const int DEP = vert_depth(L);
-        const int nch = (max_d + 31) / 32;
-        const int NCH = nch <= 1 ? 1 : nch <= 2 ? 2 : nch <= 4 ? 4 : 8;
-        // ring {segment, count} + arm words + reference arm words + target columns
-        const size_t DMb = (size_t)32 * NCH;
-        const size_t smem = (size_t)DEP * DMb * ((segk ? 4 : 8) + 2) + (size_t)DEP * 4 + DMb * 4;
         const int R = tune.vert_rows;
         rts_status vs = RTS_OK;
-        auto go = [&](auto kern) {
-            vs = set_smem(c, kern, smem, "vert_views");
-            if (vs != RTS_OK) return;
-            kern<<<grid(t.total[ST_VERT], 1, resident_blocks(kern, kVertT, smem)), kVertT, smem, s>>>(t, L, R, DEP,
-                                                                                                   rcp);
-        };
-        // non-negative costs take the fast exact division: every cost made from records,
-        // and every precomputed volume but NCC's (AD, rank and LoG differences, Hamming
-        // distances and their CombineCost terms 1 - exp(-v / lambda) are >= 0)
-        const bool pos = mode != 0 || (p.cost1 != RTS_COST_NCC && p.cost2 != RTS_COST_NCC);
-#define RTS_VERT(ST, N)                                   \
-    do {                                                  \
-        if (!pos) go(k_vert_views<ST, N, 0>);             \
-        else go(k_vert_views<ST, N, 1>);                  \
+        if (t.total[ST_BEST] > 0) {
+            // both views of every pair at once (costs from records: all >= 0)
+            auto go = [&](auto kern, int nwb, size_t smem) {
+                vs = set_smem(c, kern, smem, "vert_dual");
+                if (vs != RTS_OK) return;
+                kern<<<grid(t.total[ST_VERT], 1, resident_blocks(kern, 32 * nwb, smem)), 32 * nwb, smem, s>>>(
+                    t, L, R, vert_lane_depth(L), rcp);
+            };
+#define RTS_DUAL(ST)                                                              \
+    do {                                                                          \
+        if (dual_warps(max_d) == 4) go(k_vert_dual<ST, 4>, 4, dual_smem<ST>(4, L)); \
+        else go(k_vert_dual<ST, 8>, 8, dual_smem<ST>(8, L));                       \
     } while (0)
-        if (segk == 2) {
-            if (NCH == 1) go(k_vert_views<uint16_t, 1, 1>);
-            else if (NCH == 2) go(k_vert_views<uint16_t, 2, 1>);
-            else if (NCH == 4) go(k_vert_views<uint16_t, 4, 1>);
-            else go(k_vert_views<uint16_t, 8, 1>);
-        } else if (segk == 1) {
-            if (NCH == 1) RTS_VERT(__half, 1);
-            else if (NCH == 2) RTS_VERT(__half, 2);
-            else if (NCH == 4) RTS_VERT(__half, 4);
-            else RTS_VERT(__half, 8);
+            if (segk == 2) RTS_DUAL(uint16_t);
+            else if (segk == 1) RTS_DUAL(__half);
+            else RTS_DUAL(float);
+#undef RTS_DUAL
+            RTS_TRY(vs);
+            k_best_views<<<grid(t.total[ST_BEST], 1, 8), 256, 0, s>>>(t);
+            count_launch(c);
         } else {
-            if (NCH == 1) RTS_VERT(float, 1);
-            else if (NCH == 2) RTS_VERT(float, 2);
-            else if (NCH == 4) RTS_VERT(float, 4);
-            else RTS_VERT(float, 8);
-        }
+            const int DEP = vert_depth(L);
+            const int nch = (max_d + 31) / 32;
+            const int NCH = nch <= 1 ? 1 : nch <= 2 ? 2 : nch <= 4 ? 4 : 8;
+            // ring {segment, count} + arm words + reference arm words + target columns
+            const size_t DMb = (size_t)32 * NCH;
+            const size_t smem = (size_t)DEP * DMb * ((segk ? 4 : 8) + 2) + (size_t)DEP * 4 + DMb * 4;
+            auto go = [&](auto kern) {
+                vs = set_smem(c, kern, smem, "vert_views");
+                if (vs != RTS_OK) return;
+                kern<<<grid(t.total[ST_VERT], 1, resident_blocks(kern, kVertT, smem)), kVertT, smem, s>>>(t, L, R, DEP,
+                                                                                                       rcp);
+            };
+            // non-negative costs take the fast exact division: every cost made from records,
+            // and every precomputed volume but NCC's (AD, rank and LoG differences, Hamming
+            // distances and their CombineCost terms 1 - exp(-v / lambda) are >= 0)
+            const bool pos = mode != 0 || (p.cost1 != RTS_COST_NCC && p.cost2 != RTS_COST_NCC);
+#define RTS_VERT(ST, N)                                   \
+        do {                                                  \
+            if (!pos) go(k_vert_views<ST, N, 0>);             \
+            else go(k_vert_views<ST, N, 1>);                  \
+        } while (0)
+            if (segk == 2) {
+                if (NCH == 1) go(k_vert_views<uint16_t, 1, 1>);
+                else if (NCH == 2) go(k_vert_views<uint16_t, 2, 1>);
+                else if (NCH == 4) go(k_vert_views<uint16_t, 4, 1>);
+                else go(k_vert_views<uint16_t, 8, 1>);
+            } else if (segk == 1) {
+                if (NCH == 1) RTS_VERT(__half, 1);
+                else if (NCH == 2) RTS_VERT(__half, 2);
+                else if (NCH == 4) RTS_VERT(__half, 4);
+                else RTS_VERT(__half, 8);
+            } else {
+                if (NCH == 1) RTS_VERT(float, 1);
+                else if (NCH == 2) RTS_VERT(float, 2);
+                else if (NCH == 4) RTS_VERT(float, 4);
+                else RTS_VERT(float, 8);
+            }
 #undef RTS_VERT
+        }
         RTS_TRY(vs);
         count_launch(c);
     }

@@ -869,7 +869,7 @@ bool cross_fused_supported(const rts_params &p) {
 
 bool cross_ragged_supported(const rts_params &p) {
     // The view kernels take any range, with the results of the composed module kernels
-    // (450x375, D = 60: 571 us a pair composed, 374 us here) where costs are made from records
+    // (450x375, D = 60, photo: 571 us a pair composed, 256 us here) where costs are made from records
     // and are >= 0 (their quotients take the fast exact division): positive lambdas, no
     // negative truncation.  Other costs stay composed.
     return p.aggr == RTS_AGGR_CROSS && p.cross_arm <= 23 && p.disp_range % 8 != 0 && cross_record_costs(p) &&

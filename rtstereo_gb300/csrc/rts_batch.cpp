@@ -89,6 +89,8 @@ GraphCache *cache_of(rts_ctx *c) {
 // holds the median-filtered arm images, left and right of every pair.
 void fill_views(ViewBatch &b, int n, const rts_pair *pairs, const rts_out *outs, int right,
                 const std::vector<uint8_t *> *med) {
+    bool shared = true;  // all pairs of a launch or none
+    for (const ViewDesc &v : b.views) shared = shared && (size_t)v.W * v.D < (size_t(1) << 30);
     for (int i = 0; i < n; i++) {
         const rts_pair &q = pairs[i];
         ViewDesc &l = b.views[right ? 2 * i : i];
@@ -106,7 +108,8 @@ void fill_views(ViewBatch &b, int n, const rts_pair *pairs, const rts_out *outs,
             r.disp = outs[i].disp_right;
             r.vol = nullptr;
             l.mask = outs[i].mask;
-            link_pair(&b, 2 * i, 2 * i + 1);
+            // (the shared kernel's row offsets are 32-bit)
+            link_pair(&b, 2 * i, 2 * i + 1, shared);
         }
     }
 }
@@ -248,14 +251,15 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
         tit = gc->tunes.emplace(key, ft).first;
     }
     if (tit == gc->tunes.end() && optional) {
-        // strips that give the vertical kernel some eight blocks for each of two an SM
-        long cols = 0;
+        // strips that give the vertical kernel some five blocks an SM (450x375, D = 60, photo: strips
+        // of 375 rows 263 us, of 96 rows 161, of 48 rows 170), none shorter than 64 rows
+        long items = 0;
         int h = 1;
-        for (int i = 0; i < nv; i++) {
-            cols += W[i];
-            h = std::max(h, H[i]);
+        for (const ViewDesc &v : b.views) {
+            items += stage_items(ST_VERT, v, v.H, b.max_d);
+            h = std::max(h, v.H);
         }
-        const long strips = std::min((16L * sm_count() + cols - 1) / cols, (h + 95L) / 96);
+        const long strips = std::max(1L, std::min((5L * sm_count() + items - 1) / std::max(items, 1L), h / 64L));
         CrossTune ft;
         ft.vert_rows = (int)((h + strips - 1) / strips);
         tit = gc->tunes.emplace(key, ft).first;

@@ -363,7 +363,7 @@ static rts_status pipeline_cross_views(rts_ctx *c, const rts_params &p, int H, i
         ViewDesc &v1 = b.views[1];
         v1.gref = rg; v1.gtar = lg; v1.cref = rc; v1.ctar = lc; v1.mirror = 1; v1.disp = dr;
         v0.mask = mask;
-        link_pair(&b, 0, 1);
+        link_pair(&b, 0, 1, false);
     }
     int has_vol = 0;
     if (!cross_record_costs(p)) {

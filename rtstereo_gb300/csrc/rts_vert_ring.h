@@ -12,7 +12,7 @@
 // step s: the newest row then written and the oldest row still read must not
 // share a slot.
 //
-// Lane rings (k_cross_vol, k_cross_mod.cu).  A lane alone writes and reads its ring,
+// Lane rings (k_vert_dual, k_batch.cu; k_cross_vol, k_cross_mod.cu).  A lane alone writes and reads its ring,
 // so nothing but its own program order matters.  Rows enter kVertStep at a time;
 // step s (output rows y0 + 4 s .. + 3) first lets tick vert_lane_first - 1 + s in,
 // then reads rows y - L - 1 (the running count before the arm) .. y + L of its
@@ -54,5 +54,8 @@ __host__ __device__ constexpr int vert_lane_first(int y0, int ra, int L) {
 __host__ __device__ constexpr int vert_lane_depth(int L) {
     return kVertStep * ((2 * L + 2 * kVertStep + kVertStep - 1) / kVertStep);
 }
+
+// log2 of the power of two that covers D disparities in chunks of 32 (D <= 256)
+__host__ __device__ constexpr int vert_log_chunks(int D) { return D <= 32 ? 0 : D <= 64 ? 1 : D <= 128 ? 2 : 3; }
 
 }  // namespace rts

@@ -58,8 +58,12 @@ void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n,
     b->table = a + pos;
 }
 
-void link_pair(ViewBatch *b, int left, int right) {
+void link_pair(ViewBatch *b, int left, int right, bool shared) {
     ViewDesc &l = b->views[left], &r = b->views[right];
+    // the minima (8 bytes a pixel) take the place of the right view's own records (32), which
+    // a linked pair does not use
+    if (shared) l.best_r = r.best_r = (unsigned long long *)r.rref;
+    r.skew = shared ? 1 : 0;
     l.prep = 1;
     l.partner = right;
     r.prep = 0;
@@ -89,7 +93,7 @@ rts_status upload_views(rts_ctx *c, const ViewBatch &bc, const CrossTune &tune, 
         o[0] = 0;
         for (int i = 0; i < n; i++) {
             const ViewDesc &v = b.views[i];
-            int items = stage_items(s, v, tune.vert_rows);
+            int items = stage_items(s, v, tune.vert_rows, b.max_d);
             if (s == ST_CC && (v.partner < 0 || !v.mask)) items = 0;
             o[i + 1] = o[i] + items;
         }

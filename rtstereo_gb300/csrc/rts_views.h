@@ -29,6 +29,9 @@ struct ViewDesc {
     uint4 *rref, *rtar;          // per-pixel records {census lo, census hi, colour, l | r<<16}, image coordinates
     uint2 *aref, *atar;          // per-pixel arm words {l | r<<16, t | b<<16}, image coordinates
     void *seg;                   // row segments [H][W][D] in view coordinates, float or __half
+    unsigned long long *best_r;  // pairs whose views share the vertical kernel (both): minima {key, d} per
+                                 // right image pixel, or nullptr
+    int skew;                    // 1: such a pair's right view (its segments lie by left image column)
     uint16_t *raw;               // winner | found << 8 per pixel
     int *row_last;               // per row: last x with a winner of its own, -1 if none
     uint8_t *disp;               // output disparity (written mirrored back when mirror)
@@ -38,7 +41,7 @@ struct ViewDesc {
 };
 
 // stage offsets: item k of stage s belongs to view v with off[s][v] <= k < off[s][v+1]
-enum { ST_PREP = 0, ST_HSEG, ST_VERT, ST_FILL, ST_CC, ST_COUNT };
+enum { ST_PREP = 0, ST_HSEG, ST_VERT, ST_BEST, ST_FILL, ST_CC, ST_COUNT };
 
 struct ViewTable {
     const ViewDesc *views;  // device
@@ -55,7 +58,8 @@ struct CrossTune {
 };
 
 // Per-view item counts (host): the layout the kernels and the planner share.
-int stage_items(int stage, const ViewDesc &v, int vert_rows);
+// (max_d: the largest disparity range of the launch).
+int stage_items(int stage, const ViewDesc &v, int vert_rows, int max_d);
 
 // The costs the cross-based view kernels make from per-pixel records: AD and
 // census (alone or combined), and rank differences combined with census.
@@ -80,7 +84,7 @@ rts_status launch_cross_views(rts_ctx *c, const rts_params &p, const ViewTable &
 struct ViewBatch {
     std::vector<ViewDesc> views;     // host copy
     std::vector<int> off;            // [ST_COUNT][n + 1]
-    int total[ST_COUNT] = {0, 0, 0, 0, 0};
+    int total[ST_COUNT] = {0};
     int max_d = 0;
     int *row_last_all = nullptr;     // device, contiguous over views
     size_t row_last_count = 0;
@@ -99,7 +103,8 @@ size_t views_bytes(const int *W, const int *H, const int *D, int n, int half);
 void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n, int half, ViewBatch *b);
 // Makes views `left` and `right` one pair: the left view makes the records of
 // both images, the right view reads them (its reference is the right image).
-void link_pair(ViewBatch *b, int left, int right);
+// shared: the vertical sums of both views come from one kernel (record costs only).
+void link_pair(ViewBatch *b, int left, int right, bool shared);
 // Computes the stage offsets, copies the view table and offsets to the device
 // (through the pinned buffer `stage` when given, else directly) and fills `t`.
 rts_status upload_views(rts_ctx *c, const ViewBatch &b, const CrossTune &tune, void *stage, ViewTable *t);
