@@ -610,7 +610,7 @@ void launch_box(cudaStream_t s, const float *in, float *out, int H, int W, int D
         const size_t smem = (size_t)(kBoxDpTX + 2 * R) * (kBoxDpTY + 2 * R) * 32 * dw * sizeof(float);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         CUtensorMap tm{};
-        const int use_tma = volume_tensor_map(&tm, in, H, W, D, 4, 32 * dw, kBoxDpTX + 2 * R, kBoxDpTY + 2 * R) ? 1 : 0;
+        const int use_tma = volume_tensor_map(&tm, in, H, W, D, D, 4, 32 * dw, kBoxDpTX + 2 * R, kBoxDpTY + 2 * R) ? 1 : 0;
         const int wide = D % 2 == 0 && ((uintptr_t)in & 7) == 0 ? 1 : 0;
         const dim3 g((W + kBoxDpTX - 1) / kBoxDpTX, (H + kBoxDpTY - 1) / kBoxDpTY, (D + 32 * dw - 1) / (32 * dw));
         kern<<<g, 256, smem, s>>>(tm, use_tma, in, out, H, W, D, wide, 1.0f / (float)area);
@@ -653,7 +653,7 @@ void launch_box_best(cudaStream_t s, const float *vol, unsigned long long *best,
         const size_t smem = (size_t)(kBoxDpTX + 2 * R) * (kBoxDpTY + 2 * R) * 64 * sizeof(float);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         CUtensorMap tm{};
-        const int use_tma = volume_tensor_map(&tm, vol, H, W, D, 4, 64, kBoxDpTX + 2 * R, kBoxDpTY + 2 * R) ? 1 : 0;
+        const int use_tma = volume_tensor_map(&tm, vol, H, W, D, D, 4, 64, kBoxDpTX + 2 * R, kBoxDpTY + 2 * R) ? 1 : 0;
         kern<<<g, 256, smem, s>>>(tm, use_tma, vol, best, best_r, H, W, D, argmax, rcp_area);
     };
 #define RTS_BOX(RR)                                                \

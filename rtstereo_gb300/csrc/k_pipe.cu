@@ -74,14 +74,14 @@ __global__ void k_prep_records(const uint8_t *__restrict__ gray, const uint8_t *
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_cost_volume(const uint4 *__restrict__ rr, const uint4 *__restrict__ rt, T *__restrict__ vol, int H,
-                              int W, int D, CostCfg cfg) {
+                              int W, int D, int pitch, CostCfg cfg) {
     const int y = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= W * D) return;
     const int x = i / D, d = i - x * D;
     const int xt = tar_col(x, d, W, 1);
     const uint4 a = rr[(size_t)y * W + x], b = rt[(size_t)y * W + xt];
-    vol[((size_t)y * W + x) * D + d] = to_store<T>(pair_cost(a, b, cfg));
+    vol[((size_t)y * W + x) * pitch + d] = to_store<T>(pair_cost(a, b, cfg));
 }
 
 // AD (optionally truncated) + census combined through the two host tables, the
@@ -96,7 +96,7 @@ constexpr int kAdcTX = 8 * kAdcPx;          // pixels of a block
 constexpr int kAdcL1 = 768, kAdcL2 = 68;    // table entries staged: AD <= 765, census <= 64
 template <typename T>
 __global__ void __launch_bounds__(256) k_cost_volume_adc(const uint4 *__restrict__ rr, const uint4 *__restrict__ rt,
-                                                        T *__restrict__ vol, int H, int W, int D, int itrunc,
+                                                        T *__restrict__ vol, int H, int W, int D, int pitch, int itrunc,
                                                         const float *__restrict__ lut1, const float *__restrict__ lut2) {
     __shared__ uint4 trec[kAdcTX + 255];  // D <= 256
     __shared__ float t1[kAdcL1], t2[kAdcL2];
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) k_cost_volume_adc(const uint4 *__restrict
         const int x = xw + i;
         if (x >= W) return;
         const uint4 a = rr[(size_t)y * W + x];
-        T *out = vol + ((size_t)y * W + x) * D;
+        T *out = vol + ((size_t)y * W + x) * pitch;
         const uint4 *tb = trec + (x - base);  // target of disparity d: tb[-d]
         for (int d = lane; d < D; d += 32) {
             const uint4 b = tb[-d];
@@ -405,7 +405,9 @@ __global__ void __launch_bounds__(kAwThreads, 3) k_aw_wta(const CT *__restrict__
 // taps (their table reads in flight across a group), and the Lab rows of
 // ky + 2 are staged; one barrier per tap row.  The arithmetic per entry is
 // k_aw_wta's: EXACT (plain form, f32 volume) the reference's order, unfused;
-// otherwise (FP16 form, f16 volume staged as f16, D a multiple of 8) one FMA.
+// otherwise (FP16 form, f16 volume staged as f16, a pitch that is a multiple of 8) one
+// FMA.  pitch: values from pixel to pixel of the volume, at least D; cells past D belong to
+// no disparity, and the sums they enter are dropped.
 // E: the window edge as a constant (33, the reference driver's 33 x 33 window), so
 // that the tap loop unrolls whole, or 0 for the edge of the e argument.
 __device__ int g_aw_tma_timeouts;
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(kAwThreads, 2) k_aw_wta_pipe(const __grid_cons
                                                           const uint32_t *__restrict__ labt,
                                                           const float *__restrict__ pw, const float *__restrict__ G,
                                                           uint16_t *__restrict__ raw, int *__restrict__ row_last,
-                                                          float *__restrict__ cost_out, int H, int W, int D, int e_arg,
+                                                          float *__restrict__ cost_out, int H, int W, int D, int pitch, int e_arg,
                                                           float zero) {
     const int e = E ? E : e_arg;
     const int r = e >> 1;
@@ -469,7 +471,7 @@ __global__ void __launch_bounds__(kAwThreads, 2) k_aw_wta_pipe(const __grid_cons
         best_v[tid] = __int_as_float(0x7f800000);
         best_i[tid] = 0x7fffffff;
     }
-    const bool vec = (D & 3) == 0;
+    const bool vec = (pitch & 3) == 0;
     const bool tma_tile = sizeof(CT) == 4 && use_tma && x0 - r >= 0 && x0 + kAwTX + r <= W &&
                           ((uint32_t)__cvta_generic_to_shared(psm_) & 127) == 0;
     const uint32_t cb0 = (uint32_t)__cvta_generic_to_shared(cbar);
@@ -525,12 +527,12 @@ __global__ void __launch_bounds__(kAwThreads, 2) k_aw_wta_pipe(const __grid_cons
                 return;
             }
             if constexpr (sizeof(CT) == 2) {
-                // f16 volume: 16-byte copies of 8 disparities (D is a multiple of 8)
+                // f16 volume: 16-byte copies of 8 disparities (the pitch is a multiple of 8)
                 for (int q = tid; q < (kAwTX + 2 * r) * (kAwDC / 8); q += kAwThreads) {
                     const int xi = q >> 3, d8 = (q & 7) * 8;
                     const int xs = imin(imax(wrap1(x0 - r + xi, W), 0), W - 1);
                     const int dg = dc0 + d8;
-                    const CT *src = vol + (crow + xs) * D + (dg < D ? dg : 0);
+                    const CT *src = vol + (crow + xs) * pitch + (dg < D ? dg : 0);
                     const uint32_t dst = cbase + (uint32_t)((xi * CP + d8) * 2);
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src),
                                  "r"(dg < D ? 16 : 0)
@@ -541,7 +543,7 @@ __global__ void __launch_bounds__(kAwThreads, 2) k_aw_wta_pipe(const __grid_cons
                     const int xi = q >> 4, d4 = (q & 15) * 4;
                     const int xs = imin(imax(wrap1(x0 - r + xi, W), 0), W - 1);
                     const int dg = dc0 + d4;
-                    const float *src = vol + (crow + xs) * D + (dg < D ? dg : 0);
+                    const float *src = vol + (crow + xs) * pitch + (dg < D ? dg : 0);
                     const uint32_t dst = cbase + (uint32_t)((xi * CP + d4) * 4);
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src),
                                  "r"(dg < D ? 16 : 0)
@@ -552,7 +554,7 @@ __global__ void __launch_bounds__(kAwThreads, 2) k_aw_wta_pipe(const __grid_cons
                     const int xi = q >> 6, dd = q & 63;
                     const int xs = imin(imax(wrap1(x0 - r + xi, W), 0), W - 1);
                     const int dg = dc0 + dd;
-                    const float *src = vol + (crow + xs) * D + (dg < D ? dg : 0);
+                    const float *src = vol + (crow + xs) * pitch + (dg < D ? dg : 0);
                     const uint32_t dst = cbase + (uint32_t)((xi * CP + dd) * 4);
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src),
                                  "r"(dg < D ? 4 : 0)
@@ -843,20 +845,20 @@ static rts_status cost_cfg(rts_ctx *c, const rts_params &p, CostCfg *cfg) {
 }
 
 rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const uint4 *rr, const uint4 *rt,
-                            void *vol, int half) {
+                            void *vol, int half, int pitch) {
     CostCfg cfg;
     RTS_TRY(cost_cfg(c, p, &cfg));
     const int D = p.disp_range;
     if (cfg.int_path && cfg.k1 == RTS_COST_AD && cfg.k2 == RTS_COST_CENSUS) {
         const dim3 g((unsigned)((W + kAdcTX - 1) / kAdcTX), H);
-        if (half) k_cost_volume_adc<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, cfg.itrunc, cfg.lut1, cfg.lut2);
-        else k_cost_volume_adc<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, cfg.itrunc, cfg.lut1, cfg.lut2);
+        if (half) k_cost_volume_adc<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, pitch, cfg.itrunc, cfg.lut1, cfg.lut2);
+        else k_cost_volume_adc<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, pitch, cfg.itrunc, cfg.lut1, cfg.lut2);
         count_launch(c);
         return check_launch(c, "cost_volume");
     }
     const dim3 g((unsigned)(((long)W * D + 255) / 256), H);
-    if (half) k_cost_volume<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, cfg);
-    else k_cost_volume<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, cfg);
+    if (half) k_cost_volume<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, pitch, cfg);
+    else k_cost_volume<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, pitch, cfg);
     count_launch(c);
     return check_launch(c, "cost_volume");
 }
@@ -877,7 +879,16 @@ bool cross_ragged_supported(const rts_params &p) {
            (p.cost1 != RTS_COST_AD || p.ad_trunc >= 0.f);
 }
 
-rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, const uint8_t *labr,
+rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W) {
+    const float *t, *t2;
+    void *lp;
+    if (p.cost2 != RTS_COST_NONE) RTS_TRY(combine_luts(c, p.lambda1, p.lambda2, &t, &t2));
+    RTS_TRY(prox_weights(c, p.aw_gamma_p, p.aw_rad, &t));
+    RTS_TRY(lab_weight_lut(c, p.aw_gamma_s, &t));
+    return scratch(c, SL_V_MEAN, (size_t)H * W * 8, &lp);
+}
+
+rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, int pitch, const uint8_t *labr,
                     const uint8_t *labt, uint16_t *raw, int *rl, float *cost_out) {
     const float *pw, *g;
     RTS_TRY(prox_weights(c, p.aw_gamma_p, p.aw_rad, &pw));
@@ -902,9 +913,6 @@ rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *v
     };
     // plain form: bit-exact float volume, the pipelined kernel; FP16 form: __half
     // volume and fused multiply-add
-    // the pipelined kernel: two cost buffers (f32 rows, or f16 rows of 8-disparity
-    // copies; their space also holds the [64][65] argmin staging), two weight
-    // buffers, three Lab row pairs
     // two cost buffers (their space also holds the [64][65] arg-min staging), two
     // weight buffers, three Lab row pairs, the arg-min state and two mbarriers
     auto pipe_smem = [&](size_t row_bytes) {
@@ -915,22 +923,22 @@ rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *v
                2 * kAwTX * 4 + 24;
     };
     CUtensorMap tm{};
-    if (half && p.disp_range % 8 != 0) {
+    if (half && pitch % 8 != 0) {
         RTS_TRY(go(k_aw_wta<__half, false>, (const __half *)vol));
     } else if (half) {
         const size_t psmem = pipe_smem((size_t)kAwHPitch * 2);
         auto kern = e == 33 ? k_aw_wta_pipe<__half, false, 33> : k_aw_wta_pipe<__half, false, 0>;
         RTS_TRY(set_smem(c, kern, psmem, "aw_wta_pipe"));
         kern<<<grid, kAwThreads, psmem, c->stream>>>(tm, 0, (const __half *)vol, plr, plt, pw, g, raw, rl, cost_out,
-                                                     H, W, p.disp_range, e, 0.f);
+                                                     H, W, p.disp_range, pitch, e, 0.f);
     } else {
         // dense 64-float cost rows; the tiles whose columns need no wrap take them by TMA
         const size_t psmem = pipe_smem((size_t)kAwDC * 4);
-        const int use_tma = volume_tensor_map(&tm, vol, H, W, p.disp_range, 4, kAwDC, kAwTX + 2 * r, 1) ? 1 : 0;
+        const int use_tma = volume_tensor_map(&tm, vol, H, W, p.disp_range, pitch, 4, kAwDC, kAwTX + 2 * r, 1) ? 1 : 0;
         auto kern = e == 33 ? k_aw_wta_pipe<float, true, 33> : k_aw_wta_pipe<float, true, 0>;
         RTS_TRY(set_smem(c, kern, psmem, "aw_wta_pipe"));
         kern<<<grid, kAwThreads, psmem, c->stream>>>(tm, use_tma, (const float *)vol, plr, plt, pw, g, raw, rl,
-                                                     cost_out, H, W, p.disp_range, e, 0.f);
+                                                     cost_out, H, W, p.disp_range, pitch, e, 0.f);
     }
     count_launch(c);
     return check_launch(c, "aw_wta");

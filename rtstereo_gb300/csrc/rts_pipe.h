@@ -14,16 +14,19 @@ bool fused_supported(const rts_params &p, int H, int W);
 // 16-byte per-pixel records: census code, packed RGB, packed cross arms
 rts_status prep_records(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *gray, const uint8_t *rgb,
                         uint4 *rec, uint32_t *arms_out);
-// cost volume [H][W][D] (float, or __half when half != 0) from records
+// cost volume [H][W][D] (float, or __half when half != 0), pitch values a pixel, from records
 rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const uint4 *rr, const uint4 *rt,
-                            void *vol, int half);
+                            void *vol, int half, int pitch);
+// allocates what cost_volume_fast and aw_fused will ask for (tables, packed Lab images)
+rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W);
 // the cross-based pipeline runs over view tables (rts_views.h) when this holds
 bool cross_fused_supported(const rts_params &p);
 // ... and for a disparity range that is not a multiple of 8 when this holds (in the plain
 // form, whichever form is asked for: the composed path has no other)
 bool cross_ragged_supported(const rts_params &p);
-// adaptive-weight aggregation + arg-min over a float (half == 0) or __half volume
-rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, const uint8_t *labr,
+// adaptive-weight aggregation + arg-min over a float (half == 0) or __half volume of
+// `pitch` values a pixel
+rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, int pitch, const uint8_t *labr,
                     const uint8_t *labt, uint16_t *raw, int *row_last, float *cost_out);
 
 }  // namespace rts

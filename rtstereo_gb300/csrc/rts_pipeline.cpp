@@ -179,7 +179,7 @@ static rts_status view_composed(rts_ctx *c, const rts_params &p, int H, int W, c
         uint4 *rr = (uint4 *)recv, *rt = rr + np;
         RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr, nullptr));
         RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt, nullptr));
-        RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1, 0));
+        RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1, 0, D));
     } else {
         StageScope sc(c, "cost");
         RTS_TRY(one_cost(c, p, p.cost1, p.aggr == RTS_AGGR_CROSS, H, W, v, c1, SL_V_AUX));
@@ -298,21 +298,33 @@ static rts_status view_fused(rts_ctx *c, const rts_params &p, int H, int W, cons
     }
     const bool fast = fast_costs(p);
     const void *vol = nullptr;
-    int vol_half = 0;
+    int vol_half = 0, pitch = D;
     {
         StageScope sc(c, "cost");
         void *c1v;
         if (fast) {
             vol_half = half ? 1 : 0;
             RTS_TRY(scratch(c, SL_V_COST1, ne * (half ? 2 : 4), &c1v));
-            RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1v, vol_half));
+            // a range that is not whole 16-byte runs: the volume with its pixels that far apart, in
+            // optional scratch (taken after every other allocation of the view), so that the
+            // aggregation reads it by wide copies
+            const int run = half ? 8 : 4;
+            if (D % run) {
+                RTS_TRY(aw_reserve(c, p, H, W));
+                const int wide = (D + run - 1) / run * run;
+                if (void *w = stream_work(c, np * wide * (half ? 2 : 4))) {
+                    c1v = w;
+                    pitch = wide;
+                }
+            }
+            RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1v, vol_half, pitch));
         } else {
             RTS_TRY(scratch(c, SL_V_COST1, ne * 4, &c1v));
             RTS_TRY(cost_volume_composed(c, p, H, W, v, (float *)c1v));
         }
         vol = c1v;
     }
-    RTS_TRY(aw_fused(c, p, H, W, vol, vol_half, v.lref, v.ltar, (uint16_t *)raw, (int *)rl, cost_out));
+    RTS_TRY(aw_fused(c, p, H, W, vol, vol_half, pitch, v.lref, v.ltar, (uint16_t *)raw, (int *)rl, cost_out));
     {
         StageScope sc(c, "wta_fill");
         launch_wta_fill(s, (const uint16_t *)raw, (const int *)rl, disp, H, W, mirror);

@@ -9,12 +9,12 @@
 
 namespace rts {
 
-// The volume [H][W][D] of elem-byte values as a 3-D tensor map (d, x, y) with box
-// (bd, bw, bh), zeros past the edges.  False where a TMA rule fails (rows of D
-// values a multiple of 16 bytes, a 16-byte aligned base, boxes of at most 256 per
+// The volume [H][W][D] of elem-byte values, `pitch` values from pixel to pixel, as a 3-D
+// tensor map (d, x, y) with box (bd, bw, bh), zeros past the edges.  False where a TMA rule
+// fails (the pitch a multiple of 16 bytes, a 16-byte aligned base, boxes of at most 256 per
 // dimension) or the driver has no encoder; callers then stage by cp.async.
-inline bool volume_tensor_map(CUtensorMap *m, const void *vol, int H, int W, int D, int elem, int bd, int bw,
-                              int bh) {
+inline bool volume_tensor_map(CUtensorMap *m, const void *vol, int H, int W, int D, int pitch, int elem, int bd,
+                              int bw, int bh) {
     // looked up once (a function-local static: thread-safe initialisation)
     static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
         void *fn = nullptr;
@@ -24,10 +24,10 @@ inline bool volume_tensor_map(CUtensorMap *m, const void *vol, int H, int W, int
                         q == cudaDriverEntryPointSuccess;
         return ok ? (PFN_cuTensorMapEncodeTiled_v12000)fn : (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
     }();
-    if (!encode || ((size_t)D * elem) % 16 != 0 || ((uintptr_t)vol & 15) != 0) return false;
+    if (!encode || ((size_t)pitch * elem) % 16 != 0 || ((uintptr_t)vol & 15) != 0) return false;
     if (bd > 256 || bw > 256 || bh > 256 || ((size_t)bd * elem) % 16 != 0) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)W, (cuuint64_t)H};
-    const cuuint64_t strides[2] = {(cuuint64_t)D * elem, (cuuint64_t)W * D * elem};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch * elem, (cuuint64_t)W * pitch * elem};
     const cuuint32_t box[3] = {(cuuint32_t)bd, (cuuint32_t)bw, (cuuint32_t)bh};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapDataType t = elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;

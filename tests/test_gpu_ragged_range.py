@@ -83,3 +83,23 @@ def test_captured_call(oracle_mod):
         ctx.set_stream(None)
     o = oracle_mod.pipeline(oracle_mod.params(D=D), L, Rr, *pair(5, W, H, D, False)[1])
     assert bits_equal(want[0], o[0]) and bits_equal(want[1], o[1])
+
+
+# adaptive weights: volumes whose pixels are not whole 16-byte runs, one and two disparity chunks
+@pytest.mark.parametrize("D", [1, 5, 20, 62, 67])
+@pytest.mark.parametrize("rad", [3, 16])
+def test_adaptive_weights(ctx, oracle_mod, D, rad):
+    import rtstereo_gb300 as R
+    W, H = 90, 21
+    (L, Rr), (Lc, Rc) = pair(D, W, H, D, True)
+    ll, rl = R.rgb_to_lab(Lc), R.rgb_to_lab(Rc)
+    got = ctx.pipeline(R.params(disp_range=D, aggr=2, aw_rad=rad), L, Rr, Lc, Rc, ll, rl, want_cost=True)
+    o = oracle_mod.pipeline(oracle_mod.params(D=D, aggr=2, aw_rad=rad), L, Rr, Lc, Rc, ll, rl, want_cost=True)
+    for a, b in zip(got, o):
+        assert bits_equal(a, b)
+    # FP16: an entry does not depend on the range it is computed in
+    wide = (D + 7) // 8 * 8
+    f = [ctx.pipeline(R.params(disp_range=d, aggr=2, aw_rad=rad, precision=1), L, Rr, Lc, Rc, ll, rl, want_cost=True)
+         for d in (D, wide)]
+    assert bits_equal(f[0][3], np.ascontiguousarray(f[1][3][:, :, :D]))
+    assert bits_equal(f[0][0], oracle_mod.wta(f[0][3]))
