@@ -228,61 +228,99 @@ __global__ void __launch_bounds__(kBitsT) k_bits_pack(const uint8_t *__restrict_
 }
 
 // ---------------------------------------------------------------------------
-// Rank transform (seq/RankFilter.cpp:11-35): 1 + #{q : I(q) < I(p)}, u8 wrap.
-__global__ void k_rank(const uint8_t *__restrict__ img, uint8_t *__restrict__ out, int m, int H, int W) {
-    const int y = blockIdx.y;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= W) return;
-    const uint8_t c = img[(size_t)y * W + x];
-    int cnt = 1;
-    for (int dy = -m; dy <= m; dy++) {
-        const uint8_t *row = img + (size_t)wrap1(y + dy, H) * W;
-        for (int dx = -m; dx <= m; dx++) cnt += (row[wrap1(x + dx, W)] < c) ? 1 : 0;
+// Window filters of an image: rank, LoG convolution, window mean.  Block per 64 x 16
+// pixels; their wrapped border is staged in shared memory once (single wrap: radii are
+// below the image's sides), a thread makes four pixels of a column.  A window of up to
+// kWinMax pixels of border takes them; WR, WC: the radii as constants (the usual windows,
+// loops unrolled) or -1.  Bound: the window's shared-memory reads and operations
+// (1280x720: rank 7x7 33 us, LoG 5x5 21 us an image when every window pixel was a
+// wrapped read of the image; 14 and 13 us now).
+constexpr int kWinTX = 64, kWinTY = 16, kWinT = 256, kWinMax = 64;
+static size_t win_smem(int hr, int wr) { return (size_t)(kWinTY + 2 * hr) * (kWinTX + 2 * wr); }
+
+template <typename F, int WR, int WC>
+__global__ void __launch_bounds__(kWinT) k_window(const uint8_t *__restrict__ img, typename F::Out *__restrict__ out,
+                                                  F f, int H, int W, int hr_, int wr_) {
+    extern __shared__ uint8_t wt[];  // [16 + 2 hr][64 + 2 wr]
+    const int hr = WR >= 0 ? WR : hr_, wr = WC >= 0 ? WC : wr_;
+    const int tw = kWinTX + 2 * wr, th = kWinTY + 2 * hr, x0 = blockIdx.x * kWinTX, y0 = blockIdx.y * kWinTY;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int r = warp; r < th; r += kWinT / 32) {
+        // rows and columns past the last pixel's window are clamped into range (never used)
+        const uint8_t *row = img + (size_t)wrap1(imin(y0 - hr + r, H - 1 + hr), H) * W;
+        for (int c = lane; c < tw; c += 32) wt[r * tw + c] = row[wrap1(imin(x0 - wr + c, W - 1 + wr), W)];
     }
-    out[(size_t)y * W + x] = (uint8_t)cnt;
+    __syncthreads();
+    const int px = threadIdx.x & (kWinTX - 1), x = x0 + px;
+    if (x >= W) return;
+#pragma unroll
+    for (int i = 0; i < kWinTY; i += kWinT / kWinTX) {
+        const int py = i + threadIdx.x / kWinTX, y = y0 + py;
+        if (y >= H) return;
+        const uint8_t *w = wt + py * tw + px;  // the window's first pixel
+        typename F::Acc acc = f.begin(w[hr * tw + wr]);
+        if constexpr (WR >= 0) {
+#pragma unroll
+            for (int dy = 0; dy <= 2 * WR; dy++)
+#pragma unroll
+                for (int dx = 0; dx <= 2 * WC; dx++) f.add(acc, w[dy * tw + dx], dy * (2 * WC + 1) + dx);
+        } else {
+            for (int dy = 0, k = 0; dy <= 2 * hr; dy++)
+                for (int dx = 0; dx <= 2 * wr; dx++, k++) f.add(acc, w[dy * tw + dx], k);
+        }
+        out[(size_t)y * W + x] = f.end(acc);
+    }
 }
 
+// Rank transform (seq/RankFilter.cpp:11-35): 1 + #{q : I(q) < I(p)}, u8 wrap.
+struct RankWin {
+    using Out = uint8_t;
+    struct Acc {
+        int c, n;
+    };
+    __device__ Acc begin(int c) const { return Acc{c, 1}; }
+    __device__ void add(Acc &a, int v, int) const { a.n += (uint32_t)(v - a.c) >> 31; }
+    __device__ Out end(const Acc &a) const { return (uint8_t)a.n; }
+};
 // LoG convolution (seq/ConvolveImage.cpp:11-35): raster-order sum of rounded
 // products, |.|, min 255.
-__global__ void k_convolve(const uint8_t *__restrict__ img, float *__restrict__ out, const float *__restrict__ mask,
-                           int H, int W, int hr, int wr) {
-    const int y = blockIdx.y;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= W) return;
-    const int mw = 2 * wr + 1;
-    float acc = 0.f;
-    if (x >= wr && x < W - wr && y >= hr && y < H - hr) {
-        // the window inside the image: no wrapping (same products, same order)
-        const uint8_t *row = img + (size_t)(y - hr) * W + x;
-        for (int dy = -hr; dy <= hr; dy++, row += W) {
-            const float *mk = mask + (dy + hr) * mw + wr;
-            for (int dx = -wr; dx <= wr; dx++) acc = __fadd_rn(acc, __fmul_rn((float)row[dx], mk[dx]));
-        }
-    } else {
-        for (int dy = -hr; dy <= hr; dy++) {
-            const uint8_t *row = img + (size_t)wrap1(y + dy, H) * W;
-            const float *mk = mask + (dy + hr) * mw + wr;
-            for (int dx = -wr; dx <= wr; dx++) acc = __fadd_rn(acc, __fmul_rn((float)row[wrap1(x + dx, W)], mk[dx]));
-        }
+struct ConvWin {
+    using Out = float;
+    using Acc = float;
+    const float *mask;
+    __device__ Acc begin(int) const { return 0.f; }
+    __device__ void add(Acc &a, int v, int k) const { a = __fadd_rn(a, __fmul_rn((float)v, __ldg(mask + k))); }
+    __device__ Out end(Acc a) const {
+        a = (a > 0.f) ? a : -a;
+        return (a > 255.f) ? 255.f : a;
     }
-    acc = (acc > 0.f) ? acc : -acc;
-    out[(size_t)y * W + x] = (acc > 255.f) ? 255.f : acc;
-}
+};
+// Window mean for NCC (seq/NCCDisparity.cpp:24-35): raster-order float sum / area.  A: int
+// where the sum stays below 2^24 (the float sums are then exact), else float.  The target
+// mean of (x, d) equals this mean at column x-d (wrapped): the same pixels.
+template <typename A> struct MeanWin {
+    using Out = float;
+    using Acc = A;
+    float area;
+    __device__ Acc begin(int) const { return 0; }
+    __device__ void add(Acc &a, int v, int) const { a = a + (A)v; }
+    __device__ Out end(Acc a) const { return __fdiv_rn((float)a, area); }
+};
 
-// Window mean for NCC (seq/NCCDisparity.cpp:24-35): raster-order float sum / area.
-// The target mean of (x, d) equals this mean at column x-d (wrapped): the same
-// pixels are summed in the same order.
-__global__ void k_window_mean(const uint8_t *__restrict__ img, float *__restrict__ mean, int H, int W, int hr,
-                              int wr) {
+// windows whose border does not fit the tile (radius above kWinMax): a thread per pixel
+template <typename F>
+__global__ void k_window_any(const uint8_t *__restrict__ img, typename F::Out *__restrict__ out, F f, int H, int W,
+                             int hr, int wr) {
     const int y = blockIdx.y;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= W) return;
-    float s = 0.f;
+    typename F::Acc acc = f.begin(img[(size_t)y * W + x]);
+    int k = 0;
     for (int dy = -hr; dy <= hr; dy++) {
         const uint8_t *row = img + (size_t)wrap1(y + dy, H) * W;
-        for (int dx = -wr; dx <= wr; dx++) s = __fadd_rn(s, (float)row[wrap1(x + dx, W)]);
+        for (int dx = -wr; dx <= wr; dx++, k++) f.add(acc, row[wrap1(x + dx, W)], k);
     }
-    mean[(size_t)y * W + x] = __fdiv_rn(s, (float)((2 * hr + 1) * (2 * wr + 1)));
+    out[(size_t)y * W + x] = f.end(acc);
 }
 
 // NCC (seq/NCCDisparity.cpp:50-71): nom = sum rv*tv, den = sqrtf(sum ((rv*rv)*tv)*tv)
@@ -296,30 +334,33 @@ __global__ void k_window_mean(const uint8_t *__restrict__ img, float *__restrict
 // which are the reference's operations in its order.  A thread's 16 entries read
 // 8 reference and 8 target floats per tap: four 16-byte shared loads, the
 // target values held once (a {tv, tv} pair for a packed multiply would double
-// the shared-memory traffic, which bounds the loop).
+// the shared-memory traffic).  Bound: the FP32 pipe (5 operations a tap and entry), and the
+// staging's latency: three blocks an SM (80 registers) rather than two (124) 1334 -> 1106 us
+// for the two views of 1280x720, D = 64, 7x7; blocks whose windows do not wrap stage by one
+// offset a tap (1468 us with the wraps, a volume cleared first and costs stored four
+// bytes at a time).
 constexpr int kNccTX = 64, kNccTD = 64, kNccTaps = 49;
 static_assert(sizeof(float2) * kNccTaps * kNccTX + sizeof(float) * kNccTaps * (kNccTX + kNccTD) <= kSmemOptin,
               "NCC tile exceeds the shared-memory opt-in");
-// Reference rows hold float2 values in 16-byte chunks; chunk c is stored at
-// c ^ ((c >> 3) & 1), so the eight 16-byte reads of a quarter warp (4 pixels
-// apart) fall in distinct banks.  A quarter warp's target reads are eight
-// consecutive 16-byte chunks.
-__device__ __forceinline__ int ncc_swz(int u) { return (((u >> 1) ^ ((u >> 4) & 1)) << 1) | (u & 1); }
-
-__global__ void __launch_bounds__(256) k_ncc_tiled(const uint8_t *__restrict__ ref, const uint8_t *__restrict__ tar,
+__global__ void __launch_bounds__(256, 3) k_ncc_tiled(const uint8_t *__restrict__ ref, const uint8_t *__restrict__ tar,
                                                    const float *__restrict__ mref, const float *__restrict__ mtar,
-                                                   float *__restrict__ cost, int D, int H, int W, int hr, int wr) {
+                                                   float *__restrict__ cost, int D, int H, int W, int hr, int wr,
+                                                   int fill, int vec) {
     constexpr int NT = kNccTX + kNccTD - 1;       // target columns of a tile
     extern __shared__ __align__(16) unsigned char nsm[];
     float2 (*rq)[kNccTX] = reinterpret_cast<float2 (*)[kNccTX]>(nsm);                         // {rv, rv*rv}
     float (*tq)[NT + 1] = reinterpret_cast<float (*)[NT + 1]>(nsm + sizeof(float2) * kNccTaps * kNccTX);  // tv
     const int tid = threadIdx.x;
-    const int px0 = 4 * (tid & 15), d0 = 4 * (tid >> 4);
+    // a warp's 16 disparity groups store one pixel's 64 costs as whole lines
+    const int px0 = 4 * (tid >> 4), d0 = 4 * (tid & 15);
     const int y = blockIdx.y, x0 = blockIdx.x * kNccTX, dc0 = blockIdx.z * kNccTD;
     const int tbase = x0 - dc0 - (kNccTD - 1);    // target column of u = 0 (before wrapping)
     const int ew = 2 * wr + 1, taps = (2 * hr + 1) * ew;
-    // the tap offsets {dy, dx} of a chunk, made once per chunk
+    // the tap offsets {dy, dx} of a chunk, made once per chunk, and as one offset where no
+    // window of the block wraps
     __shared__ int2 tapoff[kNccTaps];
+    __shared__ int tapadd[kNccTaps];
+    const bool inside = y >= hr && y + hr < H && tbase >= wr && x0 + kNccTX + wr <= W;
     float2 acc[4][4];  // (nom, den) of pixel px0 + j, disparity d0 + i
 #pragma unroll
     for (int j = 0; j < 4; j++)
@@ -331,9 +372,28 @@ __global__ void __launch_bounds__(256) k_ncc_tiled(const uint8_t *__restrict__ r
         if (tid < nk) {
             const int kk = k0 + tid, ry = kk / ew;
             tapoff[tid] = make_int2(ry - hr, kk - ry * ew - wr);
+            tapadd[tid] = (ry - hr) * W + kk - ry * ew - wr;
         }
         __syncthreads();
-        {
+        if (inside) {
+            // reference and target cells as below, without the wraps
+            const size_t row = (size_t)y * W;
+            const int px = tid & (kNccTX - 1);
+            const uint8_t *rp = ref + row + x0 + px;
+            const float mr = mref[row + x0 + px];
+#pragma unroll 4
+            for (int k = tid >> 6; k < nk; k += 256 / kNccTX) {
+                const float rv = __fsub_rn((float)rp[tapadd[k]], mr);
+                rq[k][px] = make_float2(rv, __fmul_rn(rv, rv));
+            }
+            if (tid < 2 * NT) {
+                const int u = tid < NT ? tid : tid - NT;
+                const uint8_t *tp = tar + row + tbase + u;
+                const float mt = mtar[row + tbase + u];
+#pragma unroll 8
+                for (int k = tid < NT ? 0 : 1; k < nk; k += 2) tq[k][u] = __fsub_rn((float)tp[tapadd[k]], mt);
+            }
+        } else {
             // reference cells: a thread keeps one pixel (its mean loaded once) over every
             // 4th tap of the chunk
             const int px = tid & (kNccTX - 1);
@@ -342,10 +402,10 @@ __global__ void __launch_bounds__(256) k_ncc_tiled(const uint8_t *__restrict__ r
             for (int k = tid >> 6; k < nk; k += 256 / kNccTX) {
                 const int2 to = tapoff[k];
                 const float rv = __fsub_rn((float)ref[(size_t)wrap1(y + to.x, H) * W + wrap1(x + to.y, W)], mr);
-                rq[k][ncc_swz(px)] = make_float2(rv, __fmul_rn(rv, rv));
+                rq[k][px] = make_float2(rv, __fmul_rn(rv, rv));
             }
         }
-        if (tid < 2 * NT) {
+        if (!inside && tid < 2 * NT) {
             // target cells: threads 0 .. 2 NT - 1 keep one column each over every other tap
             const int u = tid < NT ? tid : tid - NT;
             // t in [-W, 2W) for real entries; columns of padding entries clamped into range
@@ -364,8 +424,8 @@ __global__ void __launch_bounds__(256) k_ncc_tiled(const uint8_t *__restrict__ r
         for (int k = 0; k < nk; k++) {
             float2 r[4];
             float tt[8];
-            const float4 ra = *reinterpret_cast<const float4 *>(&rq[k][ncc_swz(px0)]);
-            const float4 rb = *reinterpret_cast<const float4 *>(&rq[k][ncc_swz(px0 + 2)]);
+            const float4 ra = *reinterpret_cast<const float4 *>(&rq[k][px0]);
+            const float4 rb = *reinterpret_cast<const float4 *>(&rq[k][px0 + 2]);
             r[0] = make_float2(ra.x, ra.y); r[1] = make_float2(ra.z, ra.w);
             r[2] = make_float2(rb.x, rb.y); r[3] = make_float2(rb.z, rb.w);
             const float4 ta = *reinterpret_cast<const float4 *>(&tq[k][ub]);
@@ -386,15 +446,28 @@ __global__ void __launch_bounds__(256) k_ncc_tiled(const uint8_t *__restrict__ r
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int j = 0; j < 4; j++) {
+        const int x = x0 + px0 + j, d = dc0 + d0;
+        if (x >= W || d >= D) break;
+        float *o = cost + ((size_t)y * W + x) * D + d;
+        float v[4];
+        bool write[4], all = true;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int x = x0 + px0 + j, d = dc0 + d0 + i;
-            if (x < W && d < D) {
-                const float den = __fsqrt_rn(acc[j][i].y);  // seq/NCCDisparity.cpp:69
-                if (den != 0.f) cost[((size_t)y * W + x) * D + d] = __fdiv_rn(acc[j][i].x, den);
-            }
+            // a zero denominator leaves the cell unwritten (fill: writes 0)
+            const float den = __fsqrt_rn(acc[j][i].y);  // seq/NCCDisparity.cpp:69
+            v[i] = den != 0.f ? __fdiv_rn(acc[j][i].x, den) : 0.f;
+            write[i] = den != 0.f || fill;
+            all = all && write[i];
         }
+        if (vec && all) {
+            *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (d + i < D && write[i]) o[i] = v[i];
+        }
+    }
 }
 
 // LoG differences combined with census Hamming distances in one pass (the
@@ -509,21 +582,33 @@ void launch_hamming(cudaStream_t s, const uint64_t *cr, const uint64_t *ct, floa
     else if (nw == 2) cost_rows(s, CostHamming<2>{cr, ct}, cost, D, H, W, 1);
     else cost_rows(s, CostHamming<4>{cr, ct}, cost, D, H, W, 1);
 }
+template <typename F>
+static void window(cudaStream_t s, const uint8_t *img, typename F::Out *out, const F &f, int H, int W, int hr, int wr) {
+    const dim3 g((W + kWinTX - 1) / kWinTX, (H + kWinTY - 1) / kWinTY);
+    if (hr > kWinMax || wr > kWinMax)
+        k_window_any<<<row_grid(W, H, 128), 128, 0, s>>>(img, out, f, H, W, hr, wr);
+    else if (hr == 2 && wr == 2) k_window<F, 2, 2><<<g, kWinT, win_smem(2, 2), s>>>(img, out, f, H, W, hr, wr);
+    else if (hr == 3 && wr == 3) k_window<F, 3, 3><<<g, kWinT, win_smem(3, 3), s>>>(img, out, f, H, W, hr, wr);
+    else k_window<F, -1, -1><<<g, kWinT, win_smem(hr, wr), s>>>(img, out, f, H, W, hr, wr);
+}
 void launch_rank(cudaStream_t s, const uint8_t *img, uint8_t *out, int m, int H, int W) {
-    k_rank<<<row_grid(W, H, 128), 128, 0, s>>>(img, out, m, H, W);
+    window(s, img, out, RankWin{}, H, W, m, m);
 }
 void launch_convolve(cudaStream_t s, const uint8_t *img, float *out, const float *mask, int H, int W, int hr, int wr) {
-    k_convolve<<<row_grid(W, H, 128), 128, 0, s>>>(img, out, mask, H, W, hr, wr);
+    window(s, img, out, ConvWin{mask}, H, W, hr, wr);
 }
 void launch_window_mean(cudaStream_t s, const uint8_t *img, float *mean, int H, int W, int hr, int wr) {
-    k_window_mean<<<row_grid(W, H, 128), 128, 0, s>>>(img, mean, H, W, hr, wr);
+    const long area = (long)(2 * hr + 1) * (2 * wr + 1);
+    if (255 * area < (1L << 24)) window(s, img, mean, MeanWin<int>{(float)area}, H, W, hr, wr);
+    else window(s, img, mean, MeanWin<float>{(float)area}, H, W, hr, wr);
 }
 void launch_ncc(cudaStream_t s, const uint8_t *ref, const uint8_t *tar, const float *mref, const float *mtar,
-                float *cost, int D, int H, int W, int hr, int wr) {
+                float *cost, int D, int H, int W, int hr, int wr, int fill) {
     const dim3 g((W + kNccTX - 1) / kNccTX, H, (D + kNccTD - 1) / kNccTD);
     const size_t smem = sizeof(float2) * kNccTaps * kNccTX + sizeof(float) * kNccTaps * (kNccTX + kNccTD);
     cudaFuncSetAttribute(k_ncc_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_ncc_tiled<<<g, 256, smem, s>>>(ref, tar, mref, mtar, cost, D, H, W, hr, wr);
+    const int vec = D % 4 == 0 && ((uintptr_t)cost & 15) == 0 ? 1 : 0;
+    k_ncc_tiled<<<g, 256, smem, s>>>(ref, tar, mref, mtar, cost, D, H, W, hr, wr, fill, vec);
 }
 void launch_cost_log_census(cudaStream_t s, const float *lr, const float *lt, const uint64_t *cr, const uint64_t *ct,
                             int nw, float *vol, int D, int H, int W, const float *lut1, const float *lut2,

@@ -292,7 +292,7 @@ rts_status rts_calcNCCDispL2R(rts_ctx *ctx, rts_mem m, const uint8_t *ref, const
         launch_window_mean(c->stream, (const uint8_t *)dr, (float *)mr, H, W, hr, wr);
         launch_window_mean(c->stream, (const uint8_t *)dt, (float *)mt, H, W, hr, wr);
         launch_ncc(c->stream, (const uint8_t *)dr, (const uint8_t *)dt, (const float *)mr, (const float *)mt,
-                   (float *)dc, D, H, W, hr, wr);
+                   (float *)dc, D, H, W, hr, wr, 0);
         count_launch(c, 3);
     }
     RTS_TRY(check_launch(c, "ncc"));

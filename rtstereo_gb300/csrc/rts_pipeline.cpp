@@ -111,11 +111,10 @@ static rts_status one_cost(rts_ctx *c, const rts_params &p, int which, bool trun
         void *mean;
         RTS_TRY(scratch(c, SL_V_MEAN, np * 8, &mean));
         float *a = (float *)mean, *b = a + np;
-        // cells with a zero denominator stay unwritten (seq/NCCDisparity.cpp:70-71): start from 0
-        RTS_CU(c, cudaMemsetAsync(out, 0, np * D * sizeof(float), s));
         launch_window_mean(s, v.gref, a, H, W, p.ncc_hrad, p.ncc_wrad);
         launch_window_mean(s, v.gtar, b, H, W, p.ncc_hrad, p.ncc_wrad);
-        launch_ncc(s, v.gref, v.gtar, a, b, out, D, H, W, p.ncc_hrad, p.ncc_wrad);
+        // cells with a zero denominator (unwritten in seq/NCCDisparity.cpp:70-71) are 0
+        launch_ncc(s, v.gref, v.gtar, a, b, out, D, H, W, p.ncc_hrad, p.ncc_wrad, 1);
         count_launch(c, 3);
         return RTS_OK;
     }

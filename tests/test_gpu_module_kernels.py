@@ -197,3 +197,36 @@ def test_compute_weights_large_window(ctx, oracle_mod, r):
     lab = patches(r, r + 2, 20 + r)
     pw = oracle_mod.prox_weight(36.0, r)
     assert bits_equal(ctx.computeWeights(pw, lab, 7.0, r), oracle_mod.compute_weights(pw, lab, 7.0, r))
+
+
+# tiles' ends, wraps, radii as constants (2, 3) and not, borders above the tile's 64
+@pytest.mark.parametrize("H,W,r", [(1, 1, 0), (17, 65, 1), (33, 130, 2), (16, 64, 3), (40, 70, 3), (70, 90, 9), (66, 68, 65)])
+def test_window_filters(ctx, oracle_mod, H, W, r):
+    O = oracle_mod
+    rng = np.random.default_rng(H)
+    img = rng.integers(0, 256, (H, W), dtype=np.uint8)
+    assert bits_equal(ctx.calculateRankFilt(img, r), O.rank(img, r))
+    mask = rng.normal(0, 0.2, (2 * r + 1) ** 2).astype(np.float32)
+    assert bits_equal(ctx.convolveImage(img, mask, r, r), O.convolve(img, mask, r, r))
+    D = min(5, W - r)
+    if D > 0 and r < 20:  # blocks whose windows wrap and, in the widest image, blocks inside
+        other = rng.integers(0, 256, (H, W), dtype=np.uint8)
+        assert bits_equal(ctx.calcNCCDispL2R(img, other, D, r, r, fill=-7.0), O.ncc(img, other, D, r, r, fill=-7.0))
+
+
+@pytest.mark.parametrize("hr,wr", [(3, 3), (1, 5), (4, 4)])
+def test_ncc_inside_and_wrapped_blocks(ctx, oracle_mod, hr, wr):
+    rng = np.random.default_rng(hr)
+    L, R = rng.integers(0, 256, (2, 20, 330), dtype=np.uint8)
+    L[:, 100:150] = R[:, 100:150] = 7  # zero denominators
+    for D in (10, 70):
+        assert bits_equal(ctx.calcNCCDispL2R(L, R, D, hr, wr, fill=-7.0), oracle_mod.ncc(L, R, D, hr, wr, fill=-7.0))
+
+
+# tiles' ends, arms longer than the image, the longest tiled arm and one above, thresholds at their ends
+@pytest.mark.parametrize("H,W", [(1, 1), (16, 64), (17, 65), (50, 131)])
+@pytest.mark.parametrize("arm,tau", [(0, 20), (17, 20), (32, 60), (33, 60), (17, 0), (17, -3), (17, 1), (17, 255), (17, 256), (17, 1000)])
+def test_find_cross(ctx, oracle_mod, H, W, arm, tau):
+    rgb = patches(W, H, W)
+    got, want = ctx.findCross(rgb, arm, tau), oracle_mod.find_cross(rgb, arm, tau)
+    assert bits_equal(got[0], want[0]) and bits_equal(got[1], want[1])
