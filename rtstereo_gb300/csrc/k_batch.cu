@@ -1092,18 +1092,7 @@ __global__ void __launch_bounds__(256) k_fill_views(ViewTable t) {
                 break;
             }
         }
-        const uint16_t *r = raw + (size_t)y * W;
-        uint8_t *o = V.disp + (size_t)y * W;
-        for (int x0 = 0; x0 < W; x0 += 32) {
-            const int x = x0 + lane;
-            const uint16_t val = x < W ? r[x] : (uint16_t)0;
-            const unsigned fm = __ballot_sync(0xffffffffu, (val & 0x100) != 0);
-            const unsigned le = fm & (0xffffffffu >> (31 - lane));
-            const int src = le ? 31 - __clz(le) : 0;
-            const int got = __shfl_sync(0xffffffffu, val & 0xff, src);
-            if (x < W) o[V.mirror ? W - 1 - x : x] = (uint8_t)(le ? got : carry);
-            if (fm) carry = __shfl_sync(0xffffffffu, val & 0xff, 31 - __clz(fm));
-        }
+        wta_fill_row(raw + (size_t)y * W, V.disp + (size_t)y * W, W, V.mirror, carry);
     }
 }
 

@@ -90,19 +90,7 @@ __global__ void k_wta_fill(const uint16_t *__restrict__ raw, const int *__restri
             break;
         }
     }
-    const uint16_t *r = raw + (size_t)y * W;
-    uint8_t *o = out + (size_t)y * W;
-    for (int x0 = 0; x0 < W; x0 += 32) {
-        const int x = x0 + lane;
-        const uint16_t v = x < W ? r[x] : (uint16_t)0;
-        const unsigned fm = __ballot_sync(0xffffffffu, (v & 0x100) != 0);
-        const unsigned le = fm & (0xffffffffu >> (31 - lane));
-        const int src = le ? 31 - __clz(le) : 0;
-        const int got = __shfl_sync(0xffffffffu, v & 0xff, src);
-        const int val = le ? got : carry;
-        if (x < W) o[mirror ? W - 1 - x : x] = (uint8_t)val;
-        if (fm) carry = __shfl_sync(0xffffffffu, v & 0xff, 31 - __clz(fm));
-    }
+    wta_fill_row(raw + (size_t)y * W, out + (size_t)y * W, W, mirror, carry);
 }
 
 // The right view's winners from the left view's final volume (rts_diag.cuh):

@@ -43,6 +43,33 @@ __device__ __forceinline__ uint32_t wta_key(float v, int d, int argmax) {
 }
 __device__ __forceinline__ int imax(int a, int b) { return a > b ? a : b; }
 
+// One warp: the winners of a row of W pixels from its winner words (found << 8 | winner),
+// pixels without one of their own keeping the previous one's; carry: the winner before the
+// row.  Eight words a lane are in flight at a time (one at a time, each 32 pixels waited
+// for memory: 1280x720 21 us; 12 us now).
+__device__ __forceinline__ void wta_fill_row(const uint16_t *__restrict__ r, uint8_t *__restrict__ o, int W, int mirror,
+                                             int carry) {
+    constexpr int B = 8;
+    const int lane = threadIdx.x & 31;
+    for (int x0 = 0; x0 < W; x0 += 32 * B) {
+        uint32_t v[B];
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            const int x = x0 + 32 * k + lane;
+            v[k] = x < W ? r[x] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < B; k++) {
+            const int x = x0 + 32 * k + lane;
+            const unsigned fm = __ballot_sync(0xffffffffu, (v[k] & 0x100) != 0);
+            const unsigned le = fm & (0xffffffffu >> (31 - lane));
+            const int got = __shfl_sync(0xffffffffu, v[k] & 0xff, le ? 31 - __clz(le) : 0);
+            if (x < W) o[mirror ? W - 1 - x : x] = (uint8_t)(le ? got : carry);
+            if (fm) carry = __shfl_sync(0xffffffffu, v[k] & 0xff, 31 - __clz(fm));
+        }
+    }
+}
+
 // Packed cross arms of one pixel: left | right<<8 | top<<16 | bottom<<24.
 __device__ __forceinline__ int arm_l(uint32_t a) { return (int)(a & 0xff); }
 __device__ __forceinline__ int arm_r(uint32_t a) { return (int)((a >> 8) & 0xff); }
