@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kRefT) k_disp_refine(const uint16_t *__restric
         const uint16_t *row = runs + (size_t)yy * W;
         for (int xx = imax(x - h[0], 0); xx <= xr;) {
             const int w = row[xx], n = imin(w >> 8, xr - xx + 1), v = w & 0xff;
-            if (v < D) hist[v * kRefT] += n;
+            if (v < D) atomicAdd(hist + v * kRefT, n);
             xx += n;
         }
     }

@@ -5,8 +5,7 @@
 // fused pipeline is bit-identical to the composed module kernels and to the
 // reference; fusion only removes HBM round trips and adds on-chip reuse.
 //
-//   k_prep_records  per pixel one 16-byte record: 64-bit census code, packed
-//                   RGB, packed cross arms (l | r<<8 | t<<16 | b<<24)
+//   k_prep_records  per pixel one 16-byte record: 64-bit census code, packed RGB
 //   k_cost_volume   AD / census / AD+census(CombineCost) cost volume from records
 //   (the cross-based stages work over view tables and live in k_batch.cu)
 //   k_aw_wta        adaptive-weight aggregation (seq/AdaptiveWeightAggregation.cpp:73-111)
@@ -22,53 +21,62 @@
 namespace rts {
 
 // ---------------------------------------------------------------------------
-__global__ void k_prep_records(const uint8_t *__restrict__ gray, const uint8_t *__restrict__ rgb,
-                               uint4 *__restrict__ rec, uint32_t *__restrict__ arms_out, int H, int W, int hr, int wr,
-                               int L, int tau, int want_code, int want_arms) {
-    const int y = blockIdx.y;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= W) return;
-    const long p = (long)y * W + x;
-    uint64_t code = 0;
+// Block per 64 x 16 pixels, the gray census window around them (wrapped,
+// seq/CensusTransform.cpp:20-26) staged in shared memory, a thread on four pixels.  WIN: the
+// 9x7 window, its 63 comparisons unrolled (a subtraction and a funnel shift of its sign
+// bit each; the order of a code's bits is the same in all records of a launch and only
+// distances of codes are used).  Bound: instruction issue.  1920x1080: 120 us an image
+// with the window as loops over the image itself.
+constexpr int kRecTW = 64, kRecTH = 16, kRecT = 256;
+template <bool WIN>
+__global__ void __launch_bounds__(kRecT) k_prep_records(const uint8_t *__restrict__ gray,
+                                                        const uint8_t *__restrict__ rgb, uint4 *__restrict__ rec, int H,
+                                                        int W, int hr_, int wr_, int want_code) {
+    extern __shared__ uint8_t gt[];  // [16 + 2 hr][64 + 2 wr]
+    const int hr = WIN ? 4 : hr_, wr = WIN ? 3 : wr_;
+    const int gw = kRecTW + 2 * wr, gh = kRecTH + 2 * hr, x0 = blockIdx.x * kRecTW, y0 = blockIdx.y * kRecTH;
     if (want_code) {
-        // seq/CensusTransform.cpp:11-37, bit (dy+hr)*(2wr+1)+(dx+wr), strict centre > neighbour
-        const uint8_t c = gray[p];
-        int k = 0;
-        if (x >= wr && x < W - wr && y >= hr && y < H - hr) {
-            // the window inside the image: no wrapping
-            const uint8_t *row = gray + p - (size_t)hr * W - wr;
-            for (int dy = -hr; dy <= hr; dy++, row += W)
-                for (int dx = 0; dx <= 2 * wr; dx++, k++) code |= (uint64_t)(c > row[dx]) << k;
-        } else {
-            for (int dy = -hr; dy <= hr; dy++) {
-                const uint8_t *row = gray + (size_t)wrap1(y + dy, H) * W;
-                for (int dx = -wr; dx <= wr; dx++, k++) code |= (uint64_t)(c > row[wrap1(x + dx, W)]) << k;
-            }
+        const int lane = threadIdx.x & 31;
+        for (int r = threadIdx.x >> 5; r < gh; r += kRecT / 32) {
+            // past the last pixel's window: clamped into range, never used
+            const uint8_t *row = gray + (size_t)wrap1(imin(y0 - hr + r, H - 1 + hr), H) * W;
+            for (int c = lane; c < gw; c += 32) gt[r * gw + c] = row[wrap1(imin(x0 - wr + c, W - 1 + wr), W)];
         }
+        __syncthreads();
     }
-    const uint8_t *px = rgb + 3 * p;
-    const uint32_t packed = (uint32_t)px[0] | ((uint32_t)px[1] << 8) | ((uint32_t)px[2] << 16);
-    uint32_t arms = 0;
-    if (want_arms) {
-        // seq/CrossBasedAggregation.cpp:12-100, same stepping rule as k_find_cross
-        const int c0 = px[0], c1 = px[1], c2 = px[2];
-        int len[4];
-        const long step[4] = {-1, 1, -(long)W, (long)W};
-        const int room[4] = {x, W - 1 - x, y, H - 1 - y};
+    const int px = threadIdx.x & (kRecTW - 1), x = x0 + px;
+    if (x >= W) return;
+    for (int py = threadIdx.x / kRecTW; py < kRecTH; py += kRecT / kRecTW) {
+        const int y = y0 + py;
+        if (y >= H) return;
+        uint32_t lo = 0, hi = 0;
+        if (want_code) {
+            // seq/CensusTransform.cpp:11-37: strict centre > neighbour
+            const uint8_t *g0 = gt + py * gw + px;
+            const uint32_t c = g0[hr * gw + wr];
+            if constexpr (WIN) {
 #pragma unroll
-        for (int a = 0; a < 4; a++) {
-            int n = 0, delta = 0;
-            while (delta < tau && n < L && n < room[a]) {
-                n++;
-                const uint8_t *q = rgb + 3 * (p + step[a] * n);
-                delta = imax(imax(abs(c0 - (int)q[0]), abs(c1 - (int)q[1])), abs(c2 - (int)q[2]));
+                for (int r = 0; r < 9; r++)
+#pragma unroll
+                    for (int dx = 0; dx < 7; dx++) {
+                        const uint32_t below = (uint32_t)g0[r * gw + dx] - c;  // sign bit: c > neighbour
+                        if (7 * r + dx < 32) lo = __funnelshift_l(below, lo, 1);
+                        else hi = __funnelshift_l(below, hi, 1);
+                    }
+            } else {
+                int k = 0;
+                for (int r = 0; r <= 2 * hr; r++)
+                    for (int dx = 0; dx <= 2 * wr; dx++, k++) {
+                        const uint32_t bit = c > (uint32_t)g0[r * gw + dx] ? 1u : 0u;
+                        if (k < 32) lo |= bit << k;
+                        else hi |= bit << (k - 32);
+                    }
             }
-            len[a] = n;
         }
-        arms = (uint32_t)len[0] | ((uint32_t)len[1] << 8) | ((uint32_t)len[2] << 16) | ((uint32_t)len[3] << 24);
+        const size_t p = (size_t)y * W + x;
+        const uint8_t *q = rgb + 3 * p;
+        rec[p] = make_uint4(lo, hi, (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16), 0u);
     }
-    rec[p] = make_uint4((uint32_t)code, (uint32_t)(code >> 32), packed, arms);
-    if (arms_out) arms_out[p] = arms;
 }
 
 // ---------------------------------------------------------------------------
@@ -84,47 +92,88 @@ __global__ void k_cost_volume(const uint4 *__restrict__ rr, const uint4 *__restr
     vol[((size_t)y * W + x) * pitch + d] = to_store<T>(pair_cost(a, b, cfg));
 }
 
-// AD (optionally truncated) + census combined through the two host tables, the
-// integer path: warp per pixel, lane = disparity, so the reference record is a
-// broadcast and the volume row is contiguous.  Block per (row, 64 pixels): the
-// target records the block meets, columns x0 - D + 1 .. x0 + 63 (wrapped as in
-// seq/PixelBasedCost.cpp:19-20), and the two tables are staged in shared memory
-// once, so an entry reads its target record (consecutive lanes, consecutive
-// records) and its two table values from shared memory.
-constexpr int kAdcPx = 8;
-constexpr int kAdcTX = 8 * kAdcPx;          // pixels of a block
+// AD (optionally truncated) + census combined through the two host tables, the integer
+// path.  Resident blocks stride over (row, 64 pixels); an item's reference records and the
+// target records it meets, columns x0 - Dp .. x0 + 63 (wrapped as in
+// seq/PixelBasedCost.cpp:19-20; Dp = D up to a multiple of 4), are staged in shared memory,
+// target u in array u mod 4, so that a thread's 4 pixels x 4 disparities read 7 target
+// records for 16 entries, lanes (disparity groups) on consecutive ones.  The tables are
+// staged 2^lc1 and 2^lc2 times over, copy = lane: a warp's 32 lookups of one table hit
+// nearly 32 different banks (a single copy costs some 3.5 wavefronts a lookup).
+// Bound: the volume's write and the population counts.
+constexpr int kAdcTX = 64;
 constexpr int kAdcL1 = 768, kAdcL2 = 68;    // table entries staged: AD <= 765, census <= 64
+constexpr int kAdcNT = (kAdcTX + 256) / 4;  // target records of one residue
+static_assert(kAdcL1 * 16 * 4 + kAdcL2 * 32 * 4 + (4 * kAdcNT + kAdcTX) * 16 <= 75 * 1024, "three blocks an SM");
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_cost_volume_adc(const uint4 *__restrict__ rr, const uint4 *__restrict__ rt,
-                                                        T *__restrict__ vol, int H, int W, int D, int pitch, int itrunc,
-                                                        const float *__restrict__ lut1, const float *__restrict__ lut2) {
-    __shared__ uint4 trec[kAdcTX + 255];  // D <= 256
-    __shared__ float t1[kAdcL1], t2[kAdcL2];
-    const int y = blockIdx.y, lane = threadIdx.x & 31, tid = threadIdx.x;
-    const int x0 = blockIdx.x * kAdcTX, base = x0 - D + 1;
-    const uint4 *trow = rt + (size_t)y * W;
-    for (int i = tid; i < kAdcTX + D - 1; i += 256) {
-        int xt = base + i;
-        if (xt < 0) xt += W;  // seq/PixelBasedCost.cpp:19-20 (D <= W)
-        trec[i] = trow[imin(xt, W - 1)];  // columns past the row end are never read
-    }
-    for (int i = tid; i < kAdcL1; i += 256) t1[i] = lut1[i];
-    if (tid < kAdcL2) t2[tid] = lut2[tid];
-    __syncthreads();
-    // a warp takes kAdcPx consecutive pixels of the row
-    const int xw = x0 + (tid >> 5) * kAdcPx;
-#pragma unroll 2
-    for (int i = 0; i < kAdcPx; i++) {
-        const int x = xw + i;
-        if (x >= W) return;
-        const uint4 a = rr[(size_t)y * W + x];
-        T *out = vol + ((size_t)y * W + x) * pitch;
-        const uint4 *tb = trec + (x - base);  // target of disparity d: tb[-d]
-        for (int d = lane; d < D; d += 32) {
-            const uint4 b = tb[-d];
-            const int sad = imin((int)__vsadu4(a.z, b.z), itrunc);    // seq/PixelBasedCost.cpp:86-91 / :106-112
-            const int ham = __popc(a.x ^ b.x) + __popc(a.y ^ b.y);   // seq/CensusTransform.cpp:52-60
-            out[d] = to_store<T>(__fadd_rn(t1[sad], t2[ham]));       // seq/CombineCost.cpp:23
+__global__ void __launch_bounds__(256, 3) k_cost_volume_adc(const uint4 *__restrict__ rr, const uint4 *__restrict__ rt,
+                                                           T *__restrict__ vol, int H, int W, int D, int pitch,
+                                                           int itrunc, const float *__restrict__ lut1,
+                                                           const float *__restrict__ lut2, int lc1, int lc2) {
+    extern __shared__ __align__(16) unsigned char asm2_[];
+    uint4 *trec = reinterpret_cast<uint4 *>(asm2_), *rrec = trec + 4 * kAdcNT;  // [u mod 4][u / 4]; [64]
+    float *t1 = reinterpret_cast<float *>(rrec + kAdcTX), *t2 = t1 + (kAdcL1 << lc1);
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int i = tid; i < kAdcL1 << lc1; i += 256) t1[i] = lut1[i >> lc1];
+    for (int i = tid; i < kAdcL2 << lc2; i += 256) t2[i] = lut2[i >> lc2];
+    const float *l1 = t1 + (lane & ((1 << lc1) - 1)), *l2 = t2 + (lane & ((1 << lc2) - 1));
+    const int ndg = (D + 3) >> 2, Dp = 4 * ndg, xb = (W + kAdcTX - 1) / kAdcTX;
+    const bool vec = (pitch & 3) == 0;
+    for (int item = blockIdx.x; item < H * xb; item += gridDim.x) {
+        const int y = item / xb, x0 = (item - y * xb) * kAdcTX;
+        const size_t row = (size_t)y * W;
+        __syncthreads();  // the previous item's records are consumed (and the tables are in)
+        for (int i = tid; i < kAdcTX + Dp; i += 256) {
+            int xt = x0 - Dp + i;
+            if (xt < 0) xt += W;  // seq/PixelBasedCost.cpp:19-20 (D <= W)
+            trec[(i & 3) * kAdcNT + (i >> 2)] = rt[row + imax(imin(xt, W - 1), 0)];  // clamped: of no entry
+        }
+        if (tid < kAdcTX) rrec[tid] = rr[row + imin(x0 + tid, W - 1)];
+        __syncthreads();
+        const int nx = imin(kAdcTX, W - x0);
+        // pixel group xg = q / ndg, disparity group dg = q mod ndg; 256 groups at a time
+        const int sx = 256 / ndg, sd = 256 - sx * ndg;
+        for (int xg = tid / ndg, dg = tid - xg * ndg; 4 * xg < nx;) {
+            const uint4 *tb = trec + (xg - dg + ndg);  // u = 4 (xg - dg) + Dp + j - i
+            uint4 b[7];                                // j - i + 3
+#pragma unroll
+            for (int k = 0; k < 7; k++) b[k] = k < 3 ? tb[(k + 1) * kAdcNT - 1] : tb[(k - 3) * kAdcNT];
+            T *out = vol + (row + x0 + 4 * xg) * pitch + 4 * dg;
+#pragma unroll
+            for (int j = 0; j < 4; j++, out += pitch) {
+                const uint4 a = rrec[4 * xg + j];
+                float v[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const uint4 &t = b[j - i + 3];
+                    const int sad = imin((int)__vsadu4(a.z, t.z), itrunc);   // seq/PixelBasedCost.cpp:86-91 / :106-112
+                    const int ham = __popc(a.x ^ t.x) + __popc(a.y ^ t.y);  // seq/CensusTransform.cpp:52-60
+                    v[i] = __fadd_rn(l1[sad << lc1], l2[ham << lc2]);       // seq/CombineCost.cpp:23
+                }
+                if (4 * xg + j < nx) {
+                    if (vec) {
+                        // (a padded pitch takes the cells past D too)
+                        if constexpr (sizeof(T) == 4) {
+                            *reinterpret_cast<float4 *>(out) = make_float4(v[0], v[1], v[2], v[3]);
+                        } else {
+                            const __half2 h0 = __floats2half2_rn(v[0], v[1]), h1 = __floats2half2_rn(v[2], v[3]);
+                            *reinterpret_cast<uint2 *>(out) = make_uint2(*reinterpret_cast<const uint32_t *>(&h0),
+                                                                         *reinterpret_cast<const uint32_t *>(&h1));
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            if (4 * dg + i < D) out[i] = to_store<T>(v[i]);
+                    }
+                }
+            }
+            xg += sx;
+            dg += sd;
+            if (dg >= ndg) {
+                dg -= ndg;
+                xg++;
+            }
         }
     }
 }
@@ -816,12 +865,13 @@ bool fused_supported(const rts_params &p, int H, int W) {
 }
 
 rts_status prep_records(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *gray, const uint8_t *rgb,
-                        uint4 *rec, uint32_t *arms_out) {
-    const bool code = p.cost1 == RTS_COST_CENSUS || p.cost2 == RTS_COST_CENSUS;
-    const bool arms = p.aggr == RTS_AGGR_CROSS;
-    k_prep_records<<<dim3((W + 127) / 128, H), 128, 0, c->stream>>>(gray, rgb, rec, arms_out, H, W, p.census_hrad,
-                                                                   p.census_wrad, p.cross_arm, p.cross_tau,
-                                                                   code && fast_costs(p), arms);
+                        uint4 *rec) {
+    const int code = (p.cost1 == RTS_COST_CENSUS || p.cost2 == RTS_COST_CENSUS) && fast_costs(p) ? 1 : 0;
+    const int hr = code ? p.census_hrad : 0, wr = code ? p.census_wrad : 0;
+    const dim3 g((W + kRecTW - 1) / kRecTW, (H + kRecTH - 1) / kRecTH);
+    const size_t smem = (size_t)(kRecTH + 2 * hr) * (kRecTW + 2 * wr);  // a window of at most 64 bits
+    if (code && hr == 4 && wr == 3) k_prep_records<true><<<g, kRecT, smem, c->stream>>>(gray, rgb, rec, H, W, hr, wr, code);
+    else k_prep_records<false><<<g, kRecT, smem, c->stream>>>(gray, rgb, rec, H, W, hr, wr, code);
     count_launch(c);
     return check_launch(c, "prep_records");
 }
@@ -850,9 +900,19 @@ rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const
     RTS_TRY(cost_cfg(c, p, &cfg));
     const int D = p.disp_range;
     if (cfg.int_path && cfg.k1 == RTS_COST_AD && cfg.k2 == RTS_COST_CENSUS) {
-        const dim3 g((unsigned)((W + kAdcTX - 1) / kAdcTX), H);
-        if (half) k_cost_volume_adc<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, pitch, cfg.itrunc, cfg.lut1, cfg.lut2);
-        else k_cost_volume_adc<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, pitch, cfg.itrunc, cfg.lut1, cfg.lut2);
+        // copies of the tables where every resident block makes several items (staging 16 and 32
+        // copies takes about one item's time)
+        const long items = (long)((W + kAdcTX - 1) / kAdcTX) * H, res = 3L * sm_count();
+        const int lc1 = items >= 4 * res ? 4 : 0, lc2 = items >= 4 * res ? 5 : 0;
+        const size_t smem = ((size_t)(kAdcL1 << lc1) + (size_t)(kAdcL2 << lc2)) * 4 + (4 * kAdcNT + kAdcTX) * sizeof(uint4);
+        auto go = [&](auto kern, auto *v) -> rts_status {
+            RTS_TRY(set_smem(c, kern, smem, "cost_volume"));
+            kern<<<(unsigned)std::min(items, lc1 ? res : items), 256, smem, c->stream>>>(
+                rr, rt, v, H, W, D, pitch, cfg.itrunc, cfg.lut1, cfg.lut2, lc1, lc2);
+            return RTS_OK;
+        };
+        if (half) RTS_TRY(go(k_cost_volume_adc<__half>, (__half *)vol));
+        else RTS_TRY(go(k_cost_volume_adc<float>, (float *)vol));
         count_launch(c);
         return check_launch(c, "cost_volume");
     }

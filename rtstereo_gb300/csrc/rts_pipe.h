@@ -11,9 +11,9 @@ bool fast_costs(const rts_params &p);
 // adaptive-weight aggregation (radius <= 16) has a fused per-view path
 bool fused_supported(const rts_params &p, int H, int W);
 
-// 16-byte per-pixel records: census code, packed RGB, packed cross arms
+// 16-byte per-pixel records: census code, packed RGB
 rts_status prep_records(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *gray, const uint8_t *rgb,
-                        uint4 *rec, uint32_t *arms_out);
+                        uint4 *rec);
 // cost volume [H][W][D] (float, or __half when half != 0), pitch values a pixel, from records
 rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const uint4 *rr, const uint4 *rt,
                             void *vol, int half, int pitch);

@@ -176,8 +176,8 @@ static rts_status view_composed(rts_ctx *c, const rts_params &p, int H, int W, c
         void *recv;
         RTS_TRY(scratch(c, SL_V_REC, np * 32, &recv));
         uint4 *rr = (uint4 *)recv, *rt = rr + np;
-        RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr, nullptr));
-        RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt, nullptr));
+        RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr));
+        RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt));
         RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1, 0, D));
     } else {
         StageScope sc(c, "cost");
@@ -292,8 +292,8 @@ static rts_status view_fused(rts_ctx *c, const rts_params &p, int H, int W, cons
     RTS_CU(c, cudaMemsetAsync(rl, 0xff, (size_t)H * 4, s));
     {
         StageScope sc(c, "prep");
-        RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr, nullptr));
-        RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt, nullptr));
+        RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr));
+        RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt));
     }
     const bool fast = fast_costs(p);
     const void *vol = nullptr;

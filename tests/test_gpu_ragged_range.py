@@ -103,3 +103,19 @@ def test_adaptive_weights(ctx, oracle_mod, D, rad):
          for d in (D, wide)]
     assert bits_equal(f[0][3], np.ascontiguousarray(f[1][3][:, :, :D]))
     assert bits_equal(f[0][0], oracle_mod.wta(f[0][3]))
+
+
+# the AD + census volume under box and adaptive weights: disparity groups of four and remainders, pixels
+# past a block's 64, single tables (small pairs) and copied ones (many items)
+@pytest.mark.parametrize("W,H,D", [(9, 9, 3), (70, 33, 37), (200, 20, 64), (257, 12, 256), (129, 1500, 6)])
+@pytest.mark.parametrize("colour", [False, True])
+def test_ad_census_volume(ctx, oracle_mod, W, H, D, colour):
+    import rtstereo_gb300 as R
+    (L, Rr), (Lc, Rc) = pair(W, W, H, D, colour)
+    for prec in (0, 1):
+        p = R.params(disp_range=D, aggr=1, box_rad=2, precision=prec)
+        got = ctx.pipeline(p, L, Rr, Lc, Rc)
+        o = oracle_mod.pipeline(oracle_mod.params(D=D, aggr=1, box_rad=2), L, Rr, Lc, Rc)
+        assert bits_equal(got[0], o[0])
+        if prec == 0:
+            assert bits_equal(got[1], o[1]) and bits_equal(got[2], o[2])
