@@ -74,21 +74,24 @@ __global__ void __launch_bounds__(kRecT) k_prep_records(const uint8_t *__restric
             }
         }
         const size_t p = (size_t)y * W + x;
+        // without a colour image the gray in all three channels (seq/Main.cpp:87-90)
         const uint8_t *q = rgb + 3 * p;
-        rec[p] = make_uint4(lo, hi, (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16), 0u);
+        rec[p] = make_uint4(lo, hi,
+                            rgb ? (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16) : gray[p] * 0x010101u,
+                            0u);
     }
 }
 
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void k_cost_volume(const uint4 *__restrict__ rr, const uint4 *__restrict__ rt, T *__restrict__ vol, int H,
-                              int W, int D, int pitch, CostCfg cfg) {
+                              int W, int D, int pitch, int mirror, CostCfg cfg) {
     const int y = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= W * D) return;
     const int x = i / D, d = i - x * D;
     const int xt = tar_col(x, d, W, 1);
-    const uint4 a = rr[(size_t)y * W + x], b = rt[(size_t)y * W + xt];
+    const uint4 a = rr[(size_t)y * W + (mirror ? W - 1 - x : x)], b = rt[(size_t)y * W + (mirror ? W - 1 - xt : xt)];
     vol[((size_t)y * W + x) * pitch + d] = to_store<T>(pair_cost(a, b, cfg));
 }
 
@@ -109,7 +112,7 @@ static_assert(kAdcL1 * 16 * 4 + kAdcL2 * 32 * 4 + (4 * kAdcNT + kAdcTX) * 16 <= 
 template <typename T>
 __global__ void __launch_bounds__(256, 3) k_cost_volume_adc(const uint4 *__restrict__ rr, const uint4 *__restrict__ rt,
                                                            T *__restrict__ vol, int H, int W, int D, int pitch,
-                                                           int itrunc, const float *__restrict__ lut1,
+                                                           int mirror, int itrunc, const float *__restrict__ lut1,
                                                            const float *__restrict__ lut2, int lc1, int lc2) {
     extern __shared__ __align__(16) unsigned char asm2_[];
     uint4 *trec = reinterpret_cast<uint4 *>(asm2_), *rrec = trec + 4 * kAdcNT;  // [u mod 4][u / 4]; [64]
@@ -127,9 +130,13 @@ __global__ void __launch_bounds__(256, 3) k_cost_volume_adc(const uint4 *__restr
         for (int i = tid; i < kAdcTX + Dp; i += 256) {
             int xt = x0 - Dp + i;
             if (xt < 0) xt += W;  // seq/PixelBasedCost.cpp:19-20 (D <= W)
-            trec[(i & 3) * kAdcNT + (i >> 2)] = rt[row + imax(imin(xt, W - 1), 0)];  // clamped: of no entry
+            xt = imax(imin(xt, W - 1), 0);  // clamped: of no entry
+            trec[(i & 3) * kAdcNT + (i >> 2)] = rt[row + (mirror ? W - 1 - xt : xt)];
         }
-        if (tid < kAdcTX) rrec[tid] = rr[row + imin(x0 + tid, W - 1)];
+        if (tid < kAdcTX) {
+            const int x = imin(x0 + tid, W - 1);
+            rrec[tid] = rr[row + (mirror ? W - 1 - x : x)];
+        }
         __syncthreads();
         const int nx = imin(kAdcTX, W - x0);
         // pixel group xg = q / ndg, disparity group dg = q mod ndg; 256 groups at a time
@@ -199,10 +206,12 @@ constexpr int kAwCPitch = kAwDC + 4;
 constexpr int kAwHPitch = kAwDC + 8;  // f16 cost rows: 144 bytes, a multiple of 16
 constexpr uint32_t kLabOut = 0xff000000u;  // marks a column outside the image
 
-__global__ void k_pack_lab(const uint8_t *__restrict__ lab, uint32_t *__restrict__ out, long n) {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] = (uint32_t)lab[3 * i] | ((uint32_t)lab[3 * i + 1] << 8) | ((uint32_t)lab[3 * i + 2] << 16);
+__global__ void k_pack_lab(const uint8_t *__restrict__ lab, uint32_t *__restrict__ out, int W, int mirror) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= W) return;
+    const size_t row = (size_t)blockIdx.y * W;
+    const uint8_t *q = lab + 3 * (row + (mirror ? W - 1 - x : x));
+    out[row + x] = (uint32_t)q[0] | ((uint32_t)q[1] << 8) | ((uint32_t)q[2] << 16);
 }
 
 template <typename CT, bool EXACT>
@@ -895,7 +904,7 @@ static rts_status cost_cfg(rts_ctx *c, const rts_params &p, CostCfg *cfg) {
 }
 
 rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const uint4 *rr, const uint4 *rt,
-                            void *vol, int half, int pitch) {
+                            void *vol, int half, int pitch, int mirror) {
     CostCfg cfg;
     RTS_TRY(cost_cfg(c, p, &cfg));
     const int D = p.disp_range;
@@ -908,7 +917,7 @@ rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const
         auto go = [&](auto kern, auto *v) -> rts_status {
             RTS_TRY(set_smem(c, kern, smem, "cost_volume"));
             kern<<<(unsigned)std::min(items, lc1 ? res : items), 256, smem, c->stream>>>(
-                rr, rt, v, H, W, D, pitch, cfg.itrunc, cfg.lut1, cfg.lut2, lc1, lc2);
+                rr, rt, v, H, W, D, pitch, mirror, cfg.itrunc, cfg.lut1, cfg.lut2, lc1, lc2);
             return RTS_OK;
         };
         if (half) RTS_TRY(go(k_cost_volume_adc<__half>, (__half *)vol));
@@ -917,8 +926,8 @@ rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const
         return check_launch(c, "cost_volume");
     }
     const dim3 g((unsigned)(((long)W * D + 255) / 256), H);
-    if (half) k_cost_volume<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, pitch, cfg);
-    else k_cost_volume<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, pitch, cfg);
+    if (half) k_cost_volume<__half><<<g, 256, 0, c->stream>>>(rr, rt, (__half *)vol, H, W, D, pitch, mirror, cfg);
+    else k_cost_volume<float><<<g, 256, 0, c->stream>>>(rr, rt, (float *)vol, H, W, D, pitch, mirror, cfg);
     count_launch(c);
     return check_launch(c, "cost_volume");
 }
@@ -949,7 +958,7 @@ rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W) {
 }
 
 rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, int pitch, const uint8_t *labr,
-                    const uint8_t *labt, uint16_t *raw, int *rl, float *cost_out) {
+                    const uint8_t *labt, int mirror, uint16_t *raw, int *rl, float *cost_out) {
     const float *pw, *g;
     RTS_TRY(prox_weights(c, p.aw_gamma_p, p.aw_rad, &pw));
     RTS_TRY(lab_weight_lut(c, p.aw_gamma_s, &g));
@@ -957,8 +966,8 @@ rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *v
     void *lp;
     RTS_TRY(scratch(c, SL_V_MEAN, (size_t)np * 8, &lp));
     uint32_t *plr = (uint32_t *)lp, *plt = plr + np;
-    k_pack_lab<<<(unsigned)((np + 255) / 256), 256, 0, c->stream>>>(labr, plr, np);
-    k_pack_lab<<<(unsigned)((np + 255) / 256), 256, 0, c->stream>>>(labt, plt, np);
+    k_pack_lab<<<dim3((W + 255) / 256, H), 256, 0, c->stream>>>(labr, plr, W, mirror);
+    k_pack_lab<<<dim3((W + 255) / 256, H), 256, 0, c->stream>>>(labt, plt, W, mirror);
     count_launch(c, 2);
     const int r = p.aw_rad, e = 2 * r + 1;
     const size_t smem = sizeof(float) * ((size_t)(kAwTX + 2 * r + 4) * kAwCPitch + (size_t)e * kAwTX +

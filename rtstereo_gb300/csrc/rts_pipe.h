@@ -11,12 +11,15 @@ bool fast_costs(const rts_params &p);
 // adaptive-weight aggregation (radius <= 16) has a fused per-view path
 bool fused_supported(const rts_params &p, int H, int W);
 
-// 16-byte per-pixel records: census code, packed RGB
+// 16-byte per-pixel records: census code, packed RGB (rgb null: the gray in all channels)
 rts_status prep_records(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *gray, const uint8_t *rgb,
                         uint4 *rec);
-// cost volume [H][W][D] (float, or __half when half != 0), pitch values a pixel, from records
+// cost volume [H][W][D] (float, or __half when half != 0), pitch values a pixel, from
+// records; mirror: of the mirrored images (a right view: reference and target are the right
+// and the left image's records; their codes are then the mirrored images' up to one fixed
+// order of the bits, which no distance depends on)
 rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const uint4 *rr, const uint4 *rt,
-                            void *vol, int half, int pitch);
+                            void *vol, int half, int pitch, int mirror);
 // allocates what cost_volume_fast and aw_fused will ask for (tables, packed Lab images)
 rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W);
 // the cross-based pipeline runs over view tables (rts_views.h) when this holds
@@ -25,8 +28,8 @@ bool cross_fused_supported(const rts_params &p);
 // form, whichever form is asked for: the composed path has no other)
 bool cross_ragged_supported(const rts_params &p);
 // adaptive-weight aggregation + arg-min over a float (half == 0) or __half volume of
-// `pitch` values a pixel
+// `pitch` values a pixel; mirror: of the mirrored Lab images
 rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, int pitch, const uint8_t *labr,
-                    const uint8_t *labt, uint16_t *raw, int *row_last, float *cost_out);
+                    const uint8_t *labt, int mirror, uint16_t *raw, int *row_last, float *cost_out);
 
 }  // namespace rts

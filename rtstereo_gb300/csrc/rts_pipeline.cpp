@@ -58,10 +58,20 @@ rts_status validate_params(rts_ctx *c, const rts_params &p, int H, int W) {
 }
 
 // view-ordered inputs (for the right view: mirrored right image as reference,
-// mirrored left image as target)
+// mirrored left image as target; on the record path the images themselves, right and
+// left, which the kernels read mirrored)
 struct ViewIn {
     const uint8_t *gref, *gtar, *cref, *ctar, *lref, *ltar;
+    int rec = 0;  // 1: a right view that takes the left view's records, and its Lab images, mirrored
 };
+
+// The pair's costs come from per-pixel records alone, made by the left view for both: a box
+// whose means and arg-min are one pass, or fused adaptive weights.
+static bool record_path(const rts_params &p, int H, int W, bool cost_out) {
+    if (!fast_costs(p)) return false;
+    if (p.aggr == RTS_AGGR_BOX) return !cost_out && box_best_supported(p.box_rad);
+    return p.aggr == RTS_AGGR_AW && fused_supported(p, H, W);
+}
 
 // one matching cost into `out` (seq/Main.cpp:180-231)
 static rts_status one_cost(rts_ctx *c, const rts_params &p, int which, bool trunc_ad, int H, int W, const ViewIn &v,
@@ -176,9 +186,11 @@ static rts_status view_composed(rts_ctx *c, const rts_params &p, int H, int W, c
         void *recv;
         RTS_TRY(scratch(c, SL_V_REC, np * 32, &recv));
         uint4 *rr = (uint4 *)recv, *rt = rr + np;
-        RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr));
-        RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt));
-        RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1, 0, D));
+        if (!v.rec) {
+            RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr));
+            RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt));
+        }
+        RTS_TRY(cost_volume_fast(c, p, H, W, v.rec ? rt : rr, v.rec ? rr : rt, c1, 0, D, v.rec));
     } else {
         StageScope sc(c, "cost");
         RTS_TRY(one_cost(c, p, p.cost1, p.aggr == RTS_AGGR_CROSS, H, W, v, c1, SL_V_AUX));
@@ -290,12 +302,13 @@ static rts_status view_fused(rts_ctx *c, const rts_params &p, int H, int W, cons
     RTS_TRY(scratch(c, SL_V_RAW, np * 2, &raw));
     RTS_TRY(scratch(c, SL_V_ROWLAST, (size_t)H * 4, &rl));
     RTS_CU(c, cudaMemsetAsync(rl, 0xff, (size_t)H * 4, s));
-    {
+    const bool fast = fast_costs(p);
+    const int rev = v.rec;
+    if (fast && !rev) {
         StageScope sc(c, "prep");
         RTS_TRY(prep_records(c, p, H, W, v.gref, v.cref, rr));
         RTS_TRY(prep_records(c, p, H, W, v.gtar, v.ctar, rt));
     }
-    const bool fast = fast_costs(p);
     const void *vol = nullptr;
     int vol_half = 0, pitch = D;
     {
@@ -316,14 +329,14 @@ static rts_status view_fused(rts_ctx *c, const rts_params &p, int H, int W, cons
                     pitch = wide;
                 }
             }
-            RTS_TRY(cost_volume_fast(c, p, H, W, rr, rt, c1v, vol_half, pitch));
+            RTS_TRY(cost_volume_fast(c, p, H, W, rev ? rt : rr, rev ? rr : rt, c1v, vol_half, pitch, rev));
         } else {
             RTS_TRY(scratch(c, SL_V_COST1, ne * 4, &c1v));
             RTS_TRY(cost_volume_composed(c, p, H, W, v, (float *)c1v));
         }
         vol = c1v;
     }
-    RTS_TRY(aw_fused(c, p, H, W, vol, vol_half, pitch, v.lref, v.ltar, (uint16_t *)raw, (int *)rl, cost_out));
+    RTS_TRY(aw_fused(c, p, H, W, vol, vol_half, pitch, v.lref, v.ltar, rev, (uint16_t *)raw, (int *)rl, cost_out));
     {
         StageScope sc(c, "wta_fill");
         launch_wta_fill(s, (const uint16_t *)raw, (const int *)rl, disp, H, W, mirror);
@@ -453,8 +466,10 @@ rts_status pipeline_device(rts_ctx *c, const rts_params &p, int H, int W, const 
         if (st != RTS_ERR_OOM) return st;  // no room, or a captured stream: the module kernels below
     }
     const bool need_lab = p.aggr == RTS_AGGR_AW;
-    // the fused kernels read packed colour records even for gray-only costs
-    const bool need_rgb = true;
+    // the record path makes colour words from the gray image where there is no colour
+    const bool records = record_path(p, H, W, cost_out != nullptr);
+    const bool need_rgb = !records;
+    if (records && (!lc || !rc)) lc = rc = nullptr;
     void *rgbv = nullptr;
     if (need_rgb && (!lc || !rc)) {
         // gray replicated into three channels (seq/Main.cpp:87-90 reads the files as colour)
@@ -508,6 +523,17 @@ rts_status pipeline_device(rts_ctx *c, const rts_params &p, int H, int W, const 
             else launch_wta_diag(s, final_vol, (uint16_t *)raw, (int *)rlast, H, W, p.disp_range);
             launch_wta_fill(s, (const uint16_t *)raw, (const int *)rlast, dr, H, W, 1);
             count_launch(c, 2);
+        }
+        StageScope sc(c, "cross_check");
+        launch_cross_check(s, dl, dr, mask, H, W);
+        count_launch(c);
+        return check_launch(c, "pipeline");
+    }
+    if (records) {
+        {
+            StageScope sc(c, "right_view");
+            ViewIn v{rg, lg, rc, lc, rl, ll, 1};
+            RTS_TRY(run_view(c, p, H, W, v, dr, 1, nullptr));
         }
         StageScope sc(c, "cross_check");
         launch_cross_check(s, dl, dr, mask, H, W);

@@ -119,3 +119,23 @@ def test_ad_census_volume(ctx, oracle_mod, W, H, D, colour):
         assert bits_equal(got[0], o[0])
         if prec == 0:
             assert bits_equal(got[1], o[1]) and bits_equal(got[2], o[2])
+
+
+@pytest.mark.parametrize("kw", [dict(aggr=1, box_rad=3), dict(aggr=1, box_rad=9), dict(aggr=1, cost1=3, cost2=0),
+                                dict(aggr=1, cost1=3, cost2=1, lambda2=25.0), dict(aggr=2, aw_rad=4),
+                                dict(aggr=2, aw_rad=4, cost1=1, cost2=0), dict(aggr=2, aw_rad=4, cost1=2, rank_rad=3),
+                                dict(aggr=0)], ids=str)
+@pytest.mark.parametrize("colour", [False, True])
+@pytest.mark.parametrize("want_cost", [False, True])
+def test_right_view_from_shared_records(ctx, oracle_mod, kw, colour, want_cost):
+    """Both views where the right one reads the left one's records, and where it cannot."""
+    import rtstereo_gb300 as R
+    W, H, D = 83, 30, 36
+    (L, Rr), (Lc, Rc) = pair(77, W, H, D, colour)
+    ll, rl = R.rgb_to_lab(Lc), R.rgb_to_lab(Rc)
+    p = R.params(disp_range=D, **kw)
+    imgs = (L, Rr, Lc, Rc) if colour else (L, Rr, None, None)
+    got = ctx.pipeline(p, *imgs, ll, rl, want_cost=want_cost)
+    o = oracle_mod.pipeline(oracle_mod.params(D=D, **kw), L, Rr, Lc, Rc, ll, rl, want_cost=want_cost)
+    for a, b in zip(got, o):
+        assert a is None or bits_equal(a, b)
