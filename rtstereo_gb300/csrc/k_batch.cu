@@ -1031,7 +1031,8 @@ __device__ __forceinline__ void dual_item(const ViewDesc &V, const ViewDesc &VR,
 }
 
 template <typename ST, int NWB>
-__global__ void __launch_bounds__(NWB * 32, NWB == 4 ? 3 : 1)
+// (blocks an SM: the rings of 12 bytes a row and lane admit three, of 8 bytes, f16 segments, four)
+__global__ void __launch_bounds__(NWB * 32, NWB == 4 ? (std::is_same<ST, __half>::value ? 4 : 3) : 1)
     k_vert_dual(ViewTable t, int L, int R, int DEP, const float *__restrict__ rcp) {
     extern __shared__ __align__(16) unsigned char vsm[];
     const int nv = t.nviews;
