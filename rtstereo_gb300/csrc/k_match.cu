@@ -14,36 +14,53 @@ namespace rts {
 // ---------------------------------------------------------------------------
 // Cost volumes from two images: cost[y][x][d] = K::cost(ref word of x, target word of
 // x -+ d).  Block per (row, kRowTX pixels): the words of the pixels and of every target
-// column they meet (wrapped once, D <= W) are made once in shared memory, then the
-// block's kRowTX D consecutive entries are written in order, a line of 32 per warp and
-// step.  magic = ceil(2^20 / D): i / D for i below 16 * 256 (the error is below 1 / 256,
-// at most 1 / D), so each half of the block has indices of its own.
+// column they meet (wrapped once, D <= W) are made once in shared memory, target column u
+// in array u mod 4; a thread makes 4 consecutive disparities of a pixel, lanes on
+// consecutive groups (so on consecutive words), and stores them as 16 bytes where every
+// group starts on 16 (`vec`).  magic = ceil(2^20 / groups): i / groups for i below
+// 32 * 64 (the error i / 2^20 is below 1 / 64, at most 1 / groups).
 // Bound: instruction issue, then the volume's write (a division, two dependent image
-// reads and byte loads per entry before: colour AD 640x480, D = 64 79 us; 30 us now).
-constexpr int kRowTX = 32;
+// reads and byte loads per entry before: colour AD 640x480, D = 64 79 us; an entry a
+// thread 30 us; 25 us now; gray AD 1280x720, D = 64 172, 67 and 57 us).
+constexpr int kRowTX = 32, kRowNT = (kRowTX + 256) / 4;
 template <typename K>
-__global__ void __launch_bounds__(256) k_cost_rows(K k, float *__restrict__ cost, int D, int W, int dir,
+__global__ void __launch_bounds__(256) k_cost_rows(K k, float *__restrict__ cost, int D, int W, int dir, int vec,
                                                    uint32_t magic) {
     using T = typename K::T;
-    __shared__ T ref[kRowTX], tar[kRowTX + 255];
-    const int tid = threadIdx.x, x0 = blockIdx.x * kRowTX;
+    __shared__ T ref[kRowTX], tar[4][kRowNT];
+    const int tid = threadIdx.x, x0 = blockIdx.x * kRowTX, ng = (D + 3) >> 2, Dp = 4 * ng;
     const size_t row = (size_t)blockIdx.y * W;
-    const int t0 = dir > 0 ? x0 - D + 1 : x0;  // target column of tar[0]
-    for (int i = tid; i < kRowTX + D - 1; i += 256) {
+    // L2R: target column u of tar is x0 - Dp + u, entry (x, d) at u = x + Dp - d; R2L: x0 + u, x + d
+    const int t0 = dir > 0 ? x0 - Dp : x0;
+    for (int i = tid; i < kRowTX + Dp; i += 256) {
         int xt = t0 + i;
         if (xt < 0) xt += W;                                  // seq/PixelBasedCost.cpp:19-20
         else if (dir < 0 && xt >= W) xt -= W;                 // :32-33
-        tar[i] = k.load_tar(row + imin(xt, W - 1));           // columns of no pixel are clamped
+        tar[i & 3][i >> 2] = k.load_tar(row + imax(imin(xt, W - 1), 0));  // columns of no pixel are clamped
     }
     if (tid < kRowTX) ref[tid] = k.load_ref(row + imin(x0 + tid, W - 1));
     __syncthreads();
-    const int n = imin(kRowTX, W - x0) * D, half = kRowTX / 2 * D;
+    const int n = imin(kRowTX, W - x0) * ng;
     float *out = cost + (row + x0) * D;
 #pragma unroll 2
     for (int i = tid; i < n; i += 256) {
-        const int up = i >= half ? kRowTX / 2 : 0, j = i - (up ? half : 0);
-        const int px = (int)(((uint32_t)j * magic) >> 20), d = j - px * D, x = px + up;
-        out[i] = k.cost(ref[x], tar[dir > 0 ? x + D - 1 - d : x + d]);
+        const int x = (int)(((uint32_t)i * magic) >> 20), d = 4 * (i - x * ng);
+        const T a = ref[x];
+        const int u = dir > 0 ? x + Dp - d : x + d;
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int uj = dir > 0 ? u - j : u + j;
+            v[j] = k.cost(a, tar[uj & 3][uj >> 2]);
+        }
+        float *o = out + (size_t)x * D + d;
+        if (vec) {
+            *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (d + j < D) o[j] = v[j];
+        }
     }
 }
 
@@ -130,9 +147,11 @@ __global__ void k_census_bits(const uint8_t *__restrict__ img, uint8_t *__restri
 // load and compare a bit; two divisions a bit before: 640x480, 9x7 72 us an image; 19 us
 // now).
 constexpr int kBitsT = 128, kBitsMax = 256;
+template <bool WIN>  // the 9x7 window, unrolled
 __global__ void __launch_bounds__(kBitsT) k_census_bits_px(const uint8_t *__restrict__ img, uint8_t *__restrict__ bits,
-                                                           int hr, int wr, int H, int W, int wide) {
+                                                           int hr_, int wr_, int H, int W, int wide) {
     extern __shared__ __align__(16) uint8_t sb[];  // [128][nb]
+    const int hr = WIN ? 4 : hr_, wr = WIN ? 3 : wr_;
     const int nb = (2 * hr + 1) * (2 * wr + 1), tid = threadIdx.x;
     const long np = (long)H * W, p0 = (long)blockIdx.x * kBitsT, p = p0 + tid;
     if (p < np) {
@@ -142,9 +161,16 @@ __global__ void __launch_bounds__(kBitsT) k_census_bits_px(const uint8_t *__rest
         if (x >= wr && x < W - wr && y >= hr && y < H - hr) {
             // the window inside the image: no wrapping
             const uint8_t *row = img + p - (size_t)hr * W - wr;
-            for (int dy = -hr; dy <= hr; dy++, row += W)
-#pragma unroll 7
-                for (int dx = 0; dx <= 2 * wr; dx++) *o++ = c > row[dx] ? 1 : 0;
+            if constexpr (WIN) {
+                int v[63];
+#pragma unroll
+                for (int k = 0; k < 63; k++) v[k] = row[(size_t)(k / 7) * W + k % 7];
+#pragma unroll
+                for (int k = 0; k < 63; k++) o[k] = (uint8_t)((uint32_t)(v[k] - c) >> 31);
+            } else {
+                for (int dy = -hr; dy <= hr; dy++, row += W)
+                    for (int dx = 0; dx <= 2 * wr; dx++) *o++ = c > row[dx] ? 1 : 0;
+            }
         } else {
             for (int dy = -hr; dy <= hr; dy++) {
                 const uint8_t *row = img + (size_t)wrap1(y + dy, H) * W;
@@ -535,7 +561,8 @@ __global__ void __launch_bounds__(256) k_combine(float *__restrict__ c1, const f
 static dim3 row_grid(long per_row, int H, int threads) { return dim3((unsigned)((per_row + threads - 1) / threads), H); }
 
 template <typename K> static void cost_rows(cudaStream_t s, const K &k, float *cost, int D, int H, int W, int dir) {
-    k_cost_rows<<<dim3((W + kRowTX - 1) / kRowTX, H), 256, 0, s>>>(k, cost, D, W, dir, ((1u << 20) + D - 1) / D);
+    const int ng = (D + 3) / 4, vec = D % 4 == 0 && ((uintptr_t)cost & 15) == 0 ? 1 : 0;
+    k_cost_rows<<<dim3((W + kRowTX - 1) / kRowTX, H), 256, 0, s>>>(k, cost, D, W, dir, vec, ((1u << 20) + ng - 1) / ng);
 }
 void launch_ad_gray(cudaStream_t s, const uint8_t *ref, const uint8_t *tar, float *cost, int D, int H, int W, int dir) {
     cost_rows(s, CostGray{ref, tar}, cost, D, H, W, dir);
@@ -551,8 +578,10 @@ void launch_census_bits(cudaStream_t s, const uint8_t *img, uint8_t *bits, int h
     const long nb = (long)(2 * hr + 1) * (2 * wr + 1);
     if (nb <= kBitsMax) {
         const int wide = ((uintptr_t)bits & 15) == 0 ? 1 : 0;
-        k_census_bits_px<<<(unsigned)(((long)H * W + kBitsT - 1) / kBitsT), kBitsT, (size_t)kBitsT * nb, s>>>(
-            img, bits, hr, wr, H, W, wide);
+        const unsigned g = (unsigned)(((long)H * W + kBitsT - 1) / kBitsT);
+        const size_t smem = (size_t)kBitsT * nb;
+        if (hr == 4 && wr == 3) k_census_bits_px<true><<<g, kBitsT, smem, s>>>(img, bits, hr, wr, H, W, wide);
+        else k_census_bits_px<false><<<g, kBitsT, smem, s>>>(img, bits, hr, wr, H, W, wide);
         return;
     }
     k_census_bits<<<row_grid(W * nb, H, 256), 256, 0, s>>>(img, bits, hr, wr, H, W);

@@ -230,3 +230,11 @@ def test_find_cross(ctx, oracle_mod, H, W, arm, tau):
     rgb = patches(W, H, W)
     got, want = ctx.findCross(rgb, arm, tau), oracle_mod.find_cross(rgb, arm, tau)
     assert bits_equal(got[0], want[0]) and bits_equal(got[1], want[1])
+
+
+def test_disp_refinement_crosses_above_16_bits(ctx, oracle_mod):
+    """Arms of 255 on a flat image: crosses of more than 65535 pixels."""
+    H, W, D = 300, 520, 5
+    horz, vert = ctx.findCross(np.zeros((H, W, 3), np.uint8), 255, 20)
+    disp = np.random.default_rng(0).integers(0, 2, (H, W), dtype=np.uint8) * 4
+    assert bits_equal(ctx.disp_refinement(disp, horz, vert, D), oracle_mod.disp_refinement(disp, horz, vert, D))
