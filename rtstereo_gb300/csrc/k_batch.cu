@@ -54,6 +54,7 @@ __device__ __forceinline__ int find_view(const int *__restrict__ off, int n, int
 constexpr int kPrepTW = 64, kPrepTH = 16, kPrepT = 256;
 constexpr uint32_t kNoPixel = 0xff000000u;
 
+// (a tile row has at most 64 + 2 * 31 columns: arms up to 23, census windows of 64 bits, ranks up to 16)
 static size_t prep_smem(int gr, int gc, int L) {
     return (size_t)4 * (kPrepTW + 2 * L) * (kPrepTH + 2 * L) + (size_t)(kPrepTH + 2 * gr) * (kPrepTW + 2 * gc);
 }
@@ -110,25 +111,38 @@ __global__ void __launch_bounds__(kPrepT) k_prep_views(ViewTable t, int hr_, int
         uint4 *rec = img ? V.rtar : V.rref;
         uint2 *arm = img ? V.atar : V.aref;
         __syncthreads();  // previous item done with the tiles
-        // a warp per tile row
+        // a warp per tile row, the row's (at most 128) columns in flight together
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint8_t *csrc = med ? med : (rgb ? rgb : gray);
         for (int r = warp; r < chh; r += kPrepT / 32) {
             const int yy = y0 - L + r;
             const bool row = yy >= 0 && yy < H;
-            for (int cx = lane; cx < cw; cx += 32) {
-                const int xx = x0 - L + cx;
-                uint32_t col = kNoPixel;
-                if (row && xx >= 0 && xx < W) col = pixel_word<GRAYREC>(csrc, rgb != nullptr, (size_t)yy * W + xx);
-                ct[r * cw + cx] = col;
+            uint32_t col[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int xx = x0 - L + lane + 32 * k;
+                col[k] = kNoPixel;
+                if (row && lane + 32 * k < cw && xx >= 0 && xx < W)
+                    col[k] = pixel_word<GRAYREC>(csrc, rgb != nullptr, (size_t)yy * W + xx);
             }
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (lane + 32 * k < cw) ct[r * cw + lane + 32 * k] = col[k];
         }
         if (want_code || rank >= 0)
             for (int r = warp; r < gh; r += kPrepT / 32) {
                 // rows / columns past the last pixel's window are never read; clamp them
                 // into the single-wrap range (the window radii are below H and W)
                 const uint8_t *grow = gray + (size_t)wrap1(imin(y0 - gr + r, H - 1 + gr), H) * W;
-                for (int cx = lane; cx < gw; cx += 32) gt[r * gw + cx] = grow[wrap1(imin(x0 - gc + cx, W - 1 + gc), W)];
+                uint8_t g[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int cx = lane + 32 * k;
+                    g[k] = cx < gw ? grow[wrap1(imin(x0 - gc + cx, W - 1 + gc), W)] : (uint8_t)0;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (lane + 32 * k < gw) gt[r * gw + lane + 32 * k] = g[k];
             }
         __syncthreads();
         const int px = threadIdx.x & (kPrepTW - 1);

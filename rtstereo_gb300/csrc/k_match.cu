@@ -274,7 +274,15 @@ __global__ void __launch_bounds__(kWinT) k_window(const uint8_t *__restrict__ im
     for (int r = warp; r < th; r += kWinT / 32) {
         // rows and columns past the last pixel's window are clamped into range (never used)
         const uint8_t *row = img + (size_t)wrap1(imin(y0 - hr + r, H - 1 + hr), H) * W;
-        for (int c = lane; c < tw; c += 32) wt[r * tw + c] = row[wrap1(imin(x0 - wr + c, W - 1 + wr), W)];
+        uint8_t g[6];  // the row's (at most 64 + 2 kWinMax) columns in flight together
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            const int c = lane + 32 * k;
+            g[k] = c < tw ? row[wrap1(imin(x0 - wr + c, W - 1 + wr), W)] : (uint8_t)0;
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++)
+            if (lane + 32 * k < tw) wt[r * tw + lane + 32 * k] = g[k];
     }
     __syncthreads();
     const int px = threadIdx.x & (kWinTX - 1), x = x0 + px;

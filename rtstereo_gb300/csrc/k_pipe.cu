@@ -40,7 +40,15 @@ __global__ void __launch_bounds__(kRecT) k_prep_records(const uint8_t *__restric
         for (int r = threadIdx.x >> 5; r < gh; r += kRecT / 32) {
             // past the last pixel's window: clamped into range, never used
             const uint8_t *row = gray + (size_t)wrap1(imin(y0 - hr + r, H - 1 + hr), H) * W;
-            for (int c = lane; c < gw; c += 32) gt[r * gw + c] = row[wrap1(imin(x0 - wr + c, W - 1 + wr), W)];
+            uint8_t g[4];  // the row's (at most 64 + 2 * 31) columns in flight together
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int c = lane + 32 * k;
+                g[k] = c < gw ? row[wrap1(imin(x0 - wr + c, W - 1 + wr), W)] : (uint8_t)0;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (lane + 32 * k < gw) gt[r * gw + lane + 32 * k] = g[k];
         }
         __syncthreads();
     }

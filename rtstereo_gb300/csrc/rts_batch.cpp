@@ -209,6 +209,8 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
     std::string key = shape_key(n, pairs, params);
     const bool forced = c->force_tune[0] > 0;
     if (forced) key.append((const char *)c->force_tune, sizeof(c->force_tune));
+    // optional scratch is kept per stream, and a graph holds its arena's address
+    if (optional) key.append((const char *)&c->stream, sizeof(c->stream));
     // the tables the kernels read must hold this lambda pair before any replay
     RTS_TRY(cross_tables(c, p));
     int gray = 1;  // records hold the gray byte as colour only when no pair has colour images
