@@ -103,6 +103,22 @@ def test_box(ctx, oracle_mod, H, W, D, r):
     assert np.array_equal(np.isnan(got), np.isnan(want)) and bits_equal(np.nan_to_num(got), np.nan_to_num(want))
 
 
+# means of signed sums beside flat areas (sums of exactly zero), partial blocks of disparities,
+# tiles inside and at the wrap
+@pytest.mark.parametrize("H,W,D,r", [(40, 70, 64, 4), (21, 50, 34, 1), (24, 150, 130, 8)])
+def test_ncc_box_flat(ctx, oracle_mod, H, W, D, r):
+    import rtstereo_gb300 as R
+    O = oracle_mod
+    L, Rr, _ = R.synth_pair(D + r, W, H, D, 3, 0, 2.0, 4)
+    L[:, W // 2:] = 90
+    Rr[:, W // 2:] = 90
+    p = R.params(disp_range=D, cost1=R.COST_NCC, cost2=R.COST_NONE, aggr=R.AGGR_BOX, box_rad=r, ncc_hrad=2, ncc_wrad=2)
+    got = ctx.pipeline(p, L, Rr)
+    c = (R.gray_to_rgb(L), R.gray_to_rgb(Rr))
+    want = O.pipeline(O.params(cost1=5, cost2=0, aggr=1, D=D, box_rad=r, ncc_hrad=2, ncc_wrad=2), L, Rr, *c)
+    assert all(bits_equal(got[i], want[i]) for i in range(3))
+
+
 # whole and partial pixel blocks of a row, every code width, both directions
 @pytest.mark.parametrize("H,W,D", [(1, 1, 1), (3, 31, 9), (2, 64, 64), (5, 33, 33), (2, 300, 256), (70, 20, 20)])
 def test_cost_rows(ctx, oracle_mod, H, W, D):
