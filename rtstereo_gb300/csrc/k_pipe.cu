@@ -111,7 +111,9 @@ __global__ void k_cost_volume(const uint4 *__restrict__ rr, const uint4 *__restr
 // records for 16 entries, lanes (disparity groups) on consecutive ones.  The tables are
 // staged 2^lc1 and 2^lc2 times over, copy = lane: a warp's 32 lookups of one table hit
 // nearly 32 different banks (a single copy costs some 3.5 wavefronts a lookup).
-// Bound: the volume's write and the population counts.
+// Bound: the L1/shared data pipe (70 % busy: about 6 wavefronts a warp's 32 entries, records
+// 2.75, lookups and their conflicts 3.5); the next item's records are fetched under the
+// entries' work (1920x1080, D = 128, records and both volumes 608 -> 545 us).
 constexpr int kAdcTX = 64;
 constexpr int kAdcL1 = 768, kAdcL2 = 68;    // table entries staged: AD <= 765, census <= 64
 constexpr int kAdcNT = (kAdcTX + 256) / 4;  // target records of one residue
@@ -131,21 +133,36 @@ __global__ void __launch_bounds__(256, 3) k_cost_volume_adc(const uint4 *__restr
     const float *l1 = t1 + (lane & ((1 << lc1) - 1)), *l2 = t2 + (lane & ((1 << lc2) - 1));
     const int ndg = (D + 3) >> 2, Dp = 4 * ndg, xb = (W + kAdcTX - 1) / kAdcTX;
     const bool vec = (pitch & 3) == 0;
+    // an item's records, two a thread (kAdcTX + Dp targets, then the references): fetched
+    // while the previous item is worked
+    static_assert(2 * kAdcTX + 256 <= 2 * 256, "two records a thread");
+    uint4 next[2];
+    auto fetch = [&](int item) {
+        const int y = item / xb, x0 = (item - y * xb) * kAdcTX;
+        const size_t row = (size_t)y * W;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int i = tid + 256 * k, ir = i - (kAdcTX + Dp);
+            if (ir >= kAdcTX) continue;
+            int x = x0 + (ir < 0 ? i - Dp : ir);
+            if (x < 0) x += W;  // seq/PixelBasedCost.cpp:19-20 (D <= W)
+            x = imax(imin(x, W - 1), 0);  // clamped: of no entry
+            next[k] = (ir < 0 ? rt : rr)[row + (mirror ? W - 1 - x : x)];
+        }
+    };
+    if ((int)blockIdx.x < H * xb) fetch(blockIdx.x);
     for (int item = blockIdx.x; item < H * xb; item += gridDim.x) {
         const int y = item / xb, x0 = (item - y * xb) * kAdcTX;
         const size_t row = (size_t)y * W;
         __syncthreads();  // the previous item's records are consumed (and the tables are in)
-        for (int i = tid; i < kAdcTX + Dp; i += 256) {
-            int xt = x0 - Dp + i;
-            if (xt < 0) xt += W;  // seq/PixelBasedCost.cpp:19-20 (D <= W)
-            xt = imax(imin(xt, W - 1), 0);  // clamped: of no entry
-            trec[(i & 3) * kAdcNT + (i >> 2)] = rt[row + (mirror ? W - 1 - xt : xt)];
-        }
-        if (tid < kAdcTX) {
-            const int x = imin(x0 + tid, W - 1);
-            rrec[tid] = rr[row + (mirror ? W - 1 - x : x)];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int i = tid + 256 * k, ir = i - (kAdcTX + Dp);
+            if (ir < 0) trec[(i & 3) * kAdcNT + (i >> 2)] = next[k];
+            else if (ir < kAdcTX) rrec[ir] = next[k];
         }
         __syncthreads();
+        if (item + (int)gridDim.x < H * xb) fetch(item + gridDim.x);
         const int nx = imin(kAdcTX, W - x0);
         // pixel group xg = q / ndg, disparity group dg = q mod ndg; 256 groups at a time
         const int sx = 256 / ndg, sd = 256 - sx * ndg;
