@@ -70,12 +70,6 @@ __device__ __forceinline__ void wta_fill_row(const uint16_t *__restrict__ r, uin
     }
 }
 
-// Packed cross arms of one pixel: left | right<<8 | top<<16 | bottom<<24.
-__device__ __forceinline__ int arm_l(uint32_t a) { return (int)(a & 0xff); }
-__device__ __forceinline__ int arm_r(uint32_t a) { return (int)((a >> 8) & 0xff); }
-__device__ __forceinline__ int arm_t(uint32_t a) { return (int)((a >> 16) & 0xff); }
-__device__ __forceinline__ int arm_b(uint32_t a) { return (int)(a >> 24); }
-
 // One term of CombineCost (seq/CombineCost.cpp:21-22): 1 - exp(-v/lambda).
 // Integer-valued costs in range take it from a table computed on the host with
 // the C library's expf (the reference's arithmetic, so bit-identical); other

@@ -22,13 +22,6 @@ struct CostCfg {
     int itrunc;        // integral truncation, or a large value when not truncating
 };
 
-// Integer value of one cost from records: SAD of the packed RGB bytes (the
-// fourth byte is zero) or the census Hamming distance.
-__device__ __forceinline__ int rec_icost(int kind, const uint4 &a, const uint4 &b, int itrunc) {
-    if (kind == RTS_COST_CENSUS) return __popc(a.x ^ b.x) + __popc(a.y ^ b.y);
-    return imin((int)__vsadu4(a.z, b.z), itrunc);
-}
-
 __device__ __forceinline__ float rec_cost(int kind, const uint4 &a, const uint4 &b, int use_trunc, float trunc) {
     if (kind == RTS_COST_CENSUS) {
         const uint64_t ca = ((uint64_t)a.y << 32) | a.x, cb = ((uint64_t)b.y << 32) | b.x;

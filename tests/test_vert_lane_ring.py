@@ -1,4 +1,4 @@
-"""The per-lane row rings of the vertical cross-aggregation kernel (k_vert_views),
+"""The per-lane row rings of the vertical cross-aggregation kernels (k_vert_dual, k_cross_vol),
 checked on the CPU: tests/native/vert_lane_ring_check.cpp includes the kernel's own
 header (rtstereo_gb300/csrc/rts_vert_ring.h) and replays ticks, slots and walks."""
 import os
