@@ -506,7 +506,8 @@ __global__ void __launch_bounds__(256, 3) k_ncc_tiled(const uint8_t *__restrict_
 
 // LoG differences combined with census Hamming distances in one pass (composed:
 // two volumes and k_combine, seq/Main.cpp:180-234 with LoG first and census
-// second): the same expressions in the same order, one write of the volume.  A warp takes kLcPx consecutive pixels, lane = disparity.
+// second): the same expressions in the same order, one write of the volume.  A warp
+// takes kLcPx consecutive pixels, lane = disparity.
 constexpr int kLcPx = 8;
 
 template <int NW>
