@@ -69,20 +69,67 @@ struct GraphEntry {
     size_t arena_bytes = 0;
     CrossTune tune;
     uint64_t launches = 0;     // kernel launches inside the graph
+    uint64_t turn = 0;         // of the last use
 };
 
 struct GraphCache {
     std::unordered_map<std::string, GraphEntry> graphs;
     std::unordered_map<std::string, CrossTune> tunes;
+    // single pairs of ranges that are not a multiple of 8 (views_launch_pair)
+    std::unordered_map<std::string, GraphEntry> pairs;
+    uint64_t turn = 0;
     ~GraphCache() {
-        for (auto &kv : graphs)
-            if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
+        for (auto *m : {&graphs, &pairs})
+            for (auto &kv : *m)
+                if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     }
 };
 
 GraphCache *cache_of(rts_ctx *c) {
     if (!c->graph_cache) c->graph_cache = new GraphCache();
     return (GraphCache *)c->graph_cache;
+}
+
+// Replays the entry's graph of the stage launches, captured first where there is none for this
+// arena; direct: on a stream that cannot be captured (the legacy default one) the launches
+// themselves.
+template <typename F>
+rts_status launch_graph(rts_ctx *c, GraphEntry &g, void *arena, size_t bytes, const char *stage, bool direct, F launch) {
+    if (g.exec && (g.arena != arena || g.arena_bytes != bytes)) {
+        cudaGraphExecDestroy(g.exec);
+        g.exec = nullptr;
+    }
+    if (!g.exec) {
+        // capture the stage launches; the view table is read from device memory,
+        // so later calls only re-upload it before the replay
+        const bool timing = c->timing;
+        c->timing = false;
+        const uint64_t l0 = c->launches.load();
+        cudaGraph_t graph;
+        const cudaError_t cb = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+        if (cb != cudaSuccess) {
+            c->timing = timing;
+            if (!direct) return cuda_check(c, cb, "cudaStreamBeginCapture");
+            cudaGetLastError();
+            return launch();
+        }
+        rts_status st = launch();
+        cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
+        c->timing = timing;
+        if (st != RTS_OK) return st;
+        RTS_CU(c, ce);
+        ce = cudaGraphInstantiate(&g.exec, graph, 0);
+        cudaGraphDestroy(graph);
+        RTS_CU(c, ce);
+        g.arena = arena;
+        g.arena_bytes = bytes;
+        g.launches = c->launches.load() - l0;
+        c->launches.fetch_sub(g.launches);  // counted on every replay instead
+    }
+    StageScope sc(c, stage);
+    RTS_CU(c, cudaGraphLaunch(g.exec, c->stream));
+    count_launch(c, (int)g.launches);
+    return RTS_OK;
 }
 
 // Fills image/output pointers of the 2n views of n pairs; med (or nullptr)
@@ -192,8 +239,7 @@ rts_status rts_batch_run(rts_ctx *ctx, int n, const rts_pair *pairs, const rts_p
 
 // The batched cross-based pipeline on DEVICE buffers: one view table, autotuned
 // tiles, one captured graph per batch shape.  Callers have validated the pairs.
-rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs,
-                                bool optional) {
+rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs) {
     for (int i = 0; i < n; i++)
         if (!pairs[i].left_gray || !pairs[i].right_gray || !outs[i].disp_left ||
             (params[0].right_view && (!outs[i].disp_right || !outs[i].mask)))
@@ -209,8 +255,9 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
     std::string key = shape_key(n, pairs, params);
     const bool forced = c->force_tune[0] > 0;
     if (forced) key.append((const char *)c->force_tune, sizeof(c->force_tune));
-    // optional scratch is kept per stream, and a graph holds its arena's address
-    if (optional) key.append((const char *)&c->stream, sizeof(c->stream));
+    const size_t bytes = views_bytes(W.data(), H.data(), D.data(), nv, half);
+    void *arena;
+    RTS_TRY(scratch(c, SL_BATCH0, bytes, &arena));
     // the tables the kernels read must hold this lambda pair before any replay
     RTS_TRY(cross_tables(c, p));
     int gray = 1;  // records hold the gray byte as colour only when no pair has colour images
@@ -231,15 +278,6 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
         }
         median_pairs(c, p.median_ksize, n, pairs, dst.data(), med);
     }
-    // the arena last: a later allocation could give optional scratch back
-    const size_t bytes = views_bytes(W.data(), H.data(), D.data(), nv, half);
-    void *arena;
-    if (optional) {
-        arena = stream_work(c, bytes);
-        if (!arena) return set_error(c, RTS_ERR_OOM, "no optional scratch");
-    } else {
-        RTS_TRY(scratch(c, SL_BATCH0, bytes, &arena));
-    }
     ViewBatch b;
     plan_views_at(arena, W.data(), H.data(), D.data(), nv, half, &b);
     fill_views(b, n, pairs, outs, right, p.median_ksize ? &med : nullptr);
@@ -250,20 +288,6 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
         ft.vert_rows = c->force_tune[0];
         ft.grid_mult = c->force_tune[1];
         ft.persistent = c->force_tune[2];
-        tit = gc->tunes.emplace(key, ft).first;
-    }
-    if (tit == gc->tunes.end() && optional) {
-        // strips that give the vertical kernel some five blocks an SM (450x375, D = 60, photo: strips
-        // of 375 rows 263 us, of 96 rows 161, of 48 rows 170), none shorter than 64 rows
-        long items = 0;
-        int h = 1;
-        for (const ViewDesc &v : b.views) {
-            items += stage_items(ST_VERT, v, v.H, b.max_d);
-            h = std::max(h, v.H);
-        }
-        const long strips = std::max(1L, std::min((5L * sm_count() + items - 1) / std::max(items, 1L), h / 64L));
-        CrossTune ft;
-        ft.vert_rows = (int)((h + strips - 1) / strips);
         tit = gc->tunes.emplace(key, ft).first;
     }
     if (tit == gc->tunes.end()) {
@@ -306,38 +330,38 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
         return launch_cross_views(c, p, t, segk, 0, gray, b.max_d, tune, b.row_last_all, b.row_last_count);
     }
     GraphEntry &g = gc->graphs[key];
-    if (g.exec && (g.arena != arena || g.arena_bytes != bytes)) {
-        cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
+    g.tune = tune;
+    return launch_graph(c, g, arena, bytes, "batch_graph", false, [&] {
+        return launch_cross_views(c, p, t, segk, 0, gray, b.max_d, tune, b.row_last_all, b.row_last_count);
+    });
+}
+
+rts_status rts::views_launch_pair(rts_ctx *c, const rts_params &p, const ViewBatch &b, const ViewTable &t, int segk,
+                                  int gray, const CrossTune &tune, void *arena, size_t bytes) {
+    auto launch = [&] {
+        return launch_cross_views(c, p, t, segk, 0, gray, b.max_d, tune, b.row_last_all, b.row_last_count);
+    };
+    if (c->timing) return launch();
+    const int d[5] = {b.views[0].W, b.views[0].H, gray, tune.vert_rows, 16 * tune.grid_mult + tune.persistent};
+    std::string key((const char *)&p, sizeof(p));
+    key.append((const char *)d, sizeof(d));
+    GraphCache *gc = cache_of(c);
+    auto it = gc->pairs.find(key);
+    const bool first = it == gc->pairs.end();
+    if (first) {
+        constexpr size_t kMaxPairs = 16;
+        if (gc->pairs.size() == kMaxPairs) {
+            auto old = gc->pairs.begin();
+            for (auto i = gc->pairs.begin(); i != gc->pairs.end(); ++i)
+                if (i->second.turn < old->second.turn) old = i;
+            if (old->second.exec) cudaGraphExecDestroy(old->second.exec);  // (freed when it leaves the device)
+            gc->pairs.erase(old);
+        }
+        it = gc->pairs.emplace(key, GraphEntry{}).first;
     }
-    if (!g.exec) {
-        // capture the stage launches; the view table is read from device memory,
-        // so later calls only re-upload it before the replay
-        const bool timing = c->timing;
-        c->timing = false;
-        const uint64_t l0 = c->launches.load();
-        cudaGraph_t graph;
-        RTS_CU(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        rts_status st = launch_cross_views(c, p, t, segk, 0, gray, b.max_d, tune, b.row_last_all, b.row_last_count);
-        cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
-        c->timing = timing;
-        if (st != RTS_OK) return st;
-        RTS_CU(c, ce);
-        ce = cudaGraphInstantiate(&g.exec, graph, 0);
-        cudaGraphDestroy(graph);
-        RTS_CU(c, ce);
-        g.arena = arena;
-        g.arena_bytes = bytes;
-        g.tune = tune;
-        g.launches = c->launches.load() - l0;
-        c->launches.fetch_sub(g.launches);  // counted on every replay instead
-    }
-    {
-        StageScope sc(c, "batch_graph");
-        RTS_CU(c, cudaGraphLaunch(g.exec, c->stream));
-        count_launch(c, (int)g.launches);
-    }
-    return RTS_OK;
+    it->second.turn = ++gc->turn;
+    if (first) return launch();
+    return launch_graph(c, it->second, arena, bytes, "pair_graph", true, launch);
 }
 
 // ===========================================================================

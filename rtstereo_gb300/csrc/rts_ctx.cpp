@@ -51,12 +51,15 @@ rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out) {
     return dev_alloc_once(c, bytes, out);
 }
 
-void *stream_work(rts_ctx *c, size_t bytes) {
+bool stream_capturing(rts_ctx *c) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return nullptr;
-    }
+    if (cudaStreamIsCapturing(c->stream, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+void *stream_work(rts_ctx *c, size_t bytes) {
+    if (stream_capturing(c)) return nullptr;
     size_t i = 0;
     while (i < c->work.size() && c->work[i].stream != c->stream) i++;
     if (i < c->work.size() && c->work[i].buf.bytes >= bytes) return c->work[i].buf.ptr;

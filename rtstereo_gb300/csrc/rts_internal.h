@@ -111,6 +111,9 @@ rts_status scratch(rts_ctx *c, int slot, size_t bytes, void **out);
 rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out);
 void dev_free(rts_ctx *c, void *p, size_t bytes);
 
+// Whether the context's stream is being captured into a caller's graph (or cannot say).
+bool stream_capturing(rts_ctx *c);
+
 // Optional scratch of the context's current stream, for calls that can also do without
 // (their general kernels need none): at least `bytes`, kept per stream so that calls on
 // different streams of one context do not share it; null where there is no room, on a

@@ -11,6 +11,7 @@
 // Both keep the reference's per-entry arithmetic, so they agree bit for bit.
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "rts_internal.h"
@@ -445,6 +446,75 @@ static rts_status reserve_composed_cross(rts_ctx *c, const rts_params &p, int H,
     return scratch(c, SL_V_ROWLAST, (size_t)H * 4, &q);
 }
 
+// Record costs of a range that is not a multiple of 8 through the view kernels, in the plain
+// form (the composed path has no other).  *done is false, with nothing launched, where the
+// call has to go through the module kernels: on a stream that is being captured (the view
+// table is uploaded from pageable memory at each call), or without room for the records.
+// The segments lie in the volumes that reserve_composed_cross holds; what else the views need
+// is 100 bytes a pixel.
+static rts_status pipeline_ragged_views(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *lg,
+                                        const uint8_t *rg, const uint8_t *lc, const uint8_t *rc, uint8_t *dl,
+                                        uint8_t *dr, uint8_t *mask, bool *done) {
+    *done = false;
+    if (stream_capturing(c)) return RTS_OK;
+    RTS_TRY(reserve_composed_cross(c, p, H, W, lc != nullptr));
+    rts_params q = p;
+    q.precision = RTS_PREC_F32;
+    const size_t np = (size_t)H * W, ne = np * p.disp_range;
+    const int nv = p.right_view ? 2 : 1, segk = cross_seg_kind(q, W);
+    const int Ws[2] = {W, W}, Hs[2] = {H, H}, Ds[2] = {p.disp_range, p.disp_range};
+    void *seg[2], *arena = nullptr;
+    RTS_TRY(scratch(c, SL_V_COST1, ne * 4, &seg[0]));
+    RTS_TRY(scratch(c, SL_V_SEG, ne * 4, &seg[1]));
+    const std::string msg = c->last_error;
+    rts_status st = cross_tables(c, q);
+    const size_t bytes = views_bytes(Ws, Hs, Ds, nv, segk != 0, false);
+    if (st == RTS_OK) st = scratch(c, SL_BATCH1, bytes, &arena);
+    if (st == RTS_ERR_OOM) {
+        c->last_error = msg;  // not this call's failure
+        return RTS_OK;
+    }
+    RTS_TRY(st);
+    ViewBatch b;
+    plan_views_at(arena, Ws, Hs, Ds, nv, segk != 0, &b, seg);
+    ViewDesc &v0 = b.views[0];
+    v0.gref = lg; v0.gtar = rg; v0.cref = lc; v0.ctar = rc; v0.mirror = 0; v0.disp = dl;
+    if (p.median_ksize) {
+        const int ch = lc ? 3 : 1;
+        void *mv;
+        RTS_TRY(scratch(c, SL_V_MED, np * 6, &mv));
+        StageScope sc(c, "median");
+        launch_median(c->stream, lc ? lc : lg, (uint8_t *)mv, H, W, ch, p.median_ksize);
+        launch_median(c->stream, rc ? rc : rg, (uint8_t *)mv + np * ch, H, W, ch, p.median_ksize);
+        count_launch(c, 2);
+        v0.mref = (const uint8_t *)mv;
+        v0.mtar = (const uint8_t *)mv + np * ch;
+    }
+    if (nv == 2) {
+        ViewDesc &v1 = b.views[1];
+        v1.gref = rg; v1.gtar = lg; v1.cref = rc; v1.ctar = lc; v1.mirror = 1; v1.disp = dr;
+        v0.mask = mask;
+        link_pair(&b, 0, 1, (size_t)W * p.disp_range < (size_t(1) << 30));  // (32-bit row offsets)
+    }
+    // strips that give the vertical kernel some five blocks an SM (450x375, D = 60, photo: strips
+    // of 375 rows 263 us, of 96 rows 161, of 48 rows 170), none shorter than 64 rows
+    CrossTune tune;
+    if (c->force_tune[0] > 0) {
+        tune.vert_rows = c->force_tune[0];
+        tune.grid_mult = c->force_tune[1];
+        tune.persistent = c->force_tune[2];
+    } else {
+        long items = 0;
+        for (const ViewDesc &v : b.views) items += stage_items(ST_VERT, v, H, b.max_d);
+        const long strips = std::max(1L, std::min((5L * sm_count() + items - 1) / std::max(items, 1L), H / 64L));
+        tune.vert_rows = (int)((H + strips - 1) / strips);
+    }
+    ViewTable t;
+    RTS_TRY(upload_views(c, b, tune, nullptr, &t));
+    *done = true;
+    return views_launch_pair(c, q, b, t, segk, lc ? 0 : 1, tune, arena, bytes);
+}
+
 // Prepares device inputs for both views and runs them; all pointers device.
 rts_status pipeline_device(rts_ctx *c, const rts_params &p, int H, int W, const uint8_t *lg, const uint8_t *rg,
                            const uint8_t *lc, const uint8_t *rc, const uint8_t *ll, const uint8_t *rl, uint8_t *dl,
@@ -456,14 +526,10 @@ rts_status pipeline_device(rts_ctx *c, const rts_params &p, int H, int W, const 
         return pipeline_cross_views(c, p, H, W, lg, rg, lc && rc ? lc : nullptr, lc && rc ? rc : nullptr, dl, dr,
                                     mask);
     if (!cost_out && cross_ragged_supported(p)) {
-        rts_params q = p;
-        q.precision = RTS_PREC_F32;
-        const bool rgb = lc && rc;
-        rts_pair pr{W, H, lg, rg, rgb ? lc : nullptr, rgb ? rc : nullptr, nullptr, nullptr};
-        rts_out o{dl, dr, mask, nullptr};
-        RTS_TRY(reserve_composed_cross(c, p, H, W, rgb));
-        const rts_status st = batch_views_run(c, 1, &pr, &q, &o, true);
-        if (st != RTS_ERR_OOM) return st;  // no room, or a captured stream: the module kernels below
+        bool done;
+        RTS_TRY(pipeline_ragged_views(c, p, H, W, lg, rg, lc && rc ? lc : nullptr, lc && rc ? rc : nullptr, dl, dr,
+                                      mask, &done));
+        if (done) return RTS_OK;
     }
     const bool need_lab = p.aggr == RTS_AGGR_AW;
     // the record path makes colour words from the gray image where there is no colour

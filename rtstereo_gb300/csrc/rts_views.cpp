@@ -7,11 +7,12 @@ namespace rts {
 
 static size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
-size_t views_bytes(const int *W, const int *H, const int *D, int n, int half) {
+size_t views_bytes(const int *W, const int *H, const int *D, int n, int half, bool segs) {
     size_t bytes = 0, rl = 0;
     for (int i = 0; i < n; i++) {
         const size_t np = (size_t)W[i] * H[i], ne = np * D[i];
-        bytes += align256(np * 32) + align256(np * 16) + align256(ne * (half ? 2 : 4)) + align256(np * 2);
+        bytes += align256(np * 32) + align256(np * 16) + align256(np * 2);
+        if (segs) bytes += align256(ne * (half ? 2 : 4));
         rl += H[i];
     }
     bytes += align256(rl * 4);
@@ -20,7 +21,8 @@ size_t views_bytes(const int *W, const int *H, const int *D, int n, int half) {
     return bytes;
 }
 
-void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n, int half, ViewBatch *b) {
+void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n, int half, ViewBatch *b,
+                   void *const *seg) {
     b->views.assign(n, ViewDesc{});
     b->off.assign((size_t)ST_COUNT * (n + 1), 0);
     b->max_d = 0;
@@ -40,8 +42,8 @@ void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n,
         v.aref = (uint2 *)(a + pos);
         v.atar = v.aref + np;
         pos += align256(np * 16);
-        v.seg = a + pos;
-        pos += align256(ne * (half ? 2 : 4));
+        v.seg = seg ? seg[i] : a + pos;
+        if (!seg) pos += align256(ne * (half ? 2 : 4));
         v.raw = (uint16_t *)(a + pos);
         pos += align256(np * 2);
         rl += H[i];

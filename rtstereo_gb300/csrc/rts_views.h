@@ -97,10 +97,12 @@ struct ViewBatch {
 // volume pointers are left for the caller to fill before upload.
 rts_status plan_views(rts_ctx *c, int slot, const int *W, const int *H, const int *D, int n, int half,
                       const CrossTune &tune, ViewBatch *b);
-// Device bytes of the scratch, view table and offsets of n views.
-size_t views_bytes(const int *W, const int *H, const int *D, int n, int half);
-// Carves n views out of an arena of views_bytes() bytes.
-void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n, int half, ViewBatch *b);
+// Device bytes of the scratch, view table and offsets of n views (segs: with their row segments).
+size_t views_bytes(const int *W, const int *H, const int *D, int n, int half, bool segs = true);
+// Carves n views out of an arena of views_bytes() bytes; seg: the views' row segments where
+// these lie outside the arena, or null.
+void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n, int half, ViewBatch *b,
+                   void *const *seg = nullptr);
 // Makes views `left` and `right` one pair: the left view makes the records of
 // both images, the right view reads them (its reference is the right image).
 // shared: the vertical sums of both views come from one kernel (record costs only).
@@ -111,9 +113,11 @@ rts_status upload_views(rts_ctx *c, const ViewBatch &b, const CrossTune &tune, v
 
 // The batched cross-based pipeline over n validated pairs (DEVICE buffers, fast
 // costs): autotuned tiles and one captured CUDA graph per batch shape.
-// optional: in the optional scratch of the stream, tiles by a rule instead of the autotuner;
-// RTS_ERR_OOM, with nothing done, where there is no such scratch.
-rts_status batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs,
-                           bool optional = false);
+rts_status batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const rts_params *params, rts_out *outs);
+// Launches one planned and uploaded pair: directly the first time its shape is met, then through
+// a graph (450x375, D = 60: 244 and 234 us), so that a program whose sizes change with every
+// call captures nothing; the last 16 shapes are kept.
+rts_status views_launch_pair(rts_ctx *c, const rts_params &p, const ViewBatch &b, const ViewTable &t, int segk,
+                             int gray, const CrossTune &tune, void *arena, size_t bytes);
 
 }  // namespace rts

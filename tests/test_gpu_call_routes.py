@@ -1,0 +1,169 @@
+"""Calls whose route depends on the stream, the context's memory or the parameters' signs: the
+results are the oracle's on every route, and no route refuses what another takes."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import bits_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def images(seed, W, H, D):
+    """Random dots, and a colour pair of flat blocks (long arms)."""
+    import rtstereo_gb300 as R
+    L, Rr, _ = R.synth_pair(seed, W, H, D, 3, 0, 2.0, min(4, D - 1))
+    rng = np.random.default_rng(seed)
+    base = np.repeat(np.repeat(rng.integers(0, 200, (H // 11 + 1, W // 11 + 1, 3)), 11, 0), 11, 1)[:H, :W]
+    Lc = (base + L[..., None] // 16).astype(np.uint8)
+    return L, Rr, Lc, np.ascontiguousarray(np.roll(Lc, -2, 1))
+
+
+def oracle_params(O, p):
+    return O.params(cost1=p.cost1, cost2=p.cost2, aggr=p.aggr, lambda1=p.lambda1, lambda2=p.lambda2, D=p.disp_range,
+                    rank_rad=p.rank_rad, box_rad=p.box_rad, cross_L=p.cross_arm, cross_tau=p.cross_tau,
+                    ad_trunc=p.ad_trunc, right_view=p.right_view, median_ksize=p.median_ksize)
+
+
+class DeviceCall:
+    """One rts_pipeline_run on device buffers."""
+
+    def __init__(self, ctx, p, imgs, cost=False):
+        import torch
+        import rtstereo_gb300 as R
+        H, W = imgs[0].shape
+        self.ctx, self.p = ctx, p
+        self.ims = [torch.from_numpy(i).cuda() for i in imgs]
+        self.outs = [torch.zeros(H, W, dtype=torch.uint8, device="cuda") for _ in range(3)]
+        self.vol = torch.empty(H, W, p.disp_range, device="cuda") if cost else None
+        ptr = [i.data_ptr() for i in self.ims] + [None] * (4 - len(imgs))
+        self.pair = R.Pair(W, H, *ptr, None, None)
+        self.out = R.Out(*[t.data_ptr() for t in self.outs], self.vol.data_ptr() if cost else None)
+        torch.cuda.synchronize()
+
+    def __call__(self):
+        import rtstereo_gb300 as R
+        self.ctx.call("pipeline_run", R.DEVICE, C.byref(self.pair), C.byref(self.p), C.byref(self.out))
+
+    def check(self, want):
+        import torch
+        torch.cuda.synchronize()
+        for t, w in zip(self.outs, want[:3] if self.p.right_view else want[:1]):
+            assert bits_equal(t.cpu().numpy(), w)
+
+
+def last_error(ctx):
+    return ctx._lib.rts_ctx_last_error(ctx.h)
+
+
+@pytest.mark.parametrize("median", [0, 3])
+def test_recorded_after_calls_for_the_volume(oracle_mod, median):
+    """A context that has only made the volume (module kernels) can record the same pair without
+    it, and records nothing besides that call's kernels."""
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    W, H, D = 70, 45, 20
+    im = images(5, W, H, D)
+    s = torch.cuda.Stream()
+    with R.Context(0) as ctx:
+        ctx.set_stream(s.cuda_stream)
+        p = R.params(disp_range=D, median_ksize=median)
+        warm, call = DeviceCall(ctx, p, im, cost=True), DeviceCall(ctx, p, im)
+        n0 = ctx.kernel_launches
+        warm()
+        n1, msg = ctx.kernel_launches, last_error(ctx)
+        s.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            call()
+        # as many kernels as the volume's call (its cross aggregation adds up to three a view)
+        assert ctx.kernel_launches - n1 <= n1 - n0
+        assert last_error(ctx) == msg
+        g.replay()
+        call.check(oracle_mod.pipeline(oracle_params(oracle_mod, p), *im))
+        ctx.set_stream(None)
+
+
+def test_recorded_after_another_range(oracle_mod):
+    """The same after calls of a larger range that went through the view kernels."""
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    W, H = 70, 45
+    s = torch.cuda.Stream()
+    with R.Context(0) as ctx:
+        ctx.set_stream(s.cuda_stream)
+        p = R.params(disp_range=13)
+        im = images(6, W, H, 13)
+        DeviceCall(ctx, R.params(disp_range=21), im)()
+        s.synchronize()
+        for cost in (False, True):  # both forms find their scratch
+            call = DeviceCall(ctx, p, im, cost)
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                call()
+            g.replay()
+            call.check(oracle_mod.pipeline(oracle_params(oracle_mod, p), *im))
+        ctx.set_stream(None)
+
+
+@pytest.mark.parametrize("D", [20, 61])
+def test_default_stream_handles(oracle_mod, D):
+    """The legacy default stream cannot be captured; calls on it and on the per-thread one work."""
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    im = images(7, 80, 40, D)
+    p = R.params(disp_range=D)
+    want = oracle_mod.pipeline(oracle_params(oracle_mod, p), *im)
+    with R.Context(0) as ctx:
+        for handle in (1, 2):  # cudaStreamLegacy, cudaStreamPerThread
+            ctx.set_stream(handle)
+            call = DeviceCall(ctx, p, im)
+            for _ in range(3):
+                call()
+                call.check(want)
+        torch.cuda.synchronize()
+        ctx.set_stream(None)
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(right_view=0), dict(cost1=3, cost2=0), dict(median_ksize=5)], ids=str)
+def test_ragged_ranges_of_changing_size(oracle_mod, kw):
+    """Larger and smaller pairs in turn over the same scratch, with and without colour."""
+    import rtstereo_gb300 as R
+    with R.Context(0) as ctx:
+        for W, H, D in ((40, 30, 9), (90, 50, 33), (40, 30, 9), (61, 70, 60), (90, 50, 33)):
+            im = images(W, W, H, D)
+            p = R.params(disp_range=D, **kw)
+            for rgb in (True, False):
+                got = ctx.pipeline(p, *(im if rgb else im[:2]))
+                gray = [np.repeat(g[..., None], 3, 2) for g in im[:2]]
+                want = oracle_mod.pipeline(oracle_params(oracle_mod, p), *im[:2], *(im[2:] if rgb else gray))
+                for a, b in zip(got[:3] if p.right_view else got[:1], want):
+                    assert bits_equal(a, b)
+
+
+def test_ragged_pairs_hold_no_second_volume():
+    """A ragged range through the view kernels holds the module kernels' volumes and 100 bytes a
+    pixel (each slot an eighth and two pages more), whatever the range."""
+    import rtstereo_gb300 as R
+    W, H, D = 130, 70, 61
+    im = images(2, W, H, D)
+    with R.Context(0) as a, R.Context(0) as b:
+        a.pipeline(R.params(disp_range=D), *im)
+        b.pipeline(R.params(disp_range=D), *im, want_cost=True)
+        out = W * H * D * 4  # b's volume on its way to the host
+        assert a.bytes_in_use - (b.bytes_in_use - out) <= 1.125 * (100 * W * H + 16384) + 3 * 8192
+
+
+def test_more_shapes_than_graphs(oracle_mod):
+    """Ragged shapes met again and again, more of them than graphs are kept."""
+    import rtstereo_gb300 as R
+    dims = [(130 + 3 * i, 20 + i, 9 + i) for i in range(19)]
+    data = [images(W, W, H, D) for W, H, D in dims]
+    with R.Context(0) as ctx:
+        ps = [R.params(disp_range=D) for _, _, D in dims]
+        want = [oracle_mod.pipeline(oracle_params(oracle_mod, p), *im) for p, im in zip(ps, data)]
+        for order in (range(19), range(19), (0, 0, 0, 18, 18, 5, 5, 0), reversed(range(19))):
+            for i in order:
+                got = ctx.pipeline(ps[i], *data[i])
+                assert all(bits_equal(a, b) for a, b in zip(got[:3], want[i]))
