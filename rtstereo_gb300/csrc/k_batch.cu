@@ -1299,7 +1299,7 @@ rts_status launch_cross_views(rts_ctx *c, const rts_params &p, const ViewTable &
         const int R = tune.vert_rows;
         rts_status vs = RTS_OK;
         if (t.total[ST_BEST] > 0) {
-            // both views of every pair at once (costs from records: all >= 0)
+            // both views of every pair at once (costs from records, all >= 0)
             auto go = [&](auto kern, int nwb, size_t smem) {
                 vs = set_smem(c, kern, smem, "vert_dual");
                 if (vs != RTS_OK) return;
@@ -1331,10 +1331,8 @@ rts_status launch_cross_views(rts_ctx *c, const rts_params &p, const ViewTable &
                 kern<<<grid(t.total[ST_VERT], 1, resident_blocks(kern, kVertT, smem)), kVertT, smem, s>>>(t, L, R, DEP,
                                                                                                        rcp);
             };
-            // non-negative costs take the fast exact division: every cost made from records,
-            // and every precomputed volume but NCC's (AD, rank and LoG differences, Hamming
-            // distances and their CombineCost terms 1 - exp(-v / lambda) are >= 0)
-            const bool pos = mode != 0 || (p.cost1 != RTS_COST_NCC && p.cost2 != RTS_COST_NCC);
+            // non-negative costs take the fast exact division
+            const bool pos = costs_nonneg(p);
 #define RTS_VERT(ST, N)                                   \
         do {                                                  \
             if (!pos) go(k_vert_views<ST, N, 0>);             \

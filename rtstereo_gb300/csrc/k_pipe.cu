@@ -890,6 +890,12 @@ bool fast_costs(const rts_params &p) {
     return !census || (2 * p.census_hrad + 1) * (2 * p.census_wrad + 1) <= 64;
 }
 
+bool costs_nonneg(const rts_params &p) {
+    if (p.cost1 == RTS_COST_NCC || p.cost2 == RTS_COST_NCC) return false;
+    if (p.cost1 == RTS_COST_AD && p.aggr == RTS_AGGR_CROSS && !(p.ad_trunc >= 0.f)) return false;
+    return p.cost2 == RTS_COST_NONE || (p.lambda1 > 0.f && p.lambda2 > 0.f);
+}
+
 bool fused_supported(const rts_params &p, int H, int W) {
     (void)H;
     (void)W;
@@ -966,11 +972,9 @@ bool cross_fused_supported(const rts_params &p) {
 bool cross_ragged_supported(const rts_params &p) {
     // The view kernels take any range, with the results of the composed module kernels
     // (450x375, D = 60, photo: 571 us a pair composed, 256 us here) where costs are made from records
-    // and are >= 0 (their quotients take the fast exact division): positive lambdas, no
-    // negative truncation.  Other costs stay composed.
+    // and are >= 0 (their quotients take the fast exact division).  Other costs stay composed.
     return p.aggr == RTS_AGGR_CROSS && p.cross_arm <= 23 && p.disp_range % 8 != 0 && cross_record_costs(p) &&
-           (p.cost2 == RTS_COST_NONE || (p.lambda1 > 0.f && p.lambda2 > 0.f)) &&
-           (p.cost1 != RTS_COST_AD || p.ad_trunc >= 0.f);
+           costs_nonneg(p);
 }
 
 rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W) {

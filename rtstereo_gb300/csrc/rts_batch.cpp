@@ -134,9 +134,11 @@ rts_status launch_graph(rts_ctx *c, GraphEntry &g, void *arena, size_t bytes, co
 
 // Fills image/output pointers of the 2n views of n pairs; med (or nullptr)
 // holds the median-filtered arm images, left and right of every pair.
-void fill_views(ViewBatch &b, int n, const rts_pair *pairs, const rts_out *outs, int right,
+void fill_views(ViewBatch &b, const rts_params &p, int n, const rts_pair *pairs, const rts_out *outs, int right,
                 const std::vector<uint8_t *> *med) {
-    bool shared = true;  // all pairs of a launch or none
+    // all pairs of a launch or none; the shared kernel takes costs that are >= 0 (and its row
+    // offsets are 32-bit)
+    bool shared = costs_nonneg(p);
     for (const ViewDesc &v : b.views) shared = shared && (size_t)v.W * v.D < (size_t(1) << 30);
     for (int i = 0; i < n; i++) {
         const rts_pair &q = pairs[i];
@@ -155,7 +157,6 @@ void fill_views(ViewBatch &b, int n, const rts_pair *pairs, const rts_out *outs,
             r.disp = outs[i].disp_right;
             r.vol = nullptr;
             l.mask = outs[i].mask;
-            // (the shared kernel's row offsets are 32-bit)
             link_pair(&b, 2 * i, 2 * i + 1, shared);
         }
     }
@@ -280,7 +281,7 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
     }
     ViewBatch b;
     plan_views_at(arena, W.data(), H.data(), D.data(), nv, half, &b);
-    fill_views(b, n, pairs, outs, right, p.median_ksize ? &med : nullptr);
+    fill_views(b, p, n, pairs, outs, right, p.median_ksize ? &med : nullptr);
     // autotune once per shape: time every candidate on this batch
     auto tit = gc->tunes.find(key);
     if (tit == gc->tunes.end() && forced) {
@@ -680,7 +681,7 @@ rts_status launch_batch(rts_server *s, std::vector<Request *> &ids) {
     ViewBatch b;
     if (st == RTS_OK) {
         plan_views_at(bt.arena, W.data(), H.data(), D.data(), nv, half, &b);
-        fill_views(b, n, pairs.data(), outs.data(), right, p.median_ksize ? &med : nullptr);
+        fill_views(b, p, n, pairs.data(), outs.data(), right, p.median_ksize ? &med : nullptr);
         ViewTable t;
         CrossTune tune;
         // one block per work item (the default): the blocks of a large request take

@@ -8,6 +8,11 @@ namespace rts {
 
 // AD / census (<= 64-bit window) single or combined costs, computed on the fly
 bool fast_costs(const rts_params &p);
+// every cost is >= 0: absolute differences and distances, and 1 - exp(-c / lambda) of such a
+// c for a positive lambda; not NCC, nor AD cut at a negative truncation (cross-based
+// aggregation truncates the first cost).  The kernels then order costs by their bits and
+// divide by a product and its correction; others compare signed keys and divide.
+bool costs_nonneg(const rts_params &p);
 // adaptive-weight aggregation (radius <= 16) has a fused per-view path
 bool fused_supported(const rts_params &p, int H, int W);
 

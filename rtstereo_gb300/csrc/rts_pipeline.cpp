@@ -217,10 +217,8 @@ static rts_status view_composed(rts_ctx *c, const rts_params &p, int H, int W, c
             StageScope sc(c, "box_wta");
             RTS_CU(c, cudaMemsetAsync(rl, 0xff, (size_t)H * 4, s));
             RTS_CU(c, cudaMemsetAsync(bestv, 0xff, np * 8, s));
-            // every cost but NCC is >= 0 (absolute differences, distances, 1 - exp(-c/l))
-            const bool pos = p.cost1 != RTS_COST_NCC;
             launch_box_best(s, c1, (unsigned long long *)bestv, (uint16_t *)raw, (int *)rl, H, W, D, p.box_rad, argmax,
-                            pos ? 1 : 0, box_best_r);
+                            costs_nonneg(p) ? 1 : 0, box_best_r);
             count_launch(c, 2);
         }
         {

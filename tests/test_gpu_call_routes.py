@@ -142,6 +142,62 @@ def test_ragged_ranges_of_changing_size(oracle_mod, kw):
                     assert bits_equal(a, b)
 
 
+# lambdas and truncations that make costs negative: the general division and signed keys
+NEGATIVE = [dict(lambda1=-5.0, lambda2=30.0), dict(lambda1=-5.0, lambda2=-20.0), dict(ad_trunc=-3.0),
+            dict(cost1=1, cost2=0, ad_trunc=-3.0), dict(cost1=1, cost2=0, ad_trunc=-2.5),
+            dict(cost1=2, cost2=3, rank_rad=3, lambda2=-9.0), dict(cost1=4, cost2=3, lambda1=-9.0),
+            dict(cost1=3, cost2=1, lambda2=-25.0)]
+
+
+@pytest.mark.parametrize("kw", NEGATIVE, ids=str)
+@pytest.mark.parametrize("aggr", [3, 1])
+@pytest.mark.parametrize("D", [24, 36, 40])
+def test_negative_costs(ctx, oracle_mod, kw, aggr, D):
+    import rtstereo_gb300 as R
+    im = images(D, 70, 45, D)
+    p = R.params(disp_range=D, aggr=aggr, box_rad=2, **kw)
+    want = oracle_mod.pipeline(oracle_params(oracle_mod, p), *im)
+    got = ctx.pipeline(p, *im)
+    assert all(bits_equal(a, b) for a, b in zip(got[:3], want))
+
+
+@pytest.mark.parametrize("kw", NEGATIVE[:2], ids=str)
+def test_negative_costs_fp16_batch_and_server(ctx, oracle_mod, kw):
+    """A batch and the serving loop give what single calls give.  FP16 winners: a row segment of costs
+    of one sign is rounded by 2^-11 of itself at most, so a mean is, and a winner's plain cost lies
+    within twice that of the least one (and 2^-14 for the plain form's own roundings)."""
+    pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    dims = [(70, 45, 24), (90, 30, 40)]
+    data = [images(D, W, H, D) for W, H, D in dims]
+    for prec in (R.PREC_F32, R.PREC_F16):
+        ps = [R.params(disp_range=D, precision=prec, **kw) for _, _, D in dims]
+        single = [ctx.pipeline(p, *im)[:3] for p, im in zip(ps, data)]
+        for p, im, s in zip(ps, data, single):
+            plain = oracle_mod.pipeline(oracle_params(oracle_mod, p), *im, want_cost=True)
+            if prec == R.PREC_F32:
+                assert all(bits_equal(a, b) for a, b in zip(s, plain))
+            elif kw["lambda1"] < 0 and kw["lambda2"] < 0:
+                c = plain[3]
+                tol = (2.0 ** -10 + 2.0 ** -14) * np.abs(c).max(2)
+                won = c[:, :, 0] > c.min(2) + tol  # a winner of its own, whatever the roundings
+                lead = np.take_along_axis(c, s[0][..., None].astype(np.int64), 2)[..., 0] - c.min(2)
+                assert won.mean() > 0.5 and (lead[won] <= tol[won]).all()
+        calls = [DeviceCall(ctx, p, im) for p, im in zip(ps, data)]
+        ctx.batch_run([c.pair for c in calls], ps, [c.out for c in calls])
+        for c, s in zip(calls, single):
+            c.check(s)
+        srv = R.Server(ctx, hbm_budget=1 << 28, max_inflight=4, max_batch=2, precision=prec)
+        try:
+            tickets = [srv.submit(p, *im) for p, im in zip(ps, data)]
+            for t, _ in tickets:
+                srv.wait(t)
+            for (_, outs), s in zip(tickets, single):
+                assert all(bits_equal(a, b) for a, b in zip(outs, s))
+        finally:
+            srv.close()
+
+
 def test_ragged_pairs_hold_no_second_volume():
     """A ragged range through the view kernels holds the module kernels' volumes and 100 bytes a
     pixel (each slot an eighth and two pages more), whatever the range."""
