@@ -977,15 +977,6 @@ bool cross_ragged_supported(const rts_params &p) {
            costs_nonneg(p);
 }
 
-rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W) {
-    const float *t, *t2;
-    void *lp;
-    if (p.cost2 != RTS_COST_NONE) RTS_TRY(combine_luts(c, p.lambda1, p.lambda2, &t, &t2));
-    RTS_TRY(prox_weights(c, p.aw_gamma_p, p.aw_rad, &t));
-    RTS_TRY(lab_weight_lut(c, p.aw_gamma_s, &t));
-    return scratch(c, SL_V_MEAN, (size_t)H * W * 8, &lp);
-}
-
 rts_status aw_fused(rts_ctx *c, const rts_params &p, int H, int W, const void *vol, int half, int pitch, const uint8_t *labr,
                     const uint8_t *labt, int mirror, uint16_t *raw, int *rl, float *cost_out) {
     const float *pw, *g;

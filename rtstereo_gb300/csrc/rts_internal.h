@@ -74,6 +74,7 @@ struct rts_ctx {
     rts::DevBuf slots[rts::SL_COUNT];
     std::vector<rts::DevBuf> extra;  // batch / server buffers
     std::vector<rts::StreamWork> work;  // at most rts::kMaxWork (stream_work)
+    size_t padded_refused = ~size_t(0);  // least padded volume there was no room for
     // cached host-computed lookup tables (the key is what the table was made for)
     rts::LutKey lut_key[2];
     bool rcp_ready = false;

@@ -25,8 +25,6 @@ rts_status prep_records(rts_ctx *c, const rts_params &p, int H, int W, const uin
 // order of the bits, which no distance depends on)
 rts_status cost_volume_fast(rts_ctx *c, const rts_params &p, int H, int W, const uint4 *rr, const uint4 *rt,
                             void *vol, int half, int pitch, int mirror);
-// allocates what cost_volume_fast and aw_fused will ask for (tables, packed Lab images)
-rts_status aw_reserve(rts_ctx *c, const rts_params &p, int H, int W);
 // the cross-based pipeline runs over view tables (rts_views.h) when this holds
 bool cross_fused_supported(const rts_params &p);
 // ... and for a disparity range that is not a multiple of 8 when this holds (in the plain

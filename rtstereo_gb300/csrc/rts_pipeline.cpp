@@ -288,6 +288,18 @@ static rts_status view_composed(rts_ctx *c, const rts_params &p, int H, int W, c
     return check_launch(c, "pipeline view");
 }
 
+// scratch() for a size above the least one a call can do with: false, with no error left,
+// where there is no room (asked for once a context), or where a stream that is being captured
+// would have to allocate.
+static bool scratch_padded(rts_ctx *c, int slot, size_t bytes, void **out) {
+    if (c->slots[slot].bytes < bytes && (bytes >= c->padded_refused || stream_capturing(c))) return false;
+    const std::string msg = c->last_error;
+    if (scratch(c, slot, bytes, out) == RTS_OK) return true;
+    c->padded_refused = bytes;
+    c->last_error = msg;
+    return false;
+}
+
 // Fused path for one view (cross-based or adaptive-weight aggregation).
 static rts_status view_fused(rts_ctx *c, const rts_params &p, int H, int W, const ViewIn &v, uint8_t *disp,
                              int mirror, float *cost_out) {
@@ -315,19 +327,11 @@ static rts_status view_fused(rts_ctx *c, const rts_params &p, int H, int W, cons
         void *c1v;
         if (fast) {
             vol_half = half ? 1 : 0;
-            RTS_TRY(scratch(c, SL_V_COST1, ne * (half ? 2 : 4), &c1v));
-            // a range that is not whole 16-byte runs: the volume with its pixels that far apart, in
-            // optional scratch (taken after every other allocation of the view), so that the
-            // aggregation reads it by wide copies
-            const int run = half ? 8 : 4;
-            if (D % run) {
-                RTS_TRY(aw_reserve(c, p, H, W));
-                const int wide = (D + run - 1) / run * run;
-                if (void *w = stream_work(c, np * wide * (half ? 2 : 4))) {
-                    c1v = w;
-                    pitch = wide;
-                }
-            }
+            // a range that is not whole 16-byte runs: the volume with its pixels that far apart,
+            // where there is room, so that the aggregation reads it by wide copies
+            const int run = half ? 8 : 4, wide = (D + run - 1) / run * run;
+            if (scratch_padded(c, SL_V_COST1, np * wide * (half ? 2 : 4), &c1v)) pitch = wide;
+            else RTS_TRY(scratch(c, SL_V_COST1, ne * (half ? 2 : 4), &c1v));
             RTS_TRY(cost_volume_fast(c, p, H, W, rev ? rt : rr, rev ? rr : rt, c1v, vol_half, pitch, rev));
         } else {
             RTS_TRY(scratch(c, SL_V_COST1, ne * 4, &c1v));

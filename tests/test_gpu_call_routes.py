@@ -223,3 +223,68 @@ def test_more_shapes_than_graphs(oracle_mod):
             for i in order:
                 got = ctx.pipeline(ps[i], *data[i])
                 assert all(bits_equal(a, b) for a, b in zip(got[:3], want[i]))
+
+
+@pytest.mark.parametrize("kw", [dict(disp_range=21), dict(disp_range=13, cost1=3, cost2=0),
+                                dict(disp_range=21, aggr=2, aw_rad=3), dict(disp_range=21, aggr=2, aw_rad=3, precision=1),
+                                dict(disp_range=21, aggr=2, aw_rad=17)], ids=str)
+def test_smaller_budgets(kw):
+    """Every budget gives the same bits or is refused; what a call needs at least does not grow
+    with the room there is."""
+    import rtstereo_gb300 as R
+    im = images(9, 90, 40, 24)
+    p = R.params(**kw)
+    lab = [R.rgb_to_lab(i) for i in im[2:]] if p.aggr == R.AGGR_AW else [None, None]
+    with R.Context(0) as ctx:
+        want = ctx.pipeline(p, *im, *lab)[:3]
+        full = ctx.bytes_in_use
+    refused = False
+    for k in range(40, 0, -1):
+        with R.Context(0, full * k // 40) as ctx:
+            try:
+                got = [ctx.pipeline(p, *im, *lab)[:3] for _ in range(2)]
+            except R.RtsError:
+                refused = True
+                continue
+            assert not refused
+            assert all(bits_equal(a, b) for g in got for a, b in zip(g, want))
+    assert refused
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_padded_adaptive_weight_volume_is_the_only_one(prec):
+    """A range that is no multiple of 16 bytes holds no more than the padded range does."""
+    import rtstereo_gb300 as R
+    im = images(4, 90, 30, 24)
+    lab = [R.rgb_to_lab(i) for i in im[2:]]
+    held = []
+    for D in (21, 24):
+        with R.Context(0) as ctx:
+            ctx.pipeline(R.params(disp_range=D, aggr=2, aw_rad=4, precision=prec), *im, *lab)
+            held.append(ctx.bytes_in_use)
+    assert held[0] <= held[1]
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+def test_recorded_adaptive_weights(oracle_mod, prec):
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    im = images(4, 90, 30, 21)
+    lab = [torch.from_numpy(R.rgb_to_lab(i)).cuda() for i in im[2:]]
+    s = torch.cuda.Stream()
+    with R.Context(0) as ctx:
+        ctx.set_stream(s.cuda_stream)
+        p = R.params(disp_range=21, aggr=2, aw_rad=4, precision=prec)
+        call = DeviceCall(ctx, p, im)
+        call.pair.left_lab, call.pair.right_lab = (t.data_ptr() for t in lab)
+        call()
+        torch.cuda.synchronize()
+        want = [t.cpu().numpy() for t in call.outs]
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            call()
+        for t in call.outs:
+            t.zero_()
+        g.replay()
+        call.check(want)
+        ctx.set_stream(None)
