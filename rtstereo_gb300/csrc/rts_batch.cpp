@@ -806,7 +806,13 @@ rts_status rts_server_create(rts_server **out, rts_ctx *ctx, const rts_server_co
     auto *s = new rts_server();
     s->ctx = ctx;
     s->cfg = *cfg;
-    if (!s->pool.init(cfg->hbm_budget)) {
+    bool room = s->pool.init(cfg->hbm_budget);
+    if (!room) {
+        // the context's optional scratch may be in the way
+        std::lock_guard<std::recursive_mutex> lk(ctx->mu);
+        room = give_back_work(ctx) && s->pool.init(cfg->hbm_budget);
+    }
+    if (!room) {
         delete s;
         return set_error(ctx, RTS_ERR_OOM, "cannot reserve the server's device pool");
     }

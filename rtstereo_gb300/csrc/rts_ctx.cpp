@@ -26,6 +26,15 @@ rts_status cuda_check(rts_ctx *c, cudaError_t e, const char *what) {
     return set_error(c, RTS_ERR_CUDA, m);
 }
 
+// Frees one buffer of optional scratch after its last use.
+static void drop_work(rts_ctx *c, size_t i) {
+    StreamWork &w = c->work[i];
+    if (cudaEventSynchronize(w.used) != cudaSuccess) cudaGetLastError();
+    cudaEventDestroy(w.used);
+    dev_free(c, w.buf.ptr, w.buf.bytes);
+    c->work.erase(c->work.begin() + i);
+}
+
 static rts_status dev_alloc_once(rts_ctx *c, size_t bytes, void **out) {
     *out = nullptr;
     if (c->budget && c->used + bytes > c->budget)
@@ -40,15 +49,16 @@ static rts_status dev_alloc_once(rts_ctx *c, size_t bytes, void **out) {
     return RTS_OK;
 }
 
+bool give_back_work(rts_ctx *c) {
+    if (c->work.empty() || stream_capturing(c)) return false;
+    while (!c->work.empty()) drop_work(c, c->work.size() - 1);
+    return true;
+}
+
 rts_status dev_alloc(rts_ctx *c, size_t bytes, void **out) {
     if (bytes == 0) bytes = 256;
-    rts_status s = dev_alloc_once(c, bytes, out);
-    if (s != RTS_ERR_OOM || c->work.empty()) return s;
-    // give the optional scratch back once the device is done with it
-    RTS_CU(c, cudaDeviceSynchronize());
-    for (auto &w : c->work) dev_free(c, w.buf.ptr, w.buf.bytes);
-    c->work.clear();
-    return dev_alloc_once(c, bytes, out);
+    const rts_status s = dev_alloc_once(c, bytes, out);
+    return s == RTS_ERR_OOM && give_back_work(c) ? dev_alloc_once(c, bytes, out) : s;
 }
 
 bool stream_capturing(rts_ctx *c) {
@@ -58,30 +68,65 @@ bool stream_capturing(rts_ctx *c) {
     return true;
 }
 
-void *stream_work(rts_ctx *c, size_t bytes) {
-    if (stream_capturing(c)) return nullptr;
-    size_t i = 0;
-    while (i < c->work.size() && c->work[i].stream != c->stream) i++;
-    if (i < c->work.size() && c->work[i].buf.bytes >= bytes) return c->work[i].buf.ptr;
-    if (i == c->work.size() && i == kMaxWork) return nullptr;
-    const std::string msg = c->last_error;
-    if (i < c->work.size()) {
-        if (cudaStreamSynchronize(c->stream) != cudaSuccess) return nullptr;
-        dev_free(c, c->work[i].buf.ptr, c->work[i].buf.bytes);
-        c->work.erase(c->work.begin() + i);
+OptionalWork::OptionalWork(rts_ctx *c_, size_t bytes) : c(c_) {
+    if (stream_capturing(c)) return;
+    const std::string msg = c->last_error;  // no room is not the call's failure
+    auto pick = [&](auto better) {
+        size_t best = c->work.size();
+        for (size_t i = 0; i < c->work.size(); i++)
+            if (best == c->work.size() || better(c->work[i], c->work[best])) best = i;
+        return best;
+    };
+    auto oldest = [](const StreamWork &a, const StreamWork &b) { return a.turn < b.turn; };
+    // the stream's own buffer, else a new one, else the one unused for longest
+    size_t i = pick([&](const StreamWork &a, const StreamWork &b) {
+        const bool am = a.stream == c->stream, bm = b.stream == c->stream;
+        return am != bm ? am : oldest(a, b);
+    });
+    if (i < c->work.size() && c->work[i].stream != c->stream && c->work.size() < kMaxWork) i = c->work.size();
+    if (i < c->work.size() && c->work[i].buf.bytes < bytes) {
+        drop_work(c, i);
+        i = c->work.size();
     }
-    StreamWork w;
-    w.stream = c->stream;
-    w.buf.bytes = (bytes + bytes / 8 + 4095) & ~size_t(4095);  // room for slightly larger shapes
-    if (dev_alloc_once(c, w.buf.bytes, &w.buf.ptr) != RTS_OK) {
-        w.buf.bytes = bytes;
-        if (dev_alloc_once(c, w.buf.bytes, &w.buf.ptr) != RTS_OK) {
-            c->last_error = msg;  // not this call's failure
-            return nullptr;
+    if (i == c->work.size()) {
+        StreamWork w;
+        w.buf.bytes = (bytes + bytes / 8 + 4095) & ~size_t(4095);  // room for slightly larger shapes
+        bool ok = cudaEventCreateWithFlags(&w.used, cudaEventDisableTiming) == cudaSuccess;
+        if (ok && dev_alloc_once(c, w.buf.bytes, &w.buf.ptr) != RTS_OK) {
+            w.buf.bytes = bytes;
+            ok = dev_alloc_once(c, bytes, &w.buf.ptr) == RTS_OK;
+        }
+        if (ok) {
+            c->work.push_back(w);
+        } else {
+            if (w.used) cudaEventDestroy(w.used);
+            cudaGetLastError();
+            c->last_error = msg;
+            // no room for another: one that is large enough
+            i = pick([&](const StreamWork &a, const StreamWork &b) {
+                const bool al = a.buf.bytes >= bytes, bl = b.buf.bytes >= bytes;
+                return al != bl ? al : oldest(a, b);
+            });
+            if (i == c->work.size() || c->work[i].buf.bytes < bytes) return;
         }
     }
-    c->work.push_back(w);
-    return w.buf.ptr;
+    StreamWork &w = c->work[i];
+    if (cudaStreamWaitEvent(c->stream, w.used, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    w.stream = c->stream;
+    w.turn = ++c->work_turn;
+    ptr = w.buf.ptr;
+}
+
+OptionalWork::~OptionalWork() {
+    if (!ptr) return;
+    for (StreamWork &w : c->work)
+        if (w.buf.ptr == ptr && cudaEventRecord(w.used, c->stream) != cudaSuccess) {
+            cudaGetLastError();
+            cudaStreamSynchronize(c->stream);  // the event cannot stand for this use
+        }
 }
 
 void dev_free(rts_ctx *c, void *p, size_t bytes) {
@@ -102,10 +147,11 @@ rts_status scratch(rts_ctx *c, int slot, size_t bytes, void **out) {
             b.ptr = nullptr;
             b.bytes = 0;
         }
-        rts_status s = dev_alloc(c, want, &b.ptr);
+        rts_status s = dev_alloc_once(c, want, &b.ptr);
         if (s != RTS_OK) {
-            // retry at the exact size before giving up
-            s = dev_alloc(c, bytes, &b.ptr);
+            // retry at the exact size before giving up, or giving optional scratch back
+            s = dev_alloc_once(c, bytes, &b.ptr);
+            if (s != RTS_OK) s = dev_alloc(c, bytes, &b.ptr);
             if (s != RTS_OK) return s;
             want = bytes;
         }
@@ -348,7 +394,7 @@ void rts_ctx_destroy(rts_ctx *c) {
         if (b.ptr) cudaFree(b.ptr);
     for (auto &b : c->extra)
         if (b.ptr) cudaFree(b.ptr);
-    for (auto &w : c->work) cudaFree(w.buf.ptr);
+    while (!c->work.empty()) drop_work(c, c->work.size() - 1);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
 }

@@ -225,6 +225,87 @@ def test_more_shapes_than_graphs(oracle_mod):
                 assert all(bits_equal(a, b) for a, b in zip(got[:3], want[i]))
 
 
+class Aggregation:
+    """One rts_cross_stereo_aggregation on device buffers, large enough for the kernels with scratch."""
+
+    def __init__(self, O, seed, H=90, W=200, D=33):
+        import torch
+        rng = np.random.default_rng(seed)
+        a, b = images(seed, W, H, 16)[2:]
+        arms = [x for im in (a, b) for x in O.find_cross(im, 17, 20)]
+        pre = O.prefix_h(rng.normal(0.5, 1.0, (H, W, D)).astype(np.float32))
+        self.want = O.cross_aggr(pre, arms[0], arms[2], arms[1], arms[3])
+        self.dev = [torch.from_numpy(x).cuda() for x in (pre, arms[0], arms[2], arms[1], arms[3])]
+        self.out = torch.zeros(H, W, D, device="cuda")
+        self.dims = (H, W, D)
+        torch.cuda.synchronize()
+
+    def call(self, ctx):
+        import rtstereo_gb300 as R
+        ctx.call("cross_stereo_aggregation", R.DEVICE, self.dev[0], self.out, *self.dev[1:], *self.dims)
+
+    def check(self):
+        assert bits_equal(self.out.cpu().numpy(), self.want)
+        self.out.zero_()
+
+
+def test_more_streams_than_scratch_buffers(oracle_mod):
+    """Calls on any number of streams, destroyed ones among them, all get scratch and do not
+    overwrite each other's."""
+    torch = pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    jobs = [Aggregation(oracle_mod, i, D=33 + 2 * i) for i in range(7)]
+    with R.Context(0) as ctx:
+        held = []
+        for rnd in range(3):
+            streams = [torch.cuda.Stream() for _ in jobs]
+            for s, j in zip(streams, jobs):
+                ctx.set_stream(s.cuda_stream)
+                n = ctx.kernel_launches
+                j.call(ctx)
+                assert ctx.kernel_launches - n == 4
+            torch.cuda.synchronize()
+            for j in jobs:
+                j.check()
+            held.append(ctx.bytes_in_use)
+            del streams
+        assert max(held) <= 4 * 1.2 * max(4 * (np.prod(j.dims) + 4 * j.dims[0] * j.dims[1]) for j in jobs)
+        ctx.set_stream(None)
+
+
+def test_scratch_within_a_budget(oracle_mod):
+    """Without room for scratch the general kernel makes the same result, and no error is left;
+    scratch stays where another call fits at its exact size, and goes where it does not."""
+    pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    job = Aggregation(oracle_mod, 11)
+    H, W, D = job.dims
+    with R.Context(0, 1 << 20) as ctx:
+        n, msg = ctx.kernel_launches, last_error(ctx)
+        job.call(ctx)
+        assert ctx.kernel_launches - n == 1 and last_error(ctx) == msg
+        ctx.synchronize()
+        job.check()
+    with R.Context(0) as ctx:
+        job.call(ctx)
+        work = ctx.bytes_in_use
+    vol = H * W * D * 4
+    cost = np.random.default_rng(1).normal(0, 1, (H, W, D)).astype(np.float32)
+    tall = np.concatenate([cost, cost])[: H + H // 2]
+    with R.Context(0, work + vol) as ctx:
+        job.call(ctx)
+        assert bits_equal(ctx.aggregate_cost_horizontal(cost), oracle_mod.prefix_h(cost))
+        assert ctx.bytes_in_use == work + vol
+        n = ctx.kernel_launches
+        job.call(ctx)
+        assert ctx.kernel_launches - n == 4
+        assert bits_equal(ctx.aggregate_cost_horizontal(tall), oracle_mod.prefix_h(tall))
+        assert ctx.bytes_in_use <= work + vol
+        job.call(ctx)
+        ctx.synchronize()
+        job.check()
+
+
 @pytest.mark.parametrize("kw", [dict(disp_range=21), dict(disp_range=13, cost1=3, cost2=0),
                                 dict(disp_range=21, aggr=2, aw_rad=3), dict(disp_range=21, aggr=2, aw_rad=3, precision=1),
                                 dict(disp_range=21, aggr=2, aw_rad=17)], ids=str)
