@@ -729,7 +729,8 @@ void launch_disp_refine(cudaStream_t s, uint8_t *disp, uint16_t *runs, const int
                         int D) {
     k_disp_runs<<<row_grid(W, H, 128), 128, 0, s>>>(disp, runs, H, W);
     const size_t smem = (size_t)kRefT * D * sizeof(uint32_t);
-    cudaFuncSetAttribute(k_disp_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (of the largest range: the attribute is not this call's alone, see set_smem)
+    cudaFuncSetAttribute(k_disp_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, kRefT * kMaxDisp * 4);
     k_disp_refine<<<row_grid(W, H, kRefT), kRefT, smem, s>>>(runs, disp, horz, vert, H, W, D);
 }
 

@@ -165,16 +165,22 @@ struct StageScope {
 rts_status check_launch(rts_ctx *c, const char *what);
 // Opts `kern` into `smem` bytes of dynamic shared memory, checking the result
 // (a request above the device's opt-in limit fails here, with the kernel's name,
-// rather than later as a generic launch error).
+// rather than later as a generic launch error).  The attribute is the device's, not the
+// call's: it is only ever raised, and to the limit, so that a call on another thread with a
+// smaller tile cannot lower it between this and the launch.
 template <typename K> rts_status set_smem(rts_ctx *c, K kern, size_t smem, const char *what) {
-    int dev = 0, limit = 0;
+    cudaFuncAttributes at;
+    RTS_CU(c, cudaFuncGetAttributes(&at, kern));
+    if ((size_t)at.maxDynamicSharedSizeBytes >= smem) return RTS_OK;
+    int dev = 0, optin = 0;
     RTS_CU(c, cudaGetDevice(&dev));
-    RTS_CU(c, cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    if (smem > (size_t)limit)
+    RTS_CU(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    const size_t limit = (size_t)optin - at.sharedSizeBytes;
+    if (smem > limit)
         return set_error(c, RTS_ERR_UNSUPPORTED, std::string(what) + ": " + std::to_string(smem) +
                                                      " bytes of shared memory exceed the device's " +
                                                      std::to_string(limit));
-    return cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), what);
+    return cuda_check(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit), what);
 }
 
 // host-computed tables (glibc expf/sqrtf, same as the reference) ----------

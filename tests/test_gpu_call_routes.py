@@ -369,3 +369,33 @@ def test_recorded_adaptive_weights(oracle_mod, prec):
         g.replay()
         call.check(want)
         ctx.set_stream(None)
+
+
+def test_tiles_of_other_threads(oracle_mod):
+    """Contexts on threads of their own whose kernels want different amounts of shared memory."""
+    import threading
+    import rtstereo_gb300 as R
+    L, Rr, Lc, Rc = images(3, 300, 40, 64)
+    disp = np.random.default_rng(0).integers(0, 64, (40, 300), dtype=np.uint8)
+    failures = []
+
+    def work(D, arm, rad):
+        try:
+            with R.Context(0) as c:
+                horz, vert = c.findCross(Lc, 17, 20)
+                jobs = [(lambda: (c.disp_refinement(disp, horz, vert, D),)),
+                        (lambda: c.pipeline(R.params(disp_range=D, cross_arm=arm), L, Rr, Lc, Rc)[:3]),
+                        (lambda: c.pipeline(R.params(disp_range=D, aggr=R.AGGR_AW, aw_rad=rad), L, Rr, Lc, Rc, Lc, Rc)[:3])]
+                want = [j() for j in jobs]
+                for _ in range(150):
+                    for j, w in zip(jobs, want):
+                        assert all(bits_equal(a, b) for a, b in zip(j(), w))
+        except Exception as e:  # noqa: BLE001 (reported below)
+            failures.append(e)
+
+    ts = [threading.Thread(target=work, args=a) for a in ((256, 23, 16), (8, 3, 1), (64, 17, 5), (128, 20, 12))]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not failures
