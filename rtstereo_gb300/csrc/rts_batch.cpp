@@ -136,10 +136,7 @@ rts_status launch_graph(rts_ctx *c, GraphEntry &g, void *arena, size_t bytes, co
 // holds the median-filtered arm images, left and right of every pair.
 void fill_views(ViewBatch &b, const rts_params &p, int n, const rts_pair *pairs, const rts_out *outs, int right,
                 const std::vector<uint8_t *> *med) {
-    // all pairs of a launch or none; the shared kernel takes costs that are >= 0 (and its row
-    // offsets are 32-bit)
-    bool shared = costs_nonneg(p);
-    for (const ViewDesc &v : b.views) shared = shared && (size_t)v.W * v.D < (size_t(1) << 30);
+    const bool shared = pairs_shared(p, b);
     for (int i = 0; i < n; i++) {
         const rts_pair &q = pairs[i];
         ViewDesc &l = b.views[right ? 2 * i : i];
@@ -201,9 +198,13 @@ void view_dims(int n, const rts_pair *pairs, const rts_params *params, int right
         }
 }
 
-// Candidate tiles of the autotuner.
+// Candidate tiles of the autotuner: those of launches whose columns alone fill the GPU, and
+// those of pairs whose columns are few (k_vert_dual walks a column in one warp, so a small pair
+// needs short strips: 160x120, D = 16, dots 91 us at 96 rows, 67 at 16; 320x240 118 and, at 48, 108).
 // (strip rows of the vertical kernel, row-segment blocks per SM, persistent)
-const CrossTune kTuneCandidates[] = {{4096, 8, 0}, {256, 8, 0}, {96, 8, 0}, {4096, 8, 1}, {256, 8, 1}, {4096, 6, 1}};
+const CrossTune kTuneCandidates[][6] = {
+    {{4096, 8, 0}, {256, 8, 0}, {96, 8, 0}, {4096, 8, 1}, {256, 8, 1}, {4096, 6, 1}},
+    {{256, 8, 0}, {96, 8, 0}, {64, 8, 0}, {48, 8, 0}, {32, 8, 0}, {16, 8, 0}}};
 
 }  // namespace
 
@@ -294,12 +295,16 @@ rts_status rts::batch_views_run(rts_ctx *c, int n, const rts_pair *pairs, const 
     if (tit == gc->tunes.end()) {
         const bool timing = c->timing;
         c->timing = false;
-        CrossTune best = kTuneCandidates[0];
+        CrossTune best = kTuneCandidates[0][0];
         float best_ms = 1e30f;
         cudaEvent_t e0, e1;
         RTS_CU(c, cudaEventCreate(&e0));
         RTS_CU(c, cudaEventCreate(&e1));
-        for (const CrossTune &cand : kTuneCandidates) {
+        long items = 0;
+        for (const ViewDesc &v : b.views) items += stage_items(ST_VERT, v, v.H, b.max_d);
+        const bool few = b.views[0].best_r && items < 5L * sm_count();
+        if (few) best = kTuneCandidates[1][0];
+        for (const CrossTune &cand : kTuneCandidates[few ? 1 : 0]) {
             ViewTable t;
             RTS_TRY(upload_views(c, b, cand, nullptr, &t));
             // one untimed run (first launches of a kernel carry set-up costs), then
@@ -684,10 +689,11 @@ rts_status launch_batch(rts_server *s, std::vector<Request *> &ids) {
         fill_views(b, p, n, pairs.data(), outs.data(), right, p.median_ksize ? &med : nullptr);
         ViewTable t;
         CrossTune tune;
+        tune.vert_rows = vert_rows_rule(b);
         // one block per work item (the default): the blocks of a large request take
         // the SMs as the small requests' retire, and a block that starts late owns
         // no share of the items fixed at launch; the small requests' items are short
-        if (s->cfg.priority_pixels > 0 && !bt.high) tune.vert_rows = 256;
+        if (s->cfg.priority_pixels > 0 && !bt.high) tune.vert_rows = std::min(tune.vert_rows, 256);
         st = upload_views(c, b, tune, nullptr, &t);
         if (st == RTS_OK) st = launch_cross_views(c, p, t, segk, 0, gray, b.max_d, tune, b.row_last_all, b.row_last_count);
     }

@@ -11,7 +11,6 @@
 // Both keep the reference's per-entry arithmetic, so they agree bit for bit.
 #include <string.h>
 
-#include <algorithm>
 #include <vector>
 
 #include "rts_internal.h"
@@ -496,20 +495,15 @@ static rts_status pipeline_ragged_views(rts_ctx *c, const rts_params &p, int H, 
         ViewDesc &v1 = b.views[1];
         v1.gref = rg; v1.gtar = lg; v1.cref = rc; v1.ctar = lc; v1.mirror = 1; v1.disp = dr;
         v0.mask = mask;
-        link_pair(&b, 0, 1, (size_t)W * p.disp_range < (size_t(1) << 30));  // (32-bit row offsets)
+        link_pair(&b, 0, 1, pairs_shared(q, b));
     }
-    // strips that give the vertical kernel some five blocks an SM (450x375, D = 60, photo: strips
-    // of 375 rows 263 us, of 96 rows 161, of 48 rows 170), none shorter than 64 rows
     CrossTune tune;
     if (c->force_tune[0] > 0) {
         tune.vert_rows = c->force_tune[0];
         tune.grid_mult = c->force_tune[1];
         tune.persistent = c->force_tune[2];
     } else {
-        long items = 0;
-        for (const ViewDesc &v : b.views) items += stage_items(ST_VERT, v, H, b.max_d);
-        const long strips = std::max(1L, std::min((5L * sm_count() + items - 1) / std::max(items, 1L), H / 64L));
-        tune.vert_rows = (int)((H + strips - 1) / strips);
+        tune.vert_rows = vert_rows_rule(b);
     }
     ViewTable t;
     RTS_TRY(upload_views(c, b, tune, nullptr, &t));

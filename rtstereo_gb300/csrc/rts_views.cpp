@@ -1,6 +1,9 @@
 // rts_views.cpp -- host planning of view tables for the cross-based pipeline.
 #include <string.h>
 
+#include <algorithm>
+
+#include "rts_pipe.h"
 #include "rts_views.h"
 
 namespace rts {
@@ -75,6 +78,27 @@ void link_pair(ViewBatch *b, int left, int right, bool shared) {
     r.atar = l.aref;
     r.mref = l.mtar;
     r.mtar = l.mref;
+}
+
+bool pairs_shared(const rts_params &p, const ViewBatch &b) {
+    bool fits = true, wide = false;
+    for (const ViewDesc &v : b.views) {
+        fits = fits && (size_t)v.W * v.D < (size_t(1) << 30);
+        wide = wide || v.W >= 128;
+    }
+    return fits && wide && costs_nonneg(p);
+}
+
+int vert_rows_rule(const ViewBatch &b) {
+    long items = 0;
+    int h = 1;
+    for (const ViewDesc &v : b.views) {
+        items += stage_items(ST_VERT, v, v.H, b.max_d);
+        h = std::max(h, v.H);
+    }
+    const long want = (5L * sm_count() + items - 1) / std::max(items, 1L);
+    const long strips = std::max(1L, std::min(want, h / 24L));
+    return (int)((h + strips - 1) / strips);
 }
 
 rts_status plan_views(rts_ctx *c, int slot, const int *W, const int *H, const int *D, int n, int half,

@@ -103,6 +103,15 @@ size_t views_bytes(const int *W, const int *H, const int *D, int n, int half, bo
 // these lie outside the arena, or null.
 void plan_views_at(void *arena, const int *W, const int *H, const int *D, int n, int half, ViewBatch *b,
                    void *const *seg = nullptr);
+// Whether the pairs of a launch (all or none) share the vertical kernel: costs >= 0, 32-bit row
+// offsets, and images that are not all narrow (a skewed right view walks 31 columns more:
+// 64x48, D = 16, dots 50 us a pair apart, 56 together; 160x120 75 and 68).
+bool pairs_shared(const rts_params &p, const ViewBatch &b);
+// Strip rows for a launch whose tiles are not tuned by timing: as many strips as give the
+// vertical kernel some five blocks an SM (450x375, D = 60, photo: strips of 375 rows 263 us, of 96
+// rows 161, of 48 rows 170), none shorter than 24 rows (a strip repeats up to 2 L rows of
+// its neighbours; 160x120, D = 16: whole columns 52 us, strips of 24 rows 24, of 16 rows 21).
+int vert_rows_rule(const ViewBatch &b);
 // Makes views `left` and `right` one pair: the left view makes the records of
 // both images, the right view reads them (its reference is the right image).
 // shared: the vertical sums of both views come from one kernel (record costs only).

@@ -225,6 +225,36 @@ def test_more_shapes_than_graphs(oracle_mod):
                 assert all(bits_equal(a, b) for a, b in zip(got[:3], want[i]))
 
 
+def test_batch_of_narrow_and_wide_pairs(ctx, oracle_mod):
+    """Narrow pairs beside a wide one share the vertical kernel; alone they do not."""
+    pytest.importorskip("torch")
+    import rtstereo_gb300 as R
+    dims = [(9, 12, 8), (33, 20, 24), (140, 21, 128), (40, 30, 40), (260, 10, 256)]
+    data = [images(W, W, H, D) for W, H, D in dims]
+    ps = [R.params(disp_range=D) for _, _, D in dims]
+    want = [oracle_mod.pipeline(oracle_params(oracle_mod, p), *im) for p, im in zip(ps, data)]
+    for n in (2, 3, 5):
+        calls = [DeviceCall(ctx, p, im) for p, im in zip(ps[:n], data)]
+        ctx.batch_run([c.pair for c in calls], ps[:n], [c.out for c in calls])
+        for c, w in zip(calls, want):
+            c.check(w)
+
+
+@pytest.mark.parametrize("rows", [16, 24, 33, 64, 4096])
+@pytest.mark.parametrize("W,H,D", [(128, 97, 16), (300, 70, 60), (131, 50, 128)])
+def test_strips(ctx, oracle_mod, rows, W, H, D):
+    import rtstereo_gb300 as R
+    im = images(W, W, H, D)
+    p = R.params(disp_range=D)
+    want = oracle_mod.pipeline(oracle_params(oracle_mod, p), *im)
+    ctx.force_cross_tune(rows)
+    try:
+        got = ctx.pipeline(p, *im)
+    finally:
+        ctx.force_cross_tune(0)
+    assert all(bits_equal(a, b) for a, b in zip(got[:3], want))
+
+
 class Aggregation:
     """One rts_cross_stereo_aggregation on device buffers, large enough for the kernels with scratch."""
 
