@@ -61,6 +61,9 @@ void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D) {
 // Any other arms (*general != 0, known on the device alone) take k_cross_aggr, which
 // reads them as they are; each side returns at once where the other's case holds.
 // 640x480, D = 64, arms near 17: k_cross_aggr alone 1348 us, the three kernels 192 us.
+// So do volumes below kModSmall entries and ranges of one or two, where the launches cost more
+// than they save (160x120, D = 16: 15 us of short arms and 27 of long ones, against 28 and 30).
+constexpr size_t kModSmall = 512 * 1024;
 constexpr int kModArm = 20;  // ring depth 48: 48 KB a block of 4 warps, 4 blocks an SM
 
 __global__ void k_cross_pack(const int *__restrict__ hr, const int *__restrict__ ht, const int *__restrict__ vr,
@@ -120,7 +123,8 @@ __device__ __forceinline__ void add_if_bit(float &acc, uint32_t m, uint32_t bit,
 }
 
 // Vertical sums: a warp streams 32 disparities (lane = disparity) of one column down
-// a strip of rows.  Every lane keeps two rings of its own in shared memory
+// a strip of rows, or for D <= 16 (8) the disparities of 2 (4) neighbouring columns
+// (1 << lcw lanes a column).  Every lane keeps two rings of its own in shared memory
 // (schedule and depth: rts_vert_ring.h), so the warps never wait on one another:
 //   segments  [group of 4 rows][lane][4]: one 16-byte load gives four rows
 //   words     [row][lane]: running sum of l + r down the column (low half, mod 2^16) |
@@ -133,7 +137,7 @@ __device__ __forceinline__ void add_if_bit(float &acc, uint32_t m, uint32_t bit,
 constexpr int kVolWarps = 4;
 __global__ void __launch_bounds__(kVolWarps * 32, 4)
     k_cross_vol(const float *__restrict__ seg, const uint2 *__restrict__ aref, const uint2 *__restrict__ atar,
-                float *__restrict__ out, const int *__restrict__ general, int H, int W, int D, int R) {
+                float *__restrict__ out, const int *__restrict__ general, int H, int W, int D, int R, int lcw) {
     constexpr int S = kVertStep, DEP = vert_lane_depth(kModArm);
     extern __shared__ __align__(16) unsigned char vsm[];
     if (*general) return;
@@ -141,9 +145,10 @@ __global__ void __launch_bounds__(kVolWarps * 32, 4)
     float4 *segr = reinterpret_cast<float4 *>(vsm) + warp * (DEP / 4) * 32 + lane;  // group g at [32 g]
     uint32_t *wrd = reinterpret_cast<uint32_t *>(vsm + (size_t)kVolWarps * DEP * 128) + warp * DEP * 32 + lane;
     const int nch = (D + 31) >> 5, item = blockIdx.x * kVolWarps + warp;
-    const int x = item / nch, d = 32 * (item - x * nch) + lane;
-    if (x >= W) return;
-    const bool dok = d < D;  // a lane past D follows the entry d = 0 and writes nothing
+    const int xw = (item / nch) << (5 - lcw), xl = xw + (lane >> lcw);
+    if (xw >= W) return;
+    const int x = imin(xl, W - 1), d = 32 * (item % nch) + (lane & ((1 << lcw) - 1));
+    const bool dok = d < D && xl < W;  // other lanes follow an entry (x, 0) and write nothing
     const int y0 = blockIdx.y * R, y1 = imin(H, y0 + R);
     const int ra = imax(0, y0 - kModArm), rb = imin(H, y1 + kModArm);
     int xt = x - (dok ? d : 0);
@@ -256,19 +261,22 @@ __global__ void __launch_bounds__(kVolWarps * 32, 4)
     }
 }
 
-// Any arms, straight from the running sums; resident blocks (most calls leave at once).
-// general: null (always), or the flag that says whether the other kernels left the work.
+// Any arms, straight from the running sums: blocks stride over (row, 256 entries).
+// general: null (always; a block per item), or the flag that says whether the other
+// kernels left the work (as many blocks as are resident, since most calls leave at once).
+// Bound: the two reads a row and entry.
 __global__ void __launch_bounds__(256) k_cross_aggr(const float *__restrict__ pre, float *__restrict__ out,
                                                     const int *__restrict__ hr, const int *__restrict__ ht,
                                                     const int *__restrict__ vr, const int *__restrict__ vt,
                                                     const int *__restrict__ general, int H, int W, int D) {
     if (general && !*general) return;
-    const long n = (long)H * W * D;
-    for (long i = (long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
-        const long p = i / D;
-        const int d = (int)(i - p * D), y = (int)(p / W), x = (int)(p - (long)y * W);
+    const uint32_t WD = (uint32_t)W * (uint32_t)D, nb = (WD + 255) >> 8;  // W D < 2^31
+    for (uint32_t item = blockIdx.x; item < (uint32_t)H * nb; item += gridDim.x) {
+        const uint32_t row = item / nb, i = (item - row * nb) * 256 + threadIdx.x;
+        if (i >= WD) continue;
+        const int y = (int)row, x = (int)(i / (uint32_t)D), d = (int)(i - (uint32_t)x * D);
         const int xt = tar_col(x, d, W, 1);
-        const long q = (long)y * W + xt;
+        const long p = (long)y * W + x, q = (long)y * W + xt;
         const int t = imin(vr[2 * p], vt[2 * q]);
         const int b = imin(vr[2 * p + 1], vt[2 * q + 1]);
         float sum = 0.f;
@@ -287,18 +295,21 @@ __global__ void __launch_bounds__(256) k_cross_aggr(const float *__restrict__ pr
                 cnt += r + l + 1;
             }
         }
-        out[i] = __fdiv_rn(sum, (float)cnt);
+        out[(size_t)p * D + d] = __fdiv_rn(sum, (float)cnt);
     }
 }
 
-size_t cross_aggr_bytes(int H, int W, int D) { return (size_t)H * W * (4 * (size_t)D + 16) + 256; }
+size_t cross_aggr_bytes(int H, int W, int D) {
+    const size_t np = (size_t)H * W;
+    return np * D < kModSmall || D <= 2 ? 0 : np * (4 * (size_t)D + 16) + 256;
+}
 
 int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
                       const int *vt, int H, int W, int D, void *work) {
     const int sms = sm_count();
-    const unsigned gen = (unsigned)std::min(((long)H * W * D + 255) / 256, (long)sms * 8);
+    const long items = (long)H * (((long)W * D + 255) / 256);
     if (!work) {
-        k_cross_aggr<<<gen, 256, 0, s>>>(pre, out, hr, ht, vr, vt, nullptr, H, W, D);
+        k_cross_aggr<<<(unsigned)items, 256, 0, s>>>(pre, out, hr, ht, vr, vt, nullptr, H, W, D);
         return 1;
     }
     // {flag, pad to 256 bytes | arm words of both images | segments}
@@ -311,15 +322,18 @@ int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *h
     k_cross_seg<<<dim3((W + kSegTX - 1) / kSegTX, H), 256, 0, s>>>(pre, ra, ta, seg, general, W, D,
                                                                  ((1u << 20) + D - 1) / D);
     // strips: about two waves of warps where the columns alone are fewer (a strip repeats
-    // up to 2 kModArm rows of its neighbours), none shorter than 64 rows
-    const long warps = (long)W * ((D + 31) / 32);
-    const int strips = (int)std::max(1L, std::min((2L * 16 * sms + warps - 1) / warps, (long)H / 64));
+    // up to 2 kModArm rows of its neighbours), none shorter than 24 rows
+    const int lcw = D <= 8 ? 3 : D <= 16 ? 4 : 5;
+    const long warps = (long)((W + (32 >> lcw) - 1) >> (5 - lcw)) * ((D + 31) / 32);
+    const int strips = (int)std::max(1L, std::min((2L * 16 * sms + warps - 1) / warps, (long)H / 24));
     const int R = (H + strips - 1) / strips;
     const size_t smem = (size_t)kVolWarps * vert_lane_depth(kModArm) * 256;
     cudaFuncSetAttribute(k_cross_vol, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_cross_vol<<<dim3((unsigned)((warps + kVolWarps - 1) / kVolWarps), (H + R - 1) / R), kVolWarps * 32, smem, s>>>(
-        seg, ra, ta, out, general, H, W, D, R);
-    k_cross_aggr<<<gen, 256, 0, s>>>(pre, out, hr, ht, vr, vt, general, H, W, D);
+        seg, ra, ta, out, general, H, W, D, R, lcw);
+    int res = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, k_cross_aggr, 256, 0) != cudaSuccess || res < 1) res = 1;
+    k_cross_aggr<<<(unsigned)std::min(items, (long)sms * res), 256, 0, s>>>(pre, out, hr, ht, vr, vt, general, H, W, D);
     return 4;
 }
 

@@ -69,7 +69,7 @@ bool stream_capturing(rts_ctx *c) {
 }
 
 OptionalWork::OptionalWork(rts_ctx *c_, size_t bytes) : c(c_) {
-    if (stream_capturing(c)) return;
+    if (bytes == 0 || stream_capturing(c)) return;
     const std::string msg = c->last_error;  // no room is not the call's failure
     auto pick = [&](auto better) {
         size_t best = c->work.size();

@@ -247,7 +247,7 @@ inline bool median_ksize_ok(int k) { return k >= 3 && k <= 15 && (k & 1); }
 void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W, int ch, int k);
 // k_cross_mod.cu
 void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D);
-// work: cross_aggr_bytes() of scratch, or null (the general kernel
+// work: cross_aggr_bytes() of scratch (0: none is of use), or null (the general kernel
 // alone); returns the kernels launched
 size_t cross_aggr_bytes(int H, int W, int D);
 int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,

@@ -254,3 +254,29 @@ def test_disp_refinement_crosses_above_16_bits(ctx, oracle_mod):
     horz, vert = ctx.findCross(np.zeros((H, W, 3), np.uint8), 255, 20)
     disp = np.random.default_rng(0).integers(0, 2, (H, W), dtype=np.uint8) * 4
     assert bits_equal(ctx.disp_refinement(disp, horz, vert, D), oracle_mod.disp_refinement(disp, horz, vert, D))
+
+
+# columns side by side in a warp (D up to 8 and 16) and their remainders, strips of 24 rows and
+# more, volumes below the size that takes three kernels
+@pytest.mark.parametrize("H,W,D", [(300, 601, 3), (170, 403, 8), (97, 651, 9), (130, 257, 16), (100, 310, 17), (49, 331, 33)])
+@pytest.mark.parametrize("arm", [17, 21])
+def test_cross_aggregation_few_disparities(ctx, oracle_mod, H, W, D, arm):
+    O = oracle_mod
+    a, b = patches_pair(H + W, H, W)
+    (ha, va), (hb, vb) = O.find_cross(a, arm, 20), O.find_cross(b, arm, 20)
+    pre = O.prefix_h(np.random.default_rng(D).normal(0.5, 1.0, (H, W, D)).astype(np.float32))
+    assert bits_equal(ctx.cross_stereo_aggregation(pre, ha, hb, va, vb), O.cross_aggr(pre, ha, hb, va, vb))
+
+
+def test_cross_aggregation_foreign_arms_in_a_large_volume(ctx, oracle_mod):
+    """One arm that leaves the image or passes the rings sends the whole call to the general kernel."""
+    H, W, D = 100, 400, 16
+    a, b = patches_pair(7, H, W)
+    arms = list(oracle_mod.find_cross(a, 17, 20)) + list(oracle_mod.find_cross(b, 17, 20))  # horz, vert; horz, vert
+    pre = oracle_mod.prefix_h(np.random.default_rng(1).random((H, W, D), dtype=np.float32))
+    for k, at, v in ((0, (0, 0, 0), 5), (0, (50, 100, 0), 21), (1, (H - 1, 4, 1), 2), (2, (3, 7, 1), -1), (None, None, 0)):
+        m = [x.copy() for x in arms]
+        if k is not None:
+            m[k][at] = v
+        args = (pre, m[0], m[2], m[1], m[3])
+        assert bits_equal(ctx.cross_stereo_aggregation(*args), oracle_mod.cross_aggr(*args))
