@@ -538,35 +538,50 @@ __global__ void k_disp_runs(const uint8_t *__restrict__ in, uint16_t *__restrict
     if (x < W) runs[(size_t)y * W + x] = (uint16_t)(v | (__ffs(ends >> lane) << 8));
 }
 
-// k_disp_refine: thread per pixel, the histogram of the D disparities as [d][thread]
-// words, so that a warp's counters lie in distinct banks whatever the disparities
-// (a slice per thread put all 32 lanes in one bank).  Bound: the chain of
-// dependent shared-memory updates, one per run.  640x480, D = 64, arms near 17:
-// 2114 us with per-thread slices and one update a pixel, 136 us now.
+// k_disp_refine: thread per pixel, the histogram of the D disparities as [d][thread], so
+// that a warp's counters lie in distinct banks (or, as 16-bit counters, two of them in one)
+// whatever the disparities (a slice per thread put all 32 lanes in one bank).  T: 32-bit
+// counters, or above 128 disparities, where those would leave three blocks an SM, 16-bit ones
+// that stop at 65535; where a counter got there (crosses of more pixels) the full ones'
+// disparities are counted once more.
+// Bound: the chain of dependent reads and shared-memory updates, one per run.  640x480,
+// winners of a colour pair, arms up to 17: D = 64 2058 us with per-thread slices and one update
+// a pixel, 125 us now; D = 256 2097, 289 with 32-bit counters, 196 now.  (On a map of noise, runs
+// of one pixel, D = 256: 515, 857 and 533 us.)
 constexpr int kRefT = 64;
+template <typename T>
 __global__ void __launch_bounds__(kRefT) k_disp_refine(const uint16_t *__restrict__ runs, uint8_t *__restrict__ out,
                                                        const int *__restrict__ horz, const int *__restrict__ vert,
                                                        int H, int W, int D) {
-    extern __shared__ uint32_t hist_smem[];
-    uint32_t *hist = hist_smem + threadIdx.x;
+    extern __shared__ __align__(16) unsigned char hist_smem[];
+    T *hist = reinterpret_cast<T *>(hist_smem) + threadIdx.x;
     const int y = blockIdx.y;
     const int x = blockIdx.x * kRefT + threadIdx.x;
     if (x >= W) return;
     for (int i = 0; i < D; i++) hist[i * kRefT] = 0;
     const long p = (long)y * W + x;
     const int t = vert[2 * p], b = vert[2 * p + 1];
-    for (int yy = imax(y - t, 0); yy < imin(y + b, H); yy++) {
-        const int *h = horz + 2 * ((size_t)yy * W + x);
-        // the reference clamps one side (:189-192); arms made by findCross never
-        // reach past either edge, so clamping both only guards foreign input
-        const int xr = imin(x + h[1], W - 1);
-        const uint16_t *row = runs + (size_t)yy * W;
-        for (int xx = imax(x - h[0], 0); xx <= xr;) {
-            const int w = row[xx], n = imin(w >> 8, xr - xx + 1), v = w & 0xff;
-            if (v < D) atomicAdd(hist + v * kRefT, n);
-            xx += n;
+    // vote(disparity, pixels) for the runs of the cross
+    auto votes = [&](auto vote) {
+        for (int yy = imax(y - t, 0); yy < imin(y + b, H); yy++) {
+            const int *h = horz + 2 * ((size_t)yy * W + x);
+            // the reference clamps one side (:189-192); arms made by findCross never
+            // reach past either edge, so clamping both only guards foreign input
+            const int xr = imin(x + h[1], W - 1);
+            const uint16_t *row = runs + (size_t)yy * W;
+            for (int xx = imax(x - h[0], 0); xx <= xr;) {
+                const int w = row[xx], n = imin(w >> 8, xr - xx + 1);
+                vote(w & 0xff, n);
+                xx += n;
+            }
         }
-    }
+    };
+    votes([&](int v, int n) {
+        if (v >= D) return;
+        T *c = hist + v * kRefT;
+        if constexpr (sizeof(T) == 4) atomicAdd(c, (uint32_t)n);
+        else *c = (T)imin(*c + n, 0xffff);
+    });
     uint32_t best = hist[0];
     int arg = 0;
     for (int i = 1; i < D; i++) {
@@ -574,6 +589,18 @@ __global__ void __launch_bounds__(kRefT) k_disp_refine(const uint16_t *__restric
         if (c > best) {
             best = c;
             arg = i;
+        }
+    }
+    if (sizeof(T) == 2 && best == 0xffff) {
+        long most = 0;
+        for (int i = arg; i < D; i++) {
+            if (hist[i * kRefT] != 0xffff) continue;
+            long c = 0;
+            votes([&](int v, int n) { c += v == i ? n : 0; });
+            if (c > most) {
+                most = c;
+                arg = i;
+            }
         }
     }
     out[p] = (uint8_t)arg;
@@ -728,10 +755,10 @@ void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W
 void launch_disp_refine(cudaStream_t s, uint8_t *disp, uint16_t *runs, const int *horz, const int *vert, int H, int W,
                         int D) {
     k_disp_runs<<<row_grid(W, H, 128), 128, 0, s>>>(disp, runs, H, W);
-    const size_t smem = (size_t)kRefT * D * sizeof(uint32_t);
-    // (of the largest range: the attribute is not this call's alone, see set_smem)
-    cudaFuncSetAttribute(k_disp_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, kRefT * kMaxDisp * 4);
-    k_disp_refine<<<row_grid(W, H, kRefT), kRefT, smem, s>>>(runs, disp, horz, vert, H, W, D);
+    // (32 KB at most in either)
+    const dim3 g = row_grid(W, H, kRefT);
+    if (D > 128) k_disp_refine<uint16_t><<<g, kRefT, (size_t)kRefT * D * 2, s>>>(runs, disp, horz, vert, H, W, D);
+    else k_disp_refine<uint32_t><<<g, kRefT, (size_t)kRefT * D * 4, s>>>(runs, disp, horz, vert, H, W, D);
 }
 
 }  // namespace rts

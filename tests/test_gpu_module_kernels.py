@@ -280,3 +280,15 @@ def test_cross_aggregation_foreign_arms_in_a_large_volume(ctx, oracle_mod):
             m[k][at] = v
         args = (pre, m[0], m[2], m[1], m[3])
         assert bits_equal(ctx.cross_stereo_aggregation(*args), oracle_mod.cross_aggr(*args))
+
+
+# 16-bit counters (D above 128) at their end: two disparities of 78000 votes each (the first where
+# they tie), and one of 117000
+@pytest.mark.parametrize("D", [129, 256])
+def test_disp_refinement_16_bit_counters(ctx, oracle_mod, D):
+    H, W = 300, 520
+    horz, vert = ctx.findCross(np.zeros((H, W, 3), np.uint8), 255, 20)
+    x, y = np.arange(W)[None], np.arange(H)[:, None]
+    for disp in ((x + y) % 2 * (D - 1), np.where(x % 4 == 0, 7, D - 1) + 0 * y):
+        disp = np.ascontiguousarray(disp.astype(np.uint8))
+        assert bits_equal(ctx.disp_refinement(disp, horz, vert, D), oracle_mod.disp_refinement(disp, horz, vert, D))
