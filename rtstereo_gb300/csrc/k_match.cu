@@ -17,16 +17,18 @@ namespace rts {
 // column they meet (wrapped once, D <= W) are made once in shared memory, target column u
 // in array u mod 4; a thread makes 4 consecutive disparities of a pixel, lanes on
 // consecutive groups (so on consecutive words), and stores them as 16 bytes where every
-// group starts on 16 (`vec`).  magic = ceil(2^20 / groups): i / groups for i below
-// 32 * 64 (the error i / 2^20 is below 1 / 64, at most 1 / groups).
+// group starts on 16 (`vec`).  TX pixels a block: 32, and more where a pixel has few groups
+// (128 up to D = 16, 256 up to D = 8), so that every thread has some.  magic = ceil(2^20 /
+// groups): i / groups for i below 32 * 64 (the error i / 2^20 is below 1 / 64, at most
+// 1 / groups; with 128 and 256 pixels i is below 512).
 // Bound: instruction issue, then the volume's write (a division, two dependent image
 // reads and byte loads per entry before: colour AD 640x480, D = 64 79 us; an entry a
 // thread 30 us; 25 us now; gray AD 1280x720, D = 64 172, 67 and 57 us).
-constexpr int kRowTX = 32, kRowNT = (kRowTX + 256) / 4;
-template <typename K>
+template <typename K, int kRowTX>
 __global__ void __launch_bounds__(256) k_cost_rows(K k, float *__restrict__ cost, int D, int W, int dir, int vec,
                                                    uint32_t magic) {
     using T = typename K::T;
+    constexpr int kRowNT = (kRowTX + (kRowTX == 32 ? 256 : kRowTX == 128 ? 16 : 8)) / 4;
     __shared__ T ref[kRowTX], tar[4][kRowNT];
     const int tid = threadIdx.x, x0 = blockIdx.x * kRowTX, ng = (D + 3) >> 2, Dp = 4 * ng;
     const size_t row = (size_t)blockIdx.y * W;
@@ -570,7 +572,12 @@ static dim3 row_grid(long per_row, int H, int threads) { return dim3((unsigned)(
 
 template <typename K> static void cost_rows(cudaStream_t s, const K &k, float *cost, int D, int H, int W, int dir) {
     const int ng = (D + 3) / 4, vec = D % 4 == 0 && ((uintptr_t)cost & 15) == 0 ? 1 : 0;
-    k_cost_rows<<<dim3((W + kRowTX - 1) / kRowTX, H), 256, 0, s>>>(k, cost, D, W, dir, vec, ((1u << 20) + ng - 1) / ng);
+    auto go = [&](auto kern, int tx) {
+        kern<<<dim3((W + tx - 1) / tx, H), 256, 0, s>>>(k, cost, D, W, dir, vec, ((1u << 20) + ng - 1) / ng);
+    };
+    if (D <= 8) go(k_cost_rows<K, 256>, 256);
+    else if (D <= 16) go(k_cost_rows<K, 128>, 128);
+    else go(k_cost_rows<K, 32>, 32);
 }
 void launch_ad_gray(cudaStream_t s, const uint8_t *ref, const uint8_t *tar, float *cost, int D, int H, int W, int dir) {
     cost_rows(s, CostGray{ref, tar}, cost, D, H, W, dir);

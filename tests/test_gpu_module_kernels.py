@@ -292,3 +292,9 @@ def test_disp_refinement_16_bit_counters(ctx, oracle_mod, D):
     for disp in ((x + y) % 2 * (D - 1), np.where(x % 4 == 0, 7, D - 1) + 0 * y):
         disp = np.ascontiguousarray(disp.astype(np.uint8))
         assert bits_equal(ctx.disp_refinement(disp, horz, vert, D), oracle_mod.disp_refinement(disp, horz, vert, D))
+
+
+# the blocks of 128 and 256 pixels of small ranges: whole, partial, one pixel past
+@pytest.mark.parametrize("H,W,D", [(2, 256, 8), (3, 257, 5), (2, 513, 1), (3, 128, 16), (2, 129, 12), (1, 300, 9), (2, 40, 4)])
+def test_cost_rows_of_small_ranges(ctx, oracle_mod, H, W, D):
+    test_cost_rows(ctx, oracle_mod, H, W, D)
