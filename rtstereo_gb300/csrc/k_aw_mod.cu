@@ -247,6 +247,50 @@ __global__ void __launch_bounds__(4 * DC, DC == 64 ? 3 : 5)
     }
 }
 
+// A thread per entry, for ranges and windows that leave most of a tile idle (aw_tiles).  Its
+// weights come from up to 32 different lines a tap.
+// L2R: the weights of the pixels x and x - d.
+__global__ void k_aw_entry_l2r(const float *__restrict__ wr, const float *__restrict__ wt,
+                               const float *__restrict__ cost, float *__restrict__ out, int H, int W, int D, int r) {
+    const int y = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= W * D) return;
+    const int x = i / D, d = i - x * D;
+    const int e = 2 * r + 1, area = e * e;
+    const float *a = wr + ((size_t)y * W + x) * area;
+    const float *b = wt + ((size_t)y * W + tar_col(x, d, W, 1)) * area;
+    float sw = 0.f, sc = 0.f;
+    int k = 0;
+    for (int dy = -r; dy <= r; dy++) {
+        const float *crow = cost + (size_t)wrap1(y + dy, H) * W * D + d;
+        for (int dx = -r; dx <= r; dx++, k++) {
+            const float wgt = __fmul_rn(a[k], b[k]);
+            sw = __fadd_rn(sw, wgt);
+            sc = __fadd_rn(sc, __fmul_rn(crow[(size_t)wrap1(x + dx, W) * D], wgt));
+        }
+    }
+    out[((size_t)y * W + x) * D + d] = __fdiv_rn(sc, sw);
+}
+// R2L: those of the window pixel and of the window pixel + d.
+__global__ void k_aw_entry_r2l(const float *__restrict__ wr, const float *__restrict__ wt,
+                               const float *__restrict__ cost, float *__restrict__ out, int H, int W, int D, int r) {
+    const int y = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= W * D) return;
+    const int x = i / D, d = i - x * D;
+    const int e = 2 * r + 1, area = e * e;
+    float sw = 0.f, sc = 0.f;
+    int k = 0;
+    for (int dy = -r; dy <= r; dy++) {
+        const size_t row = (size_t)wrap1(y + dy, H) * W;
+        for (int dx = -r; dx <= r; dx++, k++) {
+            const int xr = wrap1(x + dx, W), xt = wrap1(x + dx + d, W);
+            const float wgt = __fmul_rn(wr[(row + xr) * area + k], wt[(row + xt) * area + k]);
+            sw = __fadd_rn(sw, wgt);
+            sc = __fadd_rn(sc, __fmul_rn(cost[(row + xr) * D + d], wgt));
+        }
+    }
+    out[((size_t)y * W + x) * D + d] = __fdiv_rn(sc, sw);
+}
+
 // ---------------------------------------------------------------------------
 static dim3 row_grid(long per_row, int H, int threads) { return dim3((unsigned)((per_row + threads - 1) / threads), H); }
 
@@ -261,10 +305,23 @@ void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw,
     k_compute_weights<<<row_grid(W * area, H, 256), 256, 0, s>>>(lab, pw, g, w, H, W, r);
 }
 
-// 32 disparities a tile where that pads less than 64
+// 32 disparities a tile where that pads less than 64.  A thread per entry where the tiles'
+// disparities are so many more than D that their share of idle lanes, and the waits of a
+// tile for its few taps, cost more than the weights' lines: below the line
+// D (24 + 9 r) = 24 (padded D), fitted to 640x480 and 240x180 (L2R, entry against tile: 640x480
+// r = 1, D = 20 91 and 105 us, D = 32 145 and 104; r = 3, D = 12 203 and 236, D = 16 271 and 237;
+// 240x180 r = 8, D = 4 80 and 122, D = 8 equal; r = 16, D = 4 278 and 330); and where the
+// tiles are fewer than half the SMs (64x48, R2L, r = 8, D = 16 43 and 84 us).
 template <bool R2L>
 static void aw_tiles(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H, int W,
                      int D, int r) {
+    const int dc = (D + 31) / 32 < 2 * ((D + 63) / 64) ? 32 : 64, padded = (D + dc - 1) / dc * dc;
+    const long tiles = (long)((W + kAmTX - 1) / kAmTX) * H * (padded / dc);
+    if (D * (24 + 9 * r) < 24 * padded || 2 * tiles < sm_count()) {
+        const auto entry = R2L ? k_aw_entry_r2l : k_aw_entry_l2r;
+        entry<<<row_grid((long)W * D, H, 128), 128, 0, s>>>(wr, wt, cost, out, H, W, D, r);
+        return;
+    }
     auto go = [&](auto kern, int dc, int floats) {
         const size_t smem = (size_t)floats * sizeof(float);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -273,7 +330,7 @@ static void aw_tiles(cudaStream_t s, const float *wr, const float *wt, const flo
         kern<<<dim3((W + kAmTX - 1) / kAmTX, H, (D + dc - 1) / dc), 4 * dc, smem, s>>>(wr, wt, cost, out, H, W, D, r,
                                                                                      vi, vo, 0.f);
     };
-    if ((D + 31) / 32 < 2 * ((D + 63) / 64)) go(k_aw_tile<32, R2L>, 32, kAmBuf<32>);
+    if (dc == 32) go(k_aw_tile<32, R2L>, 32, kAmBuf<32>);
     else go(k_aw_tile<64, R2L>, 64, kAmBuf<64>);
 }
 void launch_aw_l2r_weights(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H,

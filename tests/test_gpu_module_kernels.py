@@ -298,3 +298,15 @@ def test_disp_refinement_16_bit_counters(ctx, oracle_mod, D):
 @pytest.mark.parametrize("H,W,D", [(2, 256, 8), (3, 257, 5), (2, 513, 1), (3, 128, 16), (2, 129, 12), (1, 300, 9), (2, 40, 4)])
 def test_cost_rows_of_small_ranges(ctx, oracle_mod, H, W, D):
     test_cost_rows(ctx, oracle_mod, H, W, D)
+
+
+# enough tiles for the tiled kernels, ranges on both sides of the line to a thread per entry
+@pytest.mark.parametrize("H,W,D,r", [(80, 64, 32, 1), (90, 70, 33, 5), (78, 70, 20, 17), (30, 260, 129, 2), (41, 140, 64, 2),
+                                     (80, 70, 9, 3), (80, 70, 1, 4), (77, 65, 33, 0), (79, 66, 12, 8)])
+def test_adaptive_weight_routes(ctx, oracle_mod, H, W, D, r):
+    O = oracle_mod
+    rng = np.random.default_rng(W + r)
+    wl, wr = rng.normal(0.5, 0.5, (2, H, W, (2 * r + 1) ** 2)).astype(np.float32)
+    cost = rng.normal(0.0, 1.0, (H, W, D)).astype(np.float32)
+    assert bits_equal(ctx.calcAWCostL2R(wl, wr, cost, r), O.aw_l2r(wl, wr, cost, r))
+    assert bits_equal(ctx.calcAWCostR2L(wl, wr, cost, r), O.aw_r2l(wl, wr, cost, r))
