@@ -296,8 +296,9 @@ static dim3 row_grid(long per_row, int H, int threads) { return dim3((unsigned)(
 
 void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw, const float *g, float *w, int H, int W,
                             int r) {
-    // the tile's 48 KB end at radius 46
-    if (cw_smem(r) <= 48 * 1024) {
+    // the tile's 48 KB end at radius 51; windows below 32 weights would leave lanes of the tile's
+    // warps without one (640x480: r = 1 17 us against 41, r = 2 37 and 45)
+    if (r > 2 && cw_smem(r) <= 48 * 1024) {
         k_compute_weights_tile<<<dim3((W + kCwPx - 1) / kCwPx, H), kCwT, cw_smem(r), s>>>(lab, pw, g, w, H, W, r);
         return;
     }

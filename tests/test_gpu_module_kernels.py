@@ -310,3 +310,9 @@ def test_adaptive_weight_routes(ctx, oracle_mod, H, W, D, r):
     cost = rng.normal(0.0, 1.0, (H, W, D)).astype(np.float32)
     assert bits_equal(ctx.calcAWCostL2R(wl, wr, cost, r), O.aw_l2r(wl, wr, cost, r))
     assert bits_equal(ctx.calcAWCostR2L(wl, wr, cost, r), O.aw_r2l(wl, wr, cost, r))
+
+
+# the smallest and largest tiled windows and their neighbours
+@pytest.mark.parametrize("r", [2, 3, 51, 52])
+def test_compute_weights_window_limits(ctx, oracle_mod, r):
+    test_compute_weights_large_window(ctx, oracle_mod, r)
