@@ -257,16 +257,15 @@ __global__ void __launch_bounds__(kBitsT) k_bits_pack(const uint8_t *__restrict_
 
 // ---------------------------------------------------------------------------
 // Window filters of an image: rank, LoG convolution, window mean.  Block per 64 x 16
-// pixels; their wrapped border is staged in shared memory once (single wrap: radii are
-// below the image's sides), a thread makes four pixels of a column.  A window of up to
+// pixels (64 x 4 in small images); their wrapped border is staged in shared memory once
+// (single wrap: radii are below the image's sides), a thread makes four (one) pixels of a column.  A window of up to
 // kWinMax pixels of border takes them; WR, WC: the radii as constants (the usual windows,
 // loops unrolled) or -1.  Bound: the window's shared-memory reads and operations
 // (1280x720: rank 7x7 33 us, LoG 5x5 21 us an image when every window pixel was a
 // wrapped read of the image; 14 and 13 us now).
-constexpr int kWinTX = 64, kWinTY = 16, kWinT = 256, kWinMax = 64;
-static size_t win_smem(int hr, int wr) { return (size_t)(kWinTY + 2 * hr) * (kWinTX + 2 * wr); }
+constexpr int kWinTX = 64, kWinT = 256, kWinMax = 64;
 
-template <typename F, int WR, int WC>
+template <typename F, int WR, int WC, int kWinTY>
 __global__ void __launch_bounds__(kWinT) k_window(const uint8_t *__restrict__ img, typename F::Out *__restrict__ out,
                                                   F f, int H, int W, int hr_, int wr_) {
     extern __shared__ uint8_t wt[];  // [16 + 2 hr][64 + 2 wr]
@@ -628,12 +627,22 @@ void launch_hamming(cudaStream_t s, const uint64_t *cr, const uint64_t *ct, floa
 }
 template <typename F>
 static void window(cudaStream_t s, const uint8_t *img, typename F::Out *out, const F &f, int H, int W, int hr, int wr) {
-    const dim3 g((W + kWinTX - 1) / kWinTX, (H + kWinTY - 1) / kWinTY);
-    if (hr > kWinMax || wr > kWinMax)
+    if (hr > kWinMax || wr > kWinMax) {
         k_window_any<<<row_grid(W, H, 128), 128, 0, s>>>(img, out, f, H, W, hr, wr);
-    else if (hr == 2 && wr == 2) k_window<F, 2, 2><<<g, kWinT, win_smem(2, 2), s>>>(img, out, f, H, W, hr, wr);
-    else if (hr == 3 && wr == 3) k_window<F, 3, 3><<<g, kWinT, win_smem(3, 3), s>>>(img, out, f, H, W, hr, wr);
-    else k_window<F, -1, -1><<<g, kWinT, win_smem(hr, wr), s>>>(img, out, f, H, W, hr, wr);
+        return;
+    }
+    auto go = [&](auto kern, int ty) {
+        kern<<<dim3((W + kWinTX - 1) / kWinTX, (H + ty - 1) / ty), kWinT,
+               (size_t)(ty + 2 * hr) * (kWinTX + 2 * wr), s>>>(img, out, f, H, W, hr, wr);
+    };
+    // tiles of 4 rows where those of 16 are fewer than the SMs
+    const bool few = (long)((W + kWinTX - 1) / kWinTX) * ((H + 15) / 16) < sm_count();
+    if (few && hr == 2 && wr == 2) go(k_window<F, 2, 2, 4>, 4);
+    else if (few && hr == 3 && wr == 3) go(k_window<F, 3, 3, 4>, 4);
+    else if (few) go(k_window<F, -1, -1, 4>, 4);
+    else if (hr == 2 && wr == 2) go(k_window<F, 2, 2, 16>, 16);
+    else if (hr == 3 && wr == 3) go(k_window<F, 3, 3, 16>, 16);
+    else go(k_window<F, -1, -1, 16>, 16);
 }
 void launch_rank(cudaStream_t s, const uint8_t *img, uint8_t *out, int m, int H, int W) {
     window(s, img, out, RankWin{}, H, W, m, m);

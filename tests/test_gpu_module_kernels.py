@@ -316,3 +316,14 @@ def test_adaptive_weight_routes(ctx, oracle_mod, H, W, D, r):
 @pytest.mark.parametrize("r", [2, 3, 51, 52])
 def test_compute_weights_window_limits(ctx, oracle_mod, r):
     test_compute_weights_large_window(ctx, oracle_mod, r)
+
+
+# images of at least as many 64 x 16 tiles as SMs, and one tile fewer
+@pytest.mark.parametrize("H,W", [(16 * 39, 4 * 64 - 3), (16 * 14 + 1, 640)])
+@pytest.mark.parametrize("r", [1, 2, 3, 7])
+def test_window_filters_of_large_images(ctx, oracle_mod, H, W, r):
+    rng = np.random.default_rng(r)
+    img = rng.integers(0, 256, (H, W), dtype=np.uint8)
+    assert bits_equal(ctx.calculateRankFilt(img, r), oracle_mod.rank(img, r))
+    mask = rng.normal(0, 0.2, (2 * r + 1) ** 2).astype(np.float32)
+    assert bits_equal(ctx.convolveImage(img, mask, r, r), oracle_mod.convolve(img, mask, r, r))
