@@ -327,3 +327,10 @@ def test_window_filters_of_large_images(ctx, oracle_mod, H, W, r):
     assert bits_equal(ctx.calculateRankFilt(img, r), oracle_mod.rank(img, r))
     mask = rng.normal(0, 0.2, (2 * r + 1) ** 2).astype(np.float32)
     assert bits_equal(ctx.convolveImage(img, mask, r, r), oracle_mod.convolve(img, mask, r, r))
+
+
+# both sides of the line between the tiled and the entry's kernel, all tiled radii
+@pytest.mark.parametrize("D,r", [(7, 1), (8, 1), (5, 2), (6, 2), (4, 3), (5, 3), (3, 4), (4, 4), (2, 5), (3, 6), (3, 7), (2, 8), (1, 8)])
+def test_box_of_small_ranges(ctx, oracle_mod, D, r):
+    cost = np.random.default_rng(D * r).normal(0.2, 1.0, (30, 45, D)).astype(np.float32)
+    assert bits_equal(ctx.boxAggregate(cost, r), oracle_mod.box(cost, r))
