@@ -261,19 +261,25 @@ __global__ void __launch_bounds__(kVolWarps * 32, 4)
     }
 }
 
-// Any arms, straight from the running sums: blocks stride over (row, 256 entries).
-// general: null (always; a block per item), or the flag that says whether the other
-// kernels left the work (as many blocks as are resident, since most calls leave at once).
+// Any arms, straight from the running sums; an item is (row, 256 entries).  ctl: null (always;
+// a block per item), or {flag that says whether the other kernels left the work, next item}.
+// With the flag most calls leave at once, so the blocks are as many as are resident (an empty
+// launch of 1280x720, D = 64 takes 123 us with an item a block, 4 us so), each taking the next
+// kAggrGrab items as it comes to them: the blocks in flight have to stay on neighbouring
+// rows, which the reads of a cross share in L2 (1280x720, D = 64, arms up to 3 and 25: an item a block
+// 969 and 6952 us, resident blocks that stride over all items 1283 and 9855).
 // Bound: the two reads a row and entry.
+constexpr uint32_t kAggrGrab = 4;
 __global__ void __launch_bounds__(256) k_cross_aggr(const float *__restrict__ pre, float *__restrict__ out,
                                                     const int *__restrict__ hr, const int *__restrict__ ht,
                                                     const int *__restrict__ vr, const int *__restrict__ vt,
-                                                    const int *__restrict__ general, int H, int W, int D) {
-    if (general && !*general) return;
-    const uint32_t WD = (uint32_t)W * (uint32_t)D, nb = (WD + 255) >> 8;  // W D < 2^31
-    for (uint32_t item = blockIdx.x; item < (uint32_t)H * nb; item += gridDim.x) {
+                                                    uint32_t *__restrict__ ctl, int H, int W, int D) {
+    __shared__ uint32_t grab;
+    if (ctl && !ctl[0]) return;
+    const uint32_t WD = (uint32_t)W * (uint32_t)D, nb = (WD + 255) >> 8, items = (uint32_t)H * nb;  // W D < 2^31
+    auto one = [&](uint32_t item) {
         const uint32_t row = item / nb, i = (item - row * nb) * 256 + threadIdx.x;
-        if (i >= WD) continue;
+        if (i >= WD) return;
         const int y = (int)row, x = (int)(i / (uint32_t)D), d = (int)(i - (uint32_t)x * D);
         const int xt = tar_col(x, d, W, 1);
         const long p = (long)y * W + x, q = (long)y * W + xt;
@@ -296,28 +302,40 @@ __global__ void __launch_bounds__(256) k_cross_aggr(const float *__restrict__ pr
             }
         }
         out[(size_t)p * D + d] = __fdiv_rn(sum, (float)cnt);
+    };
+    if (!ctl) {
+        one(blockIdx.x);
+        return;
+    }
+    for (;;) {
+        __syncthreads();  // the last grab is read
+        if (threadIdx.x == 0) grab = atomicAdd(ctl + 1, kAggrGrab);
+        __syncthreads();
+        const uint32_t first = grab;
+        if (first >= items) return;
+        for (uint32_t item = first; item < items && item < first + kAggrGrab; item++) one(item);
     }
 }
 
-size_t cross_aggr_bytes(int H, int W, int D) {
+size_t cross_aggr_bytes(int H, int W, int D, int arm) {
     const size_t np = (size_t)H * W;
-    return np * D < kModSmall || D <= 2 ? 0 : np * (4 * (size_t)D + 16) + 256;
+    return np * D < kModSmall || D <= 2 || arm > kModArm ? 0 : np * (4 * (size_t)D + 16) + 256;
 }
 
 int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
                       const int *vt, int H, int W, int D, void *work) {
     const int sms = sm_count();
-    const long items = (long)H * (((long)W * D + 255) / 256);
     if (!work) {
-        k_cross_aggr<<<(unsigned)items, 256, 0, s>>>(pre, out, hr, ht, vr, vt, nullptr, H, W, D);
+        k_cross_aggr<<<(unsigned)((long)H * (((long)W * D + 255) / 256)), 256, 0, s>>>(pre, out, hr, ht, vr, vt, nullptr,
+                                                                                       H, W, D);
         return 1;
     }
-    // {flag, pad to 256 bytes | arm words of both images | segments}
+    // {flag, next item, pad to 256 bytes | arm words of both images | segments}
     const size_t np = (size_t)H * W;
     int *general = (int *)work;
     uint2 *ra = (uint2 *)((unsigned char *)work + 256), *ta = ra + np;
     float *seg = (float *)(ta + np);
-    cudaMemsetAsync(general, 0, sizeof(int), s);
+    cudaMemsetAsync(general, 0, 2 * sizeof(int), s);
     k_cross_pack<<<dim3((W + 127) / 128, H), 128, 0, s>>>(hr, ht, vr, vt, ra, ta, general, H, W);
     k_cross_seg<<<dim3((W + kSegTX - 1) / kSegTX, H), 256, 0, s>>>(pre, ra, ta, seg, general, W, D,
                                                                  ((1u << 20) + D - 1) / D);
@@ -333,7 +351,7 @@ int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *h
         seg, ra, ta, out, general, H, W, D, R, lcw);
     int res = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, k_cross_aggr, 256, 0) != cudaSuccess || res < 1) res = 1;
-    k_cross_aggr<<<(unsigned)std::min(items, (long)sms * res), 256, 0, s>>>(pre, out, hr, ht, vr, vt, general, H, W, D);
+    k_cross_aggr<<<(unsigned)(sms * res), 256, 0, s>>>(pre, out, hr, ht, vr, vt, (uint32_t *)general, H, W, D);
     return 4;
 }
 

@@ -249,7 +249,8 @@ void launch_median(cudaStream_t s, const uint8_t *in, uint8_t *out, int H, int W
 void launch_prefix_h(cudaStream_t s, float *cost, int H, int W, int D);
 // work: cross_aggr_bytes() of scratch (0: none is of use), or null (the general kernel
 // alone); returns the kernels launched
-size_t cross_aggr_bytes(int H, int W, int D);
+// (arm: no arm is longer, 0 where that is not known)
+size_t cross_aggr_bytes(int H, int W, int D, int arm);
 int launch_cross_aggr(cudaStream_t s, const float *pre, float *out, const int *hr, const int *ht, const int *vr,
                       const int *vt, int H, int W, int D, void *work);
 // k_aw_mod.cu

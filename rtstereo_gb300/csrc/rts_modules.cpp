@@ -397,7 +397,7 @@ rts_status rts_cross_stereo_aggregation(rts_ctx *ctx, rts_mem m, const float *pr
     RTS_TRY(stage_out(c, m, SL_OUT0, out, vol(D, H, W), &dout));
     {
         StageScope sc(c, "cross_aggr");
-        OptionalWork work(c, cross_aggr_bytes(H, W, D));
+        OptionalWork work(c, cross_aggr_bytes(H, W, D, 0));
         count_launch(c, launch_cross_aggr(c->stream, (const float *)dp, (float *)dout, (const int *)a, (const int *)b,
                                           (const int *)cc, (const int *)dd, H, W, D, work.ptr));
     }

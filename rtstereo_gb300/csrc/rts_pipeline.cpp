@@ -269,7 +269,7 @@ static rts_status view_composed(rts_ctx *c, const rts_params &p, int H, int W, c
         launch_find_cross(s, ar, hr, vr, H, W, p.cross_arm, p.cross_tau);
         launch_find_cross(s, at, ht, vt, H, W, p.cross_arm, p.cross_tau);
         launch_prefix_h(s, c1, H, W, D);
-        OptionalWork work(c, cross_aggr_bytes(H, W, D));
+        OptionalWork work(c, cross_aggr_bytes(H, W, D, p.cross_arm));
         count_launch(c, 3 + launch_cross_aggr(s, c1, (float *)finv, hr, ht, vr, vt, H, W, D, work.ptr));
         fin = (float *)finv;
     }
