@@ -308,19 +308,25 @@ void launch_compute_weights(cudaStream_t s, const uint8_t *lab, const float *pw,
 
 // 32 disparities a tile where that pads less than 64.  A thread per entry where the tiles'
 // disparities are so many more than D that their share of idle lanes, and the waits of a
-// tile for its few taps, cost more than the weights' lines: below the line
-// D (24 + 9 r) = 24 (padded D), fitted to 640x480 and 240x180 (L2R, entry against tile: 640x480
-// r = 1, D = 20 91 and 105 us, D = 32 145 and 104; r = 3, D = 12 203 and 236, D = 16 271 and 237;
-// 240x180 r = 8, D = 4 80 and 122, D = 8 equal; r = 16, D = 4 278 and 330); and where the
-// tiles are fewer than half the SMs (64x48, R2L, r = 8, D = 16 43 and 84 us).
+// tile for its few taps, cost more than the weights' lines: up to D = 64, below the lines
+// D (24 + 10 r) = 24 * 32 and D (24 + 16 r) = 24 * 64, fitted to 640x480 and 240x180 (L2R, entry
+// against tile: 640x480 r = 1, D = 20 91 and 105 us, D = 32 145 and 104, D = 33 148 and 197; r = 3,
+// D = 12 203 and 236, D = 16 271 and 237; 240x180 r = 8, D = 4 80 and 122, D = 8 equal; r = 16,
+// D = 4 278 and 330).  Images with fewer tiles than half the SMs: radii up to 6, and D below 32
+// except for large L2R windows (64x48, r = 8, D = 16: L2R 37 and 42 us, R2L 43 and 84;
+// L2R r = 16 124 and 105; these take tiles at D = 1 too, 240x180 437 and 376).
 template <bool R2L>
 static void aw_tiles(cudaStream_t s, const float *wr, const float *wt, const float *cost, float *out, int H, int W,
                      int D, int r) {
     const int dc = (D + 31) / 32 < 2 * ((D + 63) / 64) ? 32 : 64, padded = (D + dc - 1) / dc * dc;
     const long tiles = (long)((W + kAmTX - 1) / kAmTX) * H * (padded / dc);
-    if (D * (24 + 9 * r) < 24 * padded || 2 * tiles < sm_count()) {
-        const auto entry = R2L ? k_aw_entry_r2l : k_aw_entry_l2r;
-        entry<<<row_grid((long)W * D, H, 128), 128, 0, s>>>(wr, wt, cost, out, H, W, D, r);
+    const bool few = 2 * tiles < sm_count();
+    bool entry = D <= 64 && D * (24 + (dc == 32 ? 10 : 16) * r) < 24 * dc;
+    if (few) entry = r <= 6 || (D < 32 && (R2L || r <= 8));
+    if (!R2L && r > 8 && D == 1) entry = false;
+    if (entry) {
+        const auto kern = R2L ? k_aw_entry_r2l : k_aw_entry_l2r;
+        kern<<<row_grid((long)W * D, H, 128), 128, 0, s>>>(wr, wt, cost, out, H, W, D, r);
         return;
     }
     auto go = [&](auto kern, int dc, int floats) {
