@@ -676,9 +676,9 @@ void launch_box(cudaStream_t s, const float *in, float *out, int H, int W, int D
         if (dw == 2) go(k_box_vol<RR, 2>, RR);      \
         else go(k_box_vol<RR, 1>, RR);              \
         return;
-    // up to D (2 r + 3) = 38, k_box: a tile's warps are 32 disparities wide, a radius then saves
-    // less (1280x720, r = 1: D = 6 63 us against 82, D = 8 82 both; r = 4: D = 3 163 and 175)
-    if (D * (2 * r + 3) > 38) switch (r) {
+    // k_box for a few disparities: a tile's warps are 32 wide (1280x720, r = 1: D = 6 63 us against
+    // 82, D = 8 82 both; r = 2: D = 3 65 and 101, D = 4 84 and 74; r = 4: D = 3 163 and 175)
+    if (D > (r == 1 ? 7 : r <= 4 ? 3 : 1)) switch (r) {
         RTS_BOXV(1)
         RTS_BOXV(2)
         RTS_BOXV(3)
