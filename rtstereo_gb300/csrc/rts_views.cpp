@@ -96,8 +96,10 @@ int vert_rows_rule(const ViewBatch &b) {
         items += stage_items(ST_VERT, v, v.H, b.max_d);
         h = std::max(h, v.H);
     }
-    const long want = (5L * sm_count() + items - 1) / std::max(items, 1L);
-    const long strips = std::max(1L, std::min(want, h / 24L));
+    items = std::max(items, 1L);
+    const long sms = sm_count(), tall = std::min((5 * sms + items - 1) / items, h / 64L),
+               small = std::min(5 * sms / (2 * items), h / 16L);
+    const long strips = std::max(1L, std::max(tall, small));
     return (int)((h + strips - 1) / strips);
 }
 
