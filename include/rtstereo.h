@@ -46,7 +46,12 @@ typedef struct rts_ctx rts_ctx;
 /* hbm_budget: bytes of device memory the context may hold (0 = no limit). */
 rts_status rts_ctx_create(rts_ctx **out, int device, size_t hbm_budget);
 void rts_ctx_destroy(rts_ctx *ctx);
-/* Run on an external stream (a cudaStream_t); NULL restores the own stream. */
+/* Run on an external stream (a cudaStream_t); NULL restores the own stream.
+ * While the stream is being captured, calls use the scratch that earlier calls of
+ * the same kind allocated; rts_cross_stereo_aggregation, and cross-based pairs whose
+ * range is not a multiple of 8, then take slower kernels that need no scratch of
+ * their own.  Otherwise the former keeps one volume for each of up to four streams;
+ * calls on more streams share these, in turn. */
 rts_status rts_ctx_set_stream(rts_ctx *ctx, void *cuda_stream);
 void *rts_ctx_stream(rts_ctx *ctx);
 rts_status rts_ctx_synchronize(rts_ctx *ctx);
